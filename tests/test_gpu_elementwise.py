@@ -186,3 +186,25 @@ def test_vocab_parallel_cross_entropy_kernel_on_one_gpu(rows, V, shards):
         assert abs(l.sum().item() - want.item()) / abs(want.item()) < 2e-3
     got = torch.cat([buf[:, : hi - lo] for lo, hi, buf in work], dim=1)
     _close(got, g, name="dlogits")
+
+
+@pytest.mark.parametrize("D", [8, 504, 512, 520, 1024, 1032, 2048, 2056, 4096, 4104, 8192])
+@pytest.mark.parametrize("T", [1, 3, 301])
+def test_rmsnorm_at_the_edges_of_the_row_groups(T, D):
+    """Widths on both sides of each row-group size (32, 64, 128, 256, 512 threads per row) and row counts that leave groups of a
+    block without a row. The weight gradient comes back in bf16 from the summing kernel: the fp32 sum rounded once."""
+    from torchllmtuner_b200 import ops
+    from torchllmtuner_b200.ops import reference as ref
+    from torchllmtuner_b200.ops.cuda_ext import load
+    torch.manual_seed(T + D)
+    x, r, dy, ds = (torch.randn(T, D, device="cuda").bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+    a = [t.clone().requires_grad_() for t in (x, r, w)]
+    b = f32_leaves(*a)
+    got = torch.autograd.grad(ops.add_rms_norm(*a, 1e-6), a, [dy, ds])
+    want = torch.autograd.grad(ref.add_rms_norm(*b, 1e-6), b, [dy.float(), ds.float()])
+    for n, p, q in zip(("dx", "dres", "dw"), got, want):
+        _close(p, q, "reduced" if n == "dw" else None, n)
+    y, rstd, s = load().rmsnorm_fwd(x, r, w, 1e-6)
+    _, dw32 = load().rmsnorm_bwd(dy, s, w, rstd, ds)
+    assert torch.equal(dw32.bfloat16(), got[2])

@@ -314,16 +314,18 @@ std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& re
   return {y, rstd};
 }
 
-// Returns (dx, dw fp32 [D]). `x` is the tensor that was normalised (the sum when a residual was added).
+// Returns (dx, dw [D], fp32 or, with `dw_bf16`, rounded to bf16 by the kernel that sums it). `x` is the tensor that was
+// normalised (the sum when a residual was added).
 std::vector<Tensor> rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd,
-                                const c10::optional<Tensor>& dres) {
+                                const c10::optional<Tensor>& dres, bool dw_bf16) {
   c10::cuda::CUDAGuard guard(x.device());
   check_bf16(dy, "dy");
   check_bf16(x, "x");
   TORCH_CHECK(dy.is_contiguous() && x.is_contiguous());
   const int64_t D = x.size(-1), T = x.numel() / D;
   Tensor dx = torch::empty_like(x);
-  Tensor dw = torch::empty({D}, x.options().dtype(torch::kFloat));
+  Tensor dw = T > 0 ? torch::empty({D}, x.options().dtype(dw_bf16 ? at::kBFloat16 : at::kFloat))
+                    : torch::zeros({D}, x.options().dtype(dw_bf16 ? at::kBFloat16 : at::kFloat));
   Tensor part = torch::empty({llmt_rmsnorm_bwd_partials((int)T), D}, x.options().dtype(torch::kFloat));
   const void* dr = nullptr;
   if (dres.has_value()) {
@@ -332,7 +334,8 @@ std::vector<Tensor> rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor&
     dr = dres->data_ptr();
   }
   check_rc(llmt_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dr, dx.data_ptr(),
-                            part.data_ptr<float>(), dw.data_ptr<float>(), nullptr, 0, (int)T, (int)D, cur_stream()),
+                            part.data_ptr<float>(), dw_bf16 ? nullptr : dw.data_ptr<float>(), dw_bf16 ? dw.data_ptr() : nullptr, 0,
+                            (int)T, (int)D, cur_stream()),
            "llmt_rmsnorm_bwd", 2);
   return {dx, dw};
 }
@@ -356,7 +359,7 @@ std::vector<Tensor> qk_norm_rope_fwd(const Tensor& x, const c10::optional<Tensor
 }
 
 std::vector<Tensor> qk_norm_rope_bwd(const Tensor& dy, const Tensor& x, const c10::optional<Tensor>& w, const Tensor& cosb,
-                                     const Tensor& sinb, const Tensor& rstd) {
+                                     const Tensor& sinb, const Tensor& rstd, bool dw_bf16) {
   c10::cuda::CUDAGuard guard(x.device());
   check_bf16(dy, "dy");
   TORCH_CHECK(dy.dim() == 3 && dy.stride(2) == 1 && dy.stride(1) == dy.size(2));
@@ -366,15 +369,17 @@ std::vector<Tensor> qk_norm_rope_bwd(const Tensor& dy, const Tensor& x, const c1
   Tensor dw, part;
   const void* wp = nullptr;
   float *pp = nullptr, *dwp = nullptr;
+  void* dw16 = nullptr;
   if (w.has_value()) {
     wp = w->data_ptr();
-    dw = torch::empty({HD}, x.options().dtype(torch::kFloat));
+    dw = torch::empty({HD}, x.options().dtype(dw_bf16 ? at::kBFloat16 : at::kFloat));
     part = torch::empty({llmt_qk_norm_rope_bwd_partials(T, H), HD}, x.options().dtype(torch::kFloat));
     pp = part.data_ptr<float>();
-    dwp = dw.data_ptr<float>();
+    if (dw_bf16) dw16 = dw.data_ptr();
+    else dwp = dw.data_ptr<float>();
   }
   check_rc(llmt_qk_norm_rope_bwd(dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), wp, cosb.data_ptr<float>(),
-                                 sinb.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(), dx.stride(0), pp, dwp, nullptr,
+                                 sinb.data_ptr<float>(), rstd.data_ptr<float>(), dx.data_ptr(), dx.stride(0), pp, dwp, dw16,
                                  0, T, H, HD, cur_stream()),
            "llmt_qk_norm_rope_bwd", w.has_value() ? 2 : 1);
   if (w.has_value()) return {dx, dw};
@@ -702,9 +707,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("grouped_gemm", &grouped_gemm);
   m.def("grouped_wgrad", &grouped_wgrad);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"), py::arg("dres"), py::arg("dw_bf16") = false);
   m.def("qk_norm_rope_fwd", &qk_norm_rope_fwd);
-  m.def("qk_norm_rope_bwd", &qk_norm_rope_bwd);
+  m.def("qk_norm_rope_bwd", &qk_norm_rope_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("cos"), py::arg("sin"), py::arg("rstd"),
+        py::arg("dw_bf16") = false);
   m.def("attn_rows_probs", &attn_rows_probs);
   m.def("attn_rows_ds", &attn_rows_ds);
   m.def("swiglu_fwd", &swiglu_fwd, py::arg("gate"), py::arg("up"), py::arg("row_limit") = py::none());

@@ -3,6 +3,7 @@
 // deterministic squared-norm. bf16 storage, fp32 math, 16-byte vector accesses.
 // (reference call sites: llmtuner/models/qwen/ops.py:80-131,503; llmtuner/components/loss.py:35-70;
 //  llmtuner/components/optimizer/optimizer.py:62-106; llmtuner/accelerator/collectives.py:290-558)
+#include <type_traits>
 #include "common.cuh"
 #include "kernels.h"
 
@@ -51,21 +52,60 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
 }
 
 // ------------------------------------------------------------------------------------------ RMSNorm
+// A row is owned by TR threads (a warp up to the whole block), each holding NV groups of 8 columns:
+// col = (v * TR + t) * 8, so that narrow rows (a 512-wide model: 64 vectors) leave no thread idle. Bound by memory; TR is the
+// smallest group that covers the row with NV = 2 (two 16-byte loads per operand in flight per thread, TR = 32 needs no barrier).
+// The forward gives a group a block of its own (or a warp of an eight-row block): named barriers with a computed id reserve
+// all sixteen of a block and then only four blocks fit an SM (57 us against 42 us at 8192 x 4096). The backward, which has two
+// blocks per SM anyway, puts 256 / TR groups into a block to keep the number of weight-gradient partials down.
+// 8192 x 4096 bf16 with the residual: forward 42 us, backward 50 us + 3.5 us for the column sums (before: 95 + 14 us, one row
+// after another without the prefetch); the 268 MB that each reads and writes take 42 us at copy speed.
+template <int TR, bool ONE_GROUP>
+__device__ __forceinline__ float row_sum(float v, float* red, int& buf) {
+  v = warp_sum(v);
+  if constexpr (TR > 32) {
+    // one barrier per row: the partial sums alternate between two buffers, and no warp can be two rows ahead
+    constexpr int NW = TR / 32;
+    const int grp = threadIdx.x / TR, t = threadIdx.x % TR;
+    float* r = red + buf * ((TR > kRowThreads ? TR : kRowThreads) / 32) + grp * NW;
+    if ((t & 31) == 0) r[t >> 5] = v;
+    if constexpr (ONE_GROUP) __syncthreads();
+    else named_bar_sync(1 + grp, TR);
+    v = r[0];
+#pragma unroll
+    for (int i = 1; i < NW; ++i) v += r[i];
+    buf ^= 1;
+  }
+  return v;
+}
+__device__ __forceinline__ void unpack8(const uint4& u, float* f) {
+  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 t = __bfloat1622float2(b[j]);
+    f[2 * j] = t.x;
+    f[2 * j + 1] = t.y;
+  }
+}
+
 // y = (x [+ res]) * rsqrt(mean((x+res)^2) + eps) * w ; optionally writes s = x + res (the new residual stream).
-template <int NV>  // each thread owns NV groups of 8 columns: col = (v * kRowThreads + tid) * 8
-__global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
+template <int NV, int TR>
+__global__ void __launch_bounds__(TR > 32 ? TR : kRowThreads) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                                   const __nv_bfloat16* __restrict__ res,
                                                                   const __nv_bfloat16* __restrict__ w,
                                                                   __nv_bfloat16* __restrict__ y,
                                                                   __nv_bfloat16* __restrict__ sum_out,
                                                                   float* __restrict__ rstd, int T, int D, float eps) {
-  __shared__ float red[32];
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
+  __shared__ float red[2 * (kRowThreads / 32)];
+  constexpr int RPB = TR > 32 ? 1 : kRowThreads / TR;
+  const int t = threadIdx.x % TR;
+  int buf = 0;
+  for (int row = blockIdx.x * RPB + threadIdx.x / TR; row < T; row += gridDim.x * RPB) {
     float v[NV][8];
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int col = (i * kRowThreads + threadIdx.x) * 8;
+      const int col = (i * TR + t) * 8;
       if (col < D) {
         load8(x + (int64_t)row * D + col, v[i]);
         if (res != nullptr) {
@@ -79,12 +119,12 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfl
         for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
       }
     }
-    ss = block_sum(ss, red);
+    ss = row_sum<TR, true>(ss, red, buf);
     const float r = rsqrtf(ss / (float)D + eps);
-    if (threadIdx.x == 0 && rstd != nullptr) rstd[row] = r;
+    if (t == 0 && rstd != nullptr) rstd[row] = r;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int col = (i * kRowThreads + threadIdx.x) * 8;
+      const int col = (i * TR + t) * 8;
       if (col < D) {
         float wv[8], o[8];
         load8(w + col, wv);
@@ -97,82 +137,136 @@ __global__ void __launch_bounds__(kRowThreads) rmsnorm_fwd_kernel(const __nv_bfl
 }
 
 // dx = r * (g - x * r^2 * mean(g * x)) [+ dres], g = dy * w ; dw partial per block = sum_rows dy * x * r.
-template <int NV>
-__global__ void __launch_bounds__(kRowThreads) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                                  const __nv_bfloat16* __restrict__ x,
-                                                                  const __nv_bfloat16* __restrict__ w,
-                                                                  const float* __restrict__ rstd,
-                                                                  const __nv_bfloat16* __restrict__ dres,
-                                                                  __nv_bfloat16* __restrict__ dx,
-                                                                  float* __restrict__ dw_partial, int T, int D) {
-  __shared__ float red[32];
+// Bound by memory (x, dy, dres read, dx written). The weight gradient stays in registers over all rows of the block, so
+// there are only 512 threads per SM; the operands of the next row are fetched before the reduction of this one, which keeps
+// loads in flight across the barrier.
+template <int TR>
+struct RowBlock { static constexpr int kThreads = TR > kRowThreads ? TR : kRowThreads, kRows = kThreads / TR; };
+
+template <int NV, int TR>
+__global__ void __launch_bounds__(RowBlock<TR>::kThreads, 512 / RowBlock<TR>::kThreads) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
+                                                                     const __nv_bfloat16* __restrict__ x,
+                                                                     const __nv_bfloat16* __restrict__ w,
+                                                                     const float* __restrict__ rstd,
+                                                                     const __nv_bfloat16* __restrict__ dres,
+                                                                     __nv_bfloat16* __restrict__ dx,
+                                                                     float* __restrict__ dw_partial, int T, int D) {
+  constexpr int NT = RowBlock<TR>::kThreads, RPB = RowBlock<TR>::kRows;
+  __shared__ float red[2 * (NT / 32)];
+  __shared__ float parts[RPB > 1 ? RPB * NV * TR * 8 : 1];
+  const int t = threadIdx.x % TR, grp = threadIdx.x / TR;
+  int buf = 0;
   float dw[NV][8];
-  float wv[NV][8];
+  uint4 wr[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int col = (i * kRowThreads + threadIdx.x) * 8;
+    const int col = (i * TR + t) * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { dw[i][j] = 0.f; wv[i][j] = 0.f; }
-    if (col < D) load8(w + col, wv[i]);
+    for (int j = 0; j < 8; ++j) dw[i][j] = 0.f;
+    wr[i] = col < D ? *reinterpret_cast<const uint4*>(w + col) : make_uint4(0, 0, 0, 0);
   }
-  for (int row = blockIdx.x; row < T; row += gridDim.x) {
-    float xv[NV][8], g[NV][8];
-    const float r = rstd[row];
+  const int step = gridDim.x * RPB;
+  uint4 xr[NV], dr[NV], er[NV];
+  float r = 0.f;
+  auto fetch = [&](int row, uint4* fx, uint4* fd, uint4* fe, float& fr) {
+    fr = rstd[row];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int col = (i * TR + t) * 8;
+      const int64_t at = (int64_t)row * D + col;
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      fx[i] = fd[i] = fe[i] = zero;
+      if (col < D) {
+        fx[i] = *reinterpret_cast<const uint4*>(x + at);
+        fd[i] = *reinterpret_cast<const uint4*>(dy + at);
+        if (dres != nullptr) fe[i] = *reinterpret_cast<const uint4*>(dres + at);
+      }
+    }
+  };
+  int row = blockIdx.x * RPB + grp;
+  if (row < T) fetch(row, xr, dr, er, r);
+  for (; row < T; row += step) {
     float c = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int col = (i * kRowThreads + threadIdx.x) * 8;
-      if (col < D) {
-        float d[8];
-        load8(x + (int64_t)row * D + col, xv[i]);
-        load8(dy + (int64_t)row * D + col, d);
+      float xv[8], d[8], wv[8];
+      unpack8(xr[i], xv); unpack8(dr[i], d); unpack8(wr[i], wv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          g[i][j] = d[j] * wv[i][j];
-          c += g[i][j] * xv[i][j];
-          dw[i][j] += d[j] * xv[i][j] * r;
-        }
+      for (int j = 0; j < 8; ++j) {
+        c += d[j] * wv[j] * xv[j];
+        dw[i][j] += d[j] * xv[j] * r;
       }
     }
-    c = block_sum(c, red);
+    uint4 nx[NV], nd[NV], ne[NV];
+    float nr = 0.f;
+    if (row + step < T) fetch(row + step, nx, nd, ne, nr);
+    c = row_sum<TR, (RPB == 1)>(c, red, buf);
     const float k = r * r * r * c / (float)D;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int col = (i * kRowThreads + threadIdx.x) * 8;
+      const int col = (i * TR + t) * 8;
       if (col < D) {
-        float o[8];
+        float xv[8], d[8], wv[8], e[8], o[8];
+        unpack8(xr[i], xv); unpack8(dr[i], d); unpack8(wr[i], wv); unpack8(er[i], e);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = r * g[i][j] - xv[i][j] * k;
+        for (int j = 0; j < 8; ++j) o[j] = r * (d[j] * wv[j]) - xv[j] * k;
         if (dres != nullptr) {
-          float e[8];
-          load8(dres + (int64_t)row * D + col, e);
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += e[j];
         }
         store8(dx + (int64_t)row * D + col, o);
       }
     }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) { xr[i] = nx[i]; dr[i] = nd[i]; er[i] = ne[i]; }
+    r = nr;
   }
+  if constexpr (RPB > 1) {                         // the row groups of the block, added in a fixed order
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int col = (i * kRowThreads + threadIdx.x) * 8;
-    if (col < D) {
-      float* p = dw_partial + (int64_t)blockIdx.x * D + col;
+    for (int i = 0; i < NV; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) p[j] = dw[i][j];
+      for (int j = 0; j < 8; ++j) parts[grp * (NV * TR * 8) + (i * TR + t) * 8 + j] = dw[i][j];
+    __syncthreads();
+    for (int c = threadIdx.x; c < D; c += NT) {
+      float s = 0.f;
+#pragma unroll
+      for (int g = 0; g < RPB; ++g) s += parts[g * (NV * TR * 8) + c];
+      dw_partial[(int64_t)blockIdx.x * D + c] = s;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int col = (i * TR + t) * 8;
+      if (col < D) {
+        float4* p = reinterpret_cast<float4*>(dw_partial + (int64_t)blockIdx.x * D + col);
+        p[0] = make_float4(dw[i][0], dw[i][1], dw[i][2], dw[i][3]);
+        p[1] = make_float4(dw[i][4], dw[i][5], dw[i][6], dw[i][7]);
+      }
     }
   }
 }
 
-// out[c] (+)= sum_p partial[p][c]
-__global__ void colsum_kernel(const float* __restrict__ partial, float* __restrict__ out_f32,
-                              __nv_bfloat16* __restrict__ out_bf16, int P, int D, int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= D) return;
+// out[c] (+)= sum_p partial[p][c]. A block owns 32 columns; its 32 warps take every 32nd partial row (one 128-byte line
+// each) and the 32 sums of a column are added in a fixed order. One thread per column (the earlier form) was a chain of up
+// to 592 dependent loads in as few as one block: 10-15 us per call, now 3 us.
+__global__ void __launch_bounds__(1024) colsum_kernel(const float* __restrict__ partial, float* __restrict__ out_f32,
+                                                      __nv_bfloat16* __restrict__ out_bf16, int P, int D, int accumulate) {
+  __shared__ float part[32][33];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int p = 0; p < P; ++p) s += partial[(int64_t)p * D + c];
-  if (out_f32 != nullptr) out_f32[c] = accumulate ? out_f32[c] + s : s;
-  if (out_bf16 != nullptr) out_bf16[c] = __float2bfloat16_rn(accumulate ? __bfloat162float(out_bf16[c]) + s : s);
+  if (c < D) {
+#pragma unroll 4
+    for (int p = wid; p < P; p += 32) s += partial[(int64_t)p * D + c];
+  }
+  part[wid][lane] = s;
+  __syncthreads();
+  s = warp_sum(part[lane][wid]);                   // warp w adds the 32 sums of column w
+  const int oc = blockIdx.x * 32 + wid;
+  if (lane == 0 && oc < D) {
+    if (out_f32 != nullptr) out_f32[oc] = accumulate ? out_f32[oc] + s : s;
+    if (out_bf16 != nullptr) out_bf16[oc] = __float2bfloat16_rn(accumulate ? __bfloat162float(out_bf16[oc]) + s : s);
+  }
 }
 
 // ------------------------------------------------------------------------------------------ QK-norm + RoPE
@@ -591,17 +685,28 @@ using namespace llmt;
 
 #define LLMT_CHECK_LAUNCH() return (cudaGetLastError() == cudaSuccess) ? 0 : -3
 
+// The row kernels by width: the smallest thread group that covers a row with two vectors per thread. WIDE is the pair for
+// rows above 4096: the forward takes four vectors on 256 threads, the backward (which would spill) two on 512.
+template <int WIDE_NV, int WIDE_TR, typename F>
+static inline void by_row_width(int D, F&& f) {
+  if (D <= 512) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 32>{});
+  else if (D <= 1024) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 64>{});
+  else if (D <= 2048) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 128>{});
+  else if (D <= 4096) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 256>{});
+  else f(std::integral_constant<int, WIDE_NV>{}, std::integral_constant<int, WIDE_TR>{});
+}
+
 extern "C" int llmt_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* sum_out, float* rstd, int T,
                                 int D, float eps, cudaStream_t st) {
   if (T <= 0) return 0;
   if (D % 8 || D > 8 * kRowThreads * 4) return -10;
-  const int nv = (D + 8 * kRowThreads - 1) / (8 * kRowThreads);
-  const int grid = T < sm_count() * 8 ? T : sm_count() * 8;
   auto X = (const __nv_bfloat16*)x; auto R = (const __nv_bfloat16*)res; auto W = (const __nv_bfloat16*)w;
   auto Y = (__nv_bfloat16*)y; auto S = (__nv_bfloat16*)sum_out;
-  if (nv == 1) rmsnorm_fwd_kernel<1><<<grid, kRowThreads, 0, st>>>(X, R, W, Y, S, rstd, T, D, eps);
-  else if (nv == 2) rmsnorm_fwd_kernel<2><<<grid, kRowThreads, 0, st>>>(X, R, W, Y, S, rstd, T, D, eps);
-  else rmsnorm_fwd_kernel<4><<<grid, kRowThreads, 0, st>>>(X, R, W, Y, S, rstd, T, D, eps);
+  by_row_width<4, 256>(D, [&](auto nv, auto tr) {
+    constexpr int TR = decltype(tr)::value, NT = TR > 32 ? TR : kRowThreads, RPB = NT / TR;
+    const int blocks = (T + RPB - 1) / RPB, cap = sm_count() * (2048 / NT);
+    rmsnorm_fwd_kernel<decltype(nv)::value, TR><<<blocks < cap ? blocks : cap, NT, 0, st>>>(X, R, W, Y, S, rstd, T, D, eps);
+  });
   LLMT_CHECK_LAUNCH();
 }
 
@@ -616,14 +721,16 @@ extern "C" int llmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
                                 cudaStream_t st) {
   if (T <= 0) return 0;
   if (D % 8 || D > 8 * kRowThreads * 4) return -10;
-  const int nv = (D + 8 * kRowThreads - 1) / (8 * kRowThreads);
-  const int grid = llmt_rmsnorm_bwd_partials(T);
   auto DY = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
   auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
-  if (nv == 1) rmsnorm_bwd_kernel<1><<<grid, kRowThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_partial, T, D);
-  else if (nv == 2) rmsnorm_bwd_kernel<2><<<grid, kRowThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_partial, T, D);
-  else rmsnorm_bwd_kernel<4><<<grid, kRowThreads, 0, st>>>(DY, X, W, rstd, DR, DX, dw_partial, T, D);
-  colsum_kernel<<<(D + 255) / 256, 256, 0, st>>>(dw_partial, dw_f32, (__nv_bfloat16*)dw_bf16, grid, D, accumulate);
+  int grid = 0;
+  by_row_width<2, 512>(D, [&](auto nv, auto tr) {
+    constexpr int NV = decltype(nv)::value, TR = decltype(tr)::value, NT = RowBlock<TR>::kThreads, RPB = RowBlock<TR>::kRows;
+    const int blocks = (T + RPB - 1) / RPB, most = llmt_rmsnorm_bwd_partials(T), cap = NT > 256 ? (most + 1) / 2 : most;
+    grid = blocks < cap ? blocks : cap;
+    rmsnorm_bwd_kernel<NV, TR><<<grid, NT, 0, st>>>(DY, X, W, rstd, DR, DX, dw_partial, T, D);
+  });
+  colsum_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_partial, dw_f32, (__nv_bfloat16*)dw_bf16, grid, D, accumulate);
   LLMT_CHECK_LAUNCH();
 }
 
@@ -665,7 +772,7 @@ extern "C" int llmt_qk_norm_rope_bwd(const void* dy, int64_t dy_tok_stride, cons
   else if (HD == 256) qk_norm_rope_bwd_kernel<4><<<grid, 256, 0, st>>>(DY, dy_tok_stride, X, tok_stride, W, cosb, sinb, rstd, DX, dx_tok_stride, dw_partial, T, H);
   else return -10;
   if (w != nullptr && dw_partial != nullptr)
-    colsum_kernel<<<(HD + 255) / 256, 256, 0, st>>>(dw_partial, dw_f32, (__nv_bfloat16*)dw_bf16, grid, HD, accumulate);
+    colsum_kernel<<<(HD + 31) / 32, 1024, 0, st>>>(dw_partial, dw_f32, (__nv_bfloat16*)dw_bf16, grid, HD, accumulate);
   LLMT_CHECK_LAUNCH();
 }
 

@@ -239,8 +239,8 @@ class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
-        dx, dw = _ext().rmsnorm_bwd(_c(dy), x, w, rstd, None)
-        return dx, dw.to(w.dtype), None
+        dx, dw = _ext().rmsnorm_bwd(_c(dy), x, w, rstd, None, True)        # the weight is bf16: the forward checked it
+        return dx, dw, None
 
 
 class _AddRMSNorm(torch.autograd.Function):
@@ -253,8 +253,8 @@ class _AddRMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, ds):
         s, w, rstd = ctx.saved_tensors
-        dsum, dw = _ext().rmsnorm_bwd(_c(dy), s, w, rstd, _c(ds) if ds is not None else None)
-        return dsum, dsum, dw.to(w.dtype), None
+        dsum, dw = _ext().rmsnorm_bwd(_c(dy), s, w, rstd, _c(ds) if ds is not None else None, True)
+        return dsum, dsum, dw, None
 
 
 def rms_norm(x, weight, eps: float):
@@ -288,7 +288,7 @@ class _QKNormRope(torch.autograd.Function):
         x, w, cos, sin, rstd = ctx.saved_tensors
         if dy.stride(2) != 1 or dy.stride(1) != dy.shape[2]:
             dy = dy.contiguous()
-        out = _ext().qk_norm_rope_bwd(dy, x, w if ctx.has_w else None, cos, sin, rstd)
+        out = _ext().qk_norm_rope_bwd(dy, x, w if ctx.has_w else None, cos, sin, rstd, ctx.has_w and w.dtype == torch.bfloat16)
         return out[0], (out[1].to(w.dtype) if ctx.has_w else None), None, None, None
 
 
