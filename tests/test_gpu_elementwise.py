@@ -208,3 +208,17 @@ def test_rmsnorm_at_the_edges_of_the_row_groups(T, D):
     y, rstd, s = load().rmsnorm_fwd(x, r, w, 1e-6)
     _, dw32 = load().rmsnorm_bwd(dy, s, w, rstd, ds)
     assert torch.equal(dw32.bfloat16(), got[2])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [1, 7, 8, 255, 257, 4097, 303104, 303105, 5000003, 20000008])
+def test_sq_norm_has_the_same_bits_on_any_alignment(n, dtype):
+    """The kernel for 16-byte aligned data and the one for any slice add the same terms in the same order: equal bits. Thousands of
+    fp32 terms per partial sum stay within 1e-5 of the 64-bit sum."""
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(n)
+    x = torch.randn(n, device="cuda").to(dtype)
+    moved = torch.empty(n + 1, device="cuda", dtype=dtype)[1:].copy_(x)
+    got, want = ops.sq_norm([x]), x.double().square().sum()
+    assert torch.equal(got, ops.sq_norm([moved]))
+    assert abs(float(got) - float(want)) <= 1e-5 * float(want)

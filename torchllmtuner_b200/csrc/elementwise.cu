@@ -654,6 +654,72 @@ __global__ void __launch_bounds__(256) sqnorm_partial_kernel(const T* __restrict
   s = block_sum(s, red);
   if (threadIdx.x == 0) scratch[blockIdx.x] = s;
 }
+// Streaming 16-byte load that stays where it is written: a batch of them is in flight before the first result is used (left to
+// itself the compiler folds each load into the chain of additions and keeps two in flight).
+__device__ __forceinline__ uint4 ld_stream(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// The same sums, bit for bit, from 16-byte loads (x on a 16-byte boundary): a warp stands for one block of the kernel above and a
+// lane for eight of its neighbouring threads, whose private sums it keeps apart; the shuffles then pair the sums exactly as
+// that block's reduction does (a warp of the block is four lanes here). Bound by memory; 256 bytes in flight per
+// thread make up for the eight warps per SM. 193 M bf16 values: 67 us against 114 us (60 us at copy speed; with a launch bound that let ptxas keep only two loads in flight: 159 us). Results keep
+// their bits because a clip coefficient off by one part in 1e7 already moves bf16 parameters that lie between two values.
+template <typename T>
+__global__ void __launch_bounds__(256, 1) sqnorm_partial_vec_kernel(const T* __restrict__ x, int64_t n, int nblocks, float* __restrict__ scratch) {
+  constexpr int kWords = sizeof(T) == 2 ? 1 : 2, U = sizeof(T) == 2 ? 16 : 8;
+  const int lane = threadIdx.x & 31, vb = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (vb >= nblocks) return;
+  const int64_t nt = (int64_t)nblocks * 256;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  auto add = [&](const uint4* u) {
+    float f[8];
+    if constexpr (kWords == 1) unpack8(u[0], f);
+    else {
+      f[0] = __uint_as_float(u[0].x); f[1] = __uint_as_float(u[0].y); f[2] = __uint_as_float(u[0].z); f[3] = __uint_as_float(u[0].w);
+      f[4] = __uint_as_float(u[1].x); f[5] = __uint_as_float(u[1].y); f[6] = __uint_as_float(u[1].z); f[7] = __uint_as_float(u[1].w);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] += f[e] * f[e];
+  };
+  int64_t i = (int64_t)vb * 256 + lane * 8;
+  for (; i + (U - 1) * nt + 8 <= n; i += U * nt) {
+    uint4 u[U][kWords];
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+#pragma unroll
+      for (int w = 0; w < kWords; ++w) u[k][w] = ld_stream(reinterpret_cast<const uint4*>(x + i + k * nt) + w);
+#pragma unroll
+    for (int k = 0; k < U; ++k) add(u[k]);
+  }
+  for (; i + 8 <= n; i += nt) {
+    uint4 u[kWords];
+#pragma unroll
+    for (int w = 0; w < kWords; ++w) u[w] = ld_stream(reinterpret_cast<const uint4*>(x + i) + w);
+    add(u);
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (i + e < n) {
+      const float f = (float)x[i + e];
+      s[e] += f * f;
+    }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);
+    s[e] += __shfl_xor_sync(0xffffffffu, s[e], 1);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (e < o) s[e] += s[e + o];
+  float t = s[0];
+#pragma unroll
+  for (int o = 16; o >= 4; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) scratch[vb] = t;
+}
 __global__ void __launch_bounds__(256) sqnorm_final_kernel(const float* __restrict__ scratch, int nparts,
                                                            float* __restrict__ out, int accumulate) {
   __shared__ float red[32];
@@ -844,7 +910,10 @@ extern "C" int llmt_sqnorm(const void* x, int is_bf16, int64_t n, float* scratch
     return 0;
   }
   const int grid = grid_for(n, 256);
-  if (is_bf16) sqnorm_partial_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, n, scratch);
+  if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    if (is_bf16) sqnorm_partial_vec_kernel<__nv_bfloat16><<<(grid + 7) / 8, 256, 0, st>>>((const __nv_bfloat16*)x, n, grid, scratch);
+    else sqnorm_partial_vec_kernel<float><<<(grid + 7) / 8, 256, 0, st>>>((const float*)x, n, grid, scratch);
+  } else if (is_bf16) sqnorm_partial_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, n, scratch);
   else sqnorm_partial_kernel<float><<<grid, 256, 0, st>>>((const float*)x, n, scratch);
   sqnorm_final_kernel<<<1, 256, 0, st>>>(scratch, grid, out, accumulate);
   LLMT_CHECK_LAUNCH();
