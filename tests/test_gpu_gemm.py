@@ -174,3 +174,32 @@ def test_projections_of_the_same_rows_sum_their_input_gradient_in_the_epilogue()
     assert (got[0].float() - x.grad.float()).abs().max() <= 0.02 * ref_dx.abs().max()
     for a, w in zip(got[1:], ws):
         assert torch.equal(a, w.grad)
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 264, 8), (256, 256, 64), (257, 1000, 72), (511, 136, 4104), (3001, 520, 200), (640, 19000, 136)])
+@pytest.mark.parametrize("layout", ["tn", "nn", "tt"])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gemm_pair_tiles(M, N, K, layout, accumulate):
+    """More than 128 rows: tiles of 256 x 256 on pairs of CTAs, where the second CTA's rows, the tile's columns or the last
+    k-block may lie outside the product; with accumulation the epilogue reads clamped addresses. A strided output off the 16-byte
+    grid takes the element-wise epilogue. Same bounds as the other layouts' tests; adding bf16 C costs one more rounding."""
+    from torchllmtuner_b200.ops import gemm
+    from torchllmtuner_b200.ops.cuda_ext import check_status
+    torch.manual_seed(M + N)
+    A, B = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    a = A.t().contiguous() if layout == "tt" and M % 8 == 0 else A
+    a_mn = layout == "tt" and M % 8 == 0
+    b = B if layout == "tn" else B.t().contiguous()
+    b_mn = layout != "tn"
+    ref = A.float() @ B.float().t()
+    for dtype, off in ((torch.bfloat16, 0), (torch.float32, 0), (torch.bfloat16, 3)):
+        if accumulate and (not b_mn or (dtype == torch.float32 and not a_mn)):
+            continue                                  # not one of the linear layer's products
+        big = torch.randn(M + 2, N + 8 + off, device="cuda").to(dtype)
+        keep = big.clone()
+        out = big[1:M + 1, off:off + N]
+        gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, accumulate=accumulate)
+        check_status("gemm")
+        _close(out.contiguous(), ref + keep[1:M + 1, off:off + N].float() if accumulate else ref)
+        big[1:M + 1, off:off + N] = keep[1:M + 1, off:off + N]
+        assert torch.equal(big, keep)                 # nothing outside the output was touched

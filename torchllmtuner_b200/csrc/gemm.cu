@@ -10,6 +10,7 @@
 //
 // CTA = 6 warps: warp 0 issues TMA, warp 1 owns TMEM and issues MMAs, warps 2-5 drain the accumulator.
 // The accumulator is double buffered in TMEM so the epilogue of tile i overlaps the MMAs of tile i+1.
+#include <type_traits>
 #include "comm.cuh"
 #include "kernels.h"
 
@@ -20,14 +21,19 @@ constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;                       // TMA warp, MMA warp, 4 epilogue warps
 constexpr int kGemmThreadsComm = 192 + kCommThreads;   // plus the comm warps that carry a SideJob
 
-template <int BN>
+// CG: CTAs that work on one tile. 1: a 128 x BN tile per CTA. 2: a 256 x BN tile per cluster of two CTAs (cta_group::2): each
+// CTA loads its 128 rows of A and its half of the B tile, the tensor cores of both SMs read both halves of B, and each CTA's
+// tensor memory receives its 128 rows of the product. See pick_tile() for when which is used.
+template <int CG, int BN>
 struct GemmCfg {
-  static constexpr int kStages = (BN == 256) ? 4 : 6;
+  static constexpr int kBRows = BN / CG;           // rows of B that this CTA loads
+  static constexpr int kStages = (kBRows == 256) ? 4 : 6;
   static constexpr int kABytes = BM * BK * 2;
-  static constexpr int kBBytes = BN * BK * 2;
+  static constexpr int kBBytes = kBRows * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kTmemCols = 2 * BN;  // two accumulators
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align slack*/ + 256 /*barriers*/;
+  static constexpr int kEpiBytes = 4 * 4096;  // staging of the epilogue: 32 rows of 128 bytes per warp
+  static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024 /*align slack*/ + 256 /*barriers*/;
 };
 
 struct GroupedArgs {
@@ -35,14 +41,16 @@ struct GroupedArgs {
   int num_groups;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE>
-__global__ void __launch_bounds__(kGemmThreadsComm, 1)
+template <int CG, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE>
+__global__ void __launch_bounds__(CG == 2 ? kGemmThreads : kGemmThreadsComm, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     void* __restrict__ Cptr, int M, int N, int K, int64_t ldc, GroupedArgs grp, SideJob side, TPFuse tp, int* status) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<CG, BN>;
+  static_assert(CG == 1 || MODE != 1, "segments are 128-row aligned: a 256-row tile would straddle them");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kStages * Cfg::kStageBytes);
+  uint8_t* epi = smem + Cfg::kStages * Cfg::kStageBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epi + Cfg::kEpiBytes);
   uint64_t* full = bars;
   uint64_t* empty = bars + Cfg::kStages;
   uint64_t* tfull = bars + 2 * Cfg::kStages;
@@ -53,6 +61,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  // In a pair the CTA of rank 0 leads: its full[] barriers count the bytes of both CTAs' loads, it alone issues the products,
+  // and its tempty[] barriers collect the epilogue threads of both. empty[] and tfull[] exist in both CTAs and are signalled
+  // together by the leader's commits.
+  const uint32_t rank = CG == 2 ? cluster_ctarank() : 0u;
+  const int unit = blockIdx.x / CG, num_units = gridDim.x / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) {
@@ -61,16 +74,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 128);
+      mbar_init(&tempty[a], CG * 128);
     }
     *abort_flag = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, Cfg::kTmemCols);
-    tmem_relinquish();
+    if constexpr (CG == 2) { tmem_alloc_pair(tmem_slot, Cfg::kTmemCols); tmem_relinquish_pair(); }
+    else { tmem_alloc(tmem_slot, Cfg::kTmemCols); tmem_relinquish(); }
   }
   tc_fence_before();
+  if constexpr (CG == 2) cluster_sync();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
@@ -83,7 +97,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int num_n = (N + BN - 1) / BN;
   // MODE 1: M is the capacity of the padded row buffer (a multiple of BM); only the tiles below the last segment's end
   // hold rows, the rest of a statically sized buffer is skipped.
-  int num_m = (M + BM - 1) / BM;
+  constexpr int TM = BM * CG;                      // rows of a tile
+  int num_m = (M + TM - 1) / TM;
   if constexpr (MODE == 1) {
     const int used = grp.seg_offsets[grp.num_groups] / BM;
     num_m = used < num_m ? used : num_m;
@@ -104,7 +119,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   // Tile order inside one M x N problem: super-rows of kGroupM m-tiles are swept column by column, so the CTAs that
   // run concurrently cover a near-square patch (A and B tiles are both reused out of L2).
-  constexpr int kGroupM = 16;
+  constexpr int kGroupM = 16 / CG;
   // With a fused tensor-parallel collective (MODE 0 only) the rows are walked chunk by chunk instead: the all-gather
   // form starts with this rank's own chunk, the reduce-scatter form ends with it.
   const bool tp_on = (MODE == 0) && tp.mode != kTPNone;
@@ -128,15 +143,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int first_m = grp_i * kGroupM;
     const int gm = (num_m - first_m < kGroupM) ? (num_m - first_m) : kGroupM;
     const int r = tt - grp_i * per_group;
-    m0 = (first_m + r % gm) * BM;
+    m0 = (first_m + r % gm) * TM + (int)rank * BM;        // this CTA's rows
     n0 = (r / gm) * BN;
   };
 
   auto group_of_row = [&](int row) -> int {
-    // segments are few (<= a few hundred); linear scan by one thread per tile is negligible
-    int g = 0;
-    while (g + 1 < grp.num_groups && row >= grp.seg_offsets[g + 1]) ++g;
-    return g;
+    // first segment that ends beyond `row`. A bisection: the producer thread looks it up for every tile, and a scan over 128
+    // segments (one dependent load each) took longer than the tile's loads could run ahead.
+    int lo = 0, hi = grp.num_groups - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (grp.seg_offsets[mid + 1] > row) hi = mid;
+      else lo = mid + 1;
+    }
+    return lo;
   };
 
   if (warp == 0) {
@@ -149,9 +169,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       uint32_t armed = 0, armed_parity = 0;  // per-stage bookkeeping for the abort drain
       bool ok = true;
       int landed_chunk = -1;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = unit; t < num_tiles && ok; t += num_units) {
         int m0, n0;
         tile_mn(t % tiles_per_group, m0, n0);
+        const int nb = n0 + (int)rank * Cfg::kBRows;        // this CTA's rows of the B tile
         if (tp_on && tp.mode == kTPAllGather) {
           const int c = tp_chunk_of(t);
           if (c != landed_chunk) {
@@ -170,10 +191,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
           uint8_t* sb = sa + Cfg::kABytes;
-          mbar_arrive_expect_tx(&full[stage], Cfg::kStageBytes);
-          armed |= 1u << stage;
-          armed_parity = (armed_parity & ~(1u << stage)) | (phase << stage);
+          if (rank == 0) {
+            mbar_arrive_expect_tx(&full[stage], CG * Cfg::kStageBytes);
+            armed |= 1u << stage;
+            armed_parity = (armed_parity & ~(1u << stage)) | (phase << stage);
+          }
           const int k0 = k_begin + kb * BK;
+          if constexpr (CG == 2) {
+            // a load of the second CTA may be counted before the leader has armed the phase: the transaction count may dip
+            // below zero meanwhile, and the leader's own arrival keeps the phase from completing
+            const uint32_t bar = cluster_map_u32(smem_u32(&full[stage]), 0);
+            if constexpr (!A_MN) tma_load_2d_pair(sa, &tmA, bar, k0, m0);
+            else {
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * (BK * 128), &tmA, bar, m0 + 64 * j, k0);
+            }
+            if constexpr (!B_MN) tma_load_2d_pair(sb, &tmB, bar, k0, nb);
+            else {
+#pragma unroll
+              for (int j = 0; j < Cfg::kBRows / 64; ++j) tma_load_2d_pair(sb + j * (BK * 128), &tmB, bar, nb + 64 * j, k0);
+            }
+            if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+            continue;
+          }
           if constexpr (!A_MN) {
             tma_load_2d(sa, &tmA, &full[stage], k0, m0);
           } else {
@@ -206,15 +246,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = umma_idesc_bf16(TM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        if (!mbar_wait_bounded(&tempty[acc], acc_phase ^ 1, abort_flag, status, 200 + acc)) break;
+      for (int t = unit; t < num_tiles && ok; t += num_units) {
+        if (!mbar_wait_bounded<CG == 2>(&tempty[acc], acc_phase ^ 1, abort_flag, status, 200 + acc)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         int k_begin;
@@ -233,13 +273,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t da = desc_pack(la + (A_MN ? k * 128 : k * 2));
             const uint64_t db = desc_pack(lb + (B_MN ? k * 128 : k * 2));
-            umma_bf16_ss(d_tmem, da, db, idesc, k ? 1u : acc0);
+            if constexpr (CG == 2) umma_bf16_ss_pair(d_tmem, da, db, idesc, k ? 1u : acc0);
+            else umma_bf16_ss(d_tmem, da, db, idesc, k ? 1u : acc0);
           }
-          umma_commit(&empty[stage]);  // frees the stage once these MMAs have read it
+          // frees the stage (of both CTAs) once these MMAs have read it
+          if constexpr (CG == 2) umma_commit_pair(&empty[stage]);
+          else umma_commit(&empty[stage]);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);
+        if constexpr (CG == 2) umma_commit_pair(&tfull[acc]);
+        else umma_commit(&tfull[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
@@ -254,88 +298,122 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // A thread reads one row of the accumulator, so storing from registers touches 32 rows per instruction with 16 bytes each.
+    // Every warp instead turns 32 rows x 128 bytes around in shared memory (16-byte chunks XORed with the row: no bank
+    // conflicts) and writes, and when accumulating reads, whole 128-byte lines. What is added is added in fp32.
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
+    uint8_t* stg = epi + quarter * 4096;
+    constexpr int kOutBytes = OUT_F32 ? 4 : 2;
+    constexpr bool kStageF32 = OUT_F32 || ACCUM;
+    constexpr int kChunk = kStageF32 ? 32 : 64;            // columns per 128-byte staging row
+    const bool vec_ok = ((reinterpret_cast<uintptr_t>(Cptr) | (uint64_t)(ldc * kOutBytes)) & 15) == 0;
+    const int rr0 = lane >> 3, cc = lane & 7;              // this lane's row (of every 4) and 16-byte chunk when reading back
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+    for (int t = unit; t < num_tiles; t += num_units) {
       int m0, n0;
       tile_mn(t % tiles_per_group, m0, n0);
       const int row_limit = M;  // MODE 1: padded rows are written too (their inputs are zero)
       int k_begin;
       const bool empty_k = kb_range(t, k_begin) == 0;  // MODE 2 segment without rows: the product is zero
       const int64_t c_base = (MODE == 2) ? (int64_t)(t / tiles_per_group) * M * ldc : 0;
+      const int row0 = m0 + quarter * 32;
+      if constexpr (ACCUM) {        // fetch this warp's rows of C into L2 while their product is still being computed
+        const int pr = min(row0 + lane, row_limit - 1);
+        const uint8_t* line = reinterpret_cast<const uint8_t*>(Cptr) + (c_base + (int64_t)pr * ldc + n0) * kOutBytes;
+        for (int o = 0; o < min(BN, N - n0) * kOutBytes; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + o));
+      }
       if (!mbar_wait_bounded(&tfull[acc], acc_phase, abort_flag, status, 400 + acc)) break;
       tc_fence_after();
-      const int row = m0 + quarter * 32 + lane;
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
+      const int n_chunks = (min(BN, N - n0) + kChunk - 1) / kChunk;
+      const bool tile_vec = vec_ok && ((c_base * kOutBytes) & 15) == 0;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(t_row + c * 32, r);
-        tmem_wait_ld();
-        if (empty_k) {
+      for (int c = 0; c < n_chunks; ++c) {
+        uint32_t r[kChunk];
+        tmem_ld_32x32(t_row + c * kChunk, r);
+        if constexpr (kChunk == 64) tmem_ld_32x32(t_row + c * kChunk + 32, r + 32);
+        const int col0 = n0 + c * kChunk;
+        if (tile_vec && (N & 7) == 0) {
+          constexpr int kPer = kStageF32 ? 4 : 8;          // columns per 16 staged bytes
+          const int col = col0 + cc * kPer;
+          const bool col_ok = col < N;
+          const int64_t at = c_base + (int64_t)(row0 + rr0) * ldc + col;
+          using OldT = typename std::conditional<OUT_F32, uint4, uint2>::type;
+          OldT old[8];                                     // what the product is added to: raw, converted where it is used
+          if constexpr (ACCUM) {
+            // clamped instead of skipped: eight unconditional loads are in flight together, a branch around each would
+            // leave them one after another
+            const int64_t cat = c_base + (col_ok ? col : n0);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = 0u;
-        }
-        const int col0 = n0 + c * 32;
-        if (row < row_limit && col0 < N) {
-          if constexpr (OUT_F32) {
-            float* dst = reinterpret_cast<float*>(Cptr) + c_base + (int64_t)row * ldc + col0;
-            if (col0 + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+            for (int it = 0; it < 8; ++it)
+              old[it] = *reinterpret_cast<const OldT*>(reinterpret_cast<const uint8_t*>(Cptr) +
+                                                       (cat + (int64_t)min(row0 + rr0 + it * 4, row_limit - 1) * ldc) * kOutBytes);
+          }
+          tmem_wait_ld();
+          if (empty_k) {
 #pragma unroll
-              for (int v = 0; v < 8; ++v) {
-                float4 o = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                       __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                if constexpr (ACCUM) {
-                  const float4 p = reinterpret_cast<float4*>(dst)[v];
-                  o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
-                }
-                reinterpret_cast<float4*>(dst)[v] = o;
+            for (int j = 0; j < kChunk; ++j) r[j] = 0u;
+          }
+          if constexpr (!kStageF32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = pack_bf16x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+          }
+          __syncwarp();                                    // the previous chunk has been read back by every lane
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int rr = it * 4 + rr0;
+            uint4 v = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((cc ^ (rr & 7)) << 4));
+            if (!(col_ok && row0 + rr < row_limit)) continue;
+            if constexpr (kStageF32) {
+              float4 o = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+              if constexpr (ACCUM && OUT_F32) {
+                o.x += __uint_as_float(old[it].x); o.y += __uint_as_float(old[it].y);
+                o.z += __uint_as_float(old[it].z); o.w += __uint_as_float(old[it].w);
+              } else if constexpr (ACCUM) {
+                const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old[it].x));
+                const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old[it].y));
+                o.x += a.x; o.y += a.y; o.z += b.x; o.w += b.y;
+              }
+              if constexpr (OUT_F32) {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(Cptr) + at + (int64_t)it * 4 * ldc) = o;
+              } else {
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(Cptr) + at + (int64_t)it * 4 * ldc) =
+                    make_uint2(pack_bf16x2(o.x, o.y), pack_bf16x2(o.z, o.w));
               }
             } else {
-              for (int j = 0; j < 32 && col0 + j < N; ++j) {
-                float o = __uint_as_float(r[j]);
-                if constexpr (ACCUM) o += dst[j];
-                dst[j] = o;
-              }
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(Cptr) + at + (int64_t)it * 4 * ldc) = v;
             }
-          } else {
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(Cptr) + c_base + (int64_t)row * ldc + col0;
-            if (col0 + 32 <= N && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+          }
+        } else {                                           // outputs off a 16-byte boundary, widths that are no multiple of 8
+          tmem_wait_ld();
+          const int row = row0 + lane;
+          if (row < row_limit) {
 #pragma unroll
-              for (int v = 0; v < 4; ++v) {
-                float f[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[8 * v + j]);
-                if constexpr (ACCUM) {
-                  const uint4 p = reinterpret_cast<const uint4*>(dst)[v];
-                  const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&p);
-#pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    const float2 pf = __bfloat1622float2(pb[j]);
-                    f[2 * j] += pf.x;
-                    f[2 * j + 1] += pf.y;
-                  }
-                }
-                uint4 o;
-                o.x = pack_bf16x2(f[0], f[1]);
-                o.y = pack_bf16x2(f[2], f[3]);
-                o.z = pack_bf16x2(f[4], f[5]);
-                o.w = pack_bf16x2(f[6], f[7]);
-                reinterpret_cast<uint4*>(dst)[v] = o;
-              }
-            } else {
-              for (int j = 0; j < 32 && col0 + j < N; ++j) {
-                float o = __uint_as_float(r[j]);
-                if constexpr (ACCUM) o += __bfloat162float(dst[j]);
-                dst[j] = __float2bfloat16_rn(o);
+            for (int j = 0; j < kChunk; ++j) {
+              if (col0 + j >= N) break;
+              const int64_t at = c_base + (int64_t)row * ldc + col0 + j;
+              float o = empty_k ? 0.f : __uint_as_float(r[j]);
+              if constexpr (OUT_F32) {
+                float* dst = reinterpret_cast<float*>(Cptr) + at;
+                if constexpr (ACCUM) o += *dst;
+                *dst = o;
+              } else {
+                __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(Cptr) + at;
+                if constexpr (ACCUM) o += __bfloat162float(*dst);
+                *dst = __float2bfloat16_rn(o);
               }
             }
           }
         }
       }
       tc_fence_before();
-      mbar_arrive(&tempty[acc]);
+      if constexpr (CG == 2) mbar_arrive_cluster(cluster_map_u32(smem_u32(&tempty[acc]), 0));
+      else mbar_arrive(&tempty[acc]);
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       if (tp_on && tp.mode == kTPReduceScatter) tp_tile_done(tp, tp_chunk_of(t), (uint32_t)tp_tpc * 4u, lane);
     }
@@ -343,9 +421,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   tc_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) cluster_sync();   // neither CTA leaves while the other's products or barriers still refer to it
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    if constexpr (CG == 2) tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
+    else tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
@@ -408,20 +488,45 @@ int sm_count() {
   return n;
 }
 
-template <int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE>
+// Whether a plain product takes pair tiles (256 x 256 on two SMs) or single ones (128 x 256 on one). Both give an SM the same
+// share of a full wave, so the one with fewer waves wins; at equal waves the pair is the faster one, because each SM reads
+// 8 KB instead of 12 KB of shared memory per 128 clocks of tensor work (single tiles measured 1.06 to 1.3 times the time:
+// 8192 x 12288 x 4096 504 us against 541 us, 8192 x 4096 x 4096 164 against 216, cuBLAS 529 and 176). At most 128 rows leave
+// the second CTA without work.
+static bool use_pair(int64_t M, int64_t N, int max_ctas) {
+  if (M <= BM || max_ctas == 1) return false;
+  const int64_t sms = sm_count(), n = (N + 255) / 256;
+  const int64_t pair = ((M + 255) / 256 * n + sms / 2 - 1) / (sms / 2), single = ((M + 127) / 128 * n + sms - 1) / sms;
+  return 100 * pair <= 107 * single;
+}
+
+template <int CG, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, int64_t ldc, GroupedArgs grp,
                   int* status, int max_ctas, cudaStream_t stream, const SideJob* side = nullptr, const TPFuse* tpf = nullptr) {
-  using Cfg = GemmCfg<BN>;
-  auto kern = gemm_tcgen05_kernel<BN, A_MN, B_MN, OUT_F32, ACCUM, MODE>;
+  using Cfg = GemmCfg<CG, BN>;
+  auto kern = gemm_tcgen05_kernel<CG, BN, A_MN, B_MN, OUT_F32, ACCUM, MODE>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return -2;
     configured = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * (MODE == 2 ? grp.num_groups : 1);
-  int grid = tiles < sm_count() ? tiles : sm_count();
-  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
+  const int tiles = ((M + BM * CG - 1) / (BM * CG)) * ((N + BN - 1) / BN) * (MODE == 2 ? grp.num_groups : 1);
+  int grid = tiles < sm_count() / CG ? tiles : sm_count() / CG;
+  if (max_ctas > 0 && grid > max_ctas / CG) grid = max_ctas / CG;
   if (grid < 1) return 0;
+  if constexpr (CG == 2) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid * 2);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, ta, tb, C, M, N, K, ldc, grp, SideJob{}, TPFuse{}, status) == cudaSuccess ? 0 : -3;
+  }
   SideJob none{};
   TPFuse no_tp{};
   const bool with_tp = tpf != nullptr && tpf->mode != kTPNone;
@@ -432,14 +537,14 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, 
   return (cudaGetLastError() == cudaSuccess) ? 0 : -3;
 }
 
-template <int BN>
+template <int CG, int BN>
 static int dispatch_plain(bool a_mn, bool b_mn, bool out_f32, bool accum, const CUtensorMap& ta, const CUtensorMap& tb,
                           void* C, int M, int N, int K, int64_t ldc, int* status, int max_ctas, cudaStream_t s,
                           const SideJob* side, const TPFuse* tpf = nullptr) {
   GroupedArgs grp{nullptr, 0};
 #define LLMT_CASE(AM, BMN, F32, ACC)                                                            \
   if (a_mn == AM && b_mn == BMN && out_f32 == F32 && accum == ACC)                              \
-    return launch<BN, AM, BMN, F32, ACC, 0>(ta, tb, C, M, N, K, ldc, grp, status, max_ctas, s, side, tpf);
+    return launch<CG, BN, AM, BMN, F32, ACC, 0>(ta, tb, C, M, N, K, ldc, grp, status, max_ctas, s, side, tpf);
   LLMT_CASE(false, false, false, false)
   LLMT_CASE(false, false, true, false)
   LLMT_CASE(false, true, false, false)
@@ -467,7 +572,9 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || (lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -10;
   const bool bn256 = N > 128;
-  const uint32_t bn = bn256 ? 256 : 128;
+  const bool fused = (side != nullptr && side->kind != kSideNone) || (tpf != nullptr && tpf->mode != kTPNone);
+  const bool pair = bn256 && !fused && use_pair(M, N, max_ctas);
+  const uint32_t bn = bn256 && !pair ? 256 : 128;          // rows of B per load
   CUtensorMap ta, tb;
   {
     uint64_t dims[2], str[1];
@@ -481,8 +588,9 @@ static int gemm_impl(const void* A, const void* B, void* C, int M, int N, int K,
     str[0] = (uint64_t)ldb * 2;
     if (make_tmap_bf16(&tb, B, 2, dims, str, box)) return -12;
   }
-  if (bn256) return dispatch_plain<256>(a_mn, b_mn, out_f32, accumulate, ta, tb, C, M, N, K, ldc, status, max_ctas, stream, side, tpf);
-  return dispatch_plain<128>(a_mn, b_mn, out_f32, accumulate, ta, tb, C, M, N, K, ldc, status, max_ctas, stream, side, tpf);
+  if (pair) return dispatch_plain<2, 256>(a_mn, b_mn, out_f32, accumulate, ta, tb, C, M, N, K, ldc, status, max_ctas, stream, nullptr);
+  if (bn256) return dispatch_plain<1, 256>(a_mn, b_mn, out_f32, accumulate, ta, tb, C, M, N, K, ldc, status, max_ctas, stream, side, tpf);
+  return dispatch_plain<1, 128>(a_mn, b_mn, out_f32, accumulate, ta, tb, C, M, N, K, ldc, status, max_ctas, stream, side, tpf);
 }
 
 extern "C" int llmt_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb,
@@ -562,11 +670,11 @@ extern "C" int llmt_grouped_gemm_bf16(const void* A, const void* B, void* C, con
   GroupedArgs grp{seg_offsets, num_groups};
   if (out_f32) return -4;
   if (bn256) {
-    if (b_mn) return launch<256, false, true, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
-    return launch<256, false, false, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
+    if (b_mn) return launch<1, 256, false, true, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
+    return launch<1, 256, false, false, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
   }
-  if (b_mn) return launch<128, false, true, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
-  return launch<128, false, false, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
+  if (b_mn) return launch<1, 128, false, true, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
+  return launch<1, 128, false, false, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
 }
 
 // Grouped wgrad: C[g] (M x N, row stride N) (+)= A_g^T * B_g where A is stored [rows][M], B is stored [rows][N] and
@@ -590,7 +698,7 @@ extern "C" int llmt_grouped_wgrad_bf16(const void* A, const void* B, void* C, co
   const int K = rows_padded;
 #define LLMT_W(BNV, F32, ACC) \
   if (bn256 == (BNV == 256) && (bool)out_f32 == F32 && (bool)accumulate == ACC) \
-    return launch<BNV, true, true, F32, ACC, 2>(ta, tb, C, M, N, K, (int64_t)N, grp, status, 0, stream);
+    return launch<1, BNV, true, true, F32, ACC, 2>(ta, tb, C, M, N, K, (int64_t)N, grp, status, 0, stream);
   LLMT_W(256, false, false) LLMT_W(256, true, false) LLMT_W(256, false, true) LLMT_W(256, true, true)
   LLMT_W(128, false, false) LLMT_W(128, true, false) LLMT_W(128, false, true) LLMT_W(128, true, true)
 #undef LLMT_W
