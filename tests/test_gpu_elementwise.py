@@ -222,3 +222,37 @@ def test_sq_norm_has_the_same_bits_on_any_alignment(n, dtype):
     got, want = ops.sq_norm([x]), x.double().square().sum()
     assert torch.equal(got, ops.sq_norm([moved]))
     assert abs(float(got) - float(want)) <= 1e-5 * float(want)
+
+
+@pytest.mark.parametrize("rows,V", [(1, 8), (3, 17), (5, 4096), (4, 8192), (4, 8208), (3, 20480), (3, 20520), (2, 76800), (2, 76808), (2, 151936)])
+@pytest.mark.parametrize("mask", [None, float("-inf"), torch.finfo(torch.bfloat16).min])
+def test_cross_entropy_kernel_at_its_size_limits(rows, V, mask):
+    """Both sides of each thread-count and shared-memory-cache limit, rows that end off a vector, labels in the last column, rows
+    without a label, and a masked stretch that covers whole threads. Gradients are one bf16 rounding of fp32 values."""
+    from torchllmtuner_b200.ops.cuda_ext import load
+    torch.manual_seed(V)
+    ld = -(-V // 8) * 8
+    x = torch.randn(rows, ld, device="cuda").mul_(3).bfloat16()[:, :V]
+    y = torch.randint(0, V, (rows,), device="cuda")
+    y[0] = V - 1
+    if rows > 2:
+        y[1] = -100
+    if mask is not None and V > 100:
+        x[:, : V // 2 // 8 * 8] = mask
+        y[2:] = V - 2
+    lf = x.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(lf, y, ignore_index=-100, reduction="none")
+    (dref,) = torch.autograd.grad(want.sum() * 0.5, lf)
+    loss, lse = load().ce_fwd_bwd(x, y, 0.5, None, -100, True)
+    assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
+    assert torch.allclose(lse.double(), lf.logsumexp(-1), rtol=1e-5, atol=1e-5)
+    _close(x, dref.float(), name="dlogits")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [1, 7, 8, 1000003])
+def test_scale_to_bf16(n, dtype):
+    from torchllmtuner_b200.ops.cuda_ext import load
+    torch.manual_seed(n)
+    x, g = torch.randn(n, device="cuda").to(dtype), torch.tensor(0.3, device="cuda")
+    assert torch.equal(load().scale_to_bf16(x, g), (x.float() * g).bfloat16())

@@ -463,6 +463,18 @@ std::vector<Tensor> ce_fwd_bwd(Tensor& logits, const Tensor& labels, double grad
   return {loss, lse};
 }
 
+// bf16(x * scale) in a new tensor; x contiguous fp32 or bf16, scale one fp32 value on the device.
+Tensor scale_to_bf16(const Tensor& x, const Tensor& scale) {
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16),
+              "x must be a contiguous fp32 or bf16 CUDA tensor");
+  TORCH_CHECK(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() == 1, "scale must be one fp32 value on the device");
+  Tensor out = torch::empty(x.sizes(), x.options().dtype(at::kBFloat16));
+  check_rc(llmt_scale_to_bf16(x.data_ptr(), x.scalar_type() == at::kBFloat16, scale.data_ptr<float>(), out.data_ptr(), x.numel(), cur_stream()),
+           "llmt_scale_to_bf16");
+  return out;
+}
+
 // Vocabulary-parallel cross-entropy over one shard of the logits [rows, V/R] (in place: the shard becomes its gradient);
 // `stats` / `flags` are every rank's statistics and flag tables in symmetric memory (device addresses).
 Tensor ce_vocab_parallel(Tensor& logits, const Tensor& labels, int64_t vocab_start, int64_t me, const std::vector<int64_t>& stats,
@@ -717,6 +729,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_bwd", &swiglu_bwd, py::arg("dout"), py::arg("gate"), py::arg("up"), py::arg("dgate_out"), py::arg("dup_out"),
         py::arg("row_limit") = py::none());
   m.def("ce_fwd_bwd", &ce_fwd_bwd);
+  m.def("scale_to_bf16", &scale_to_bf16);
   m.def("ce_vocab_parallel", &ce_vocab_parallel);
   m.def("vp_embed_scatter", &vp_embed_scatter);
   m.def("adamw", &adamw);

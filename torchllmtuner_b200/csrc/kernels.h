@@ -49,6 +49,7 @@ int llmt_swiglu_bwd(const void* dout, const void* gate, const void* up, void* dg
                     int64_t ld_in, int64_t ld_dout, int64_t ld_dg, const int* row_limit, cudaStream_t st);
 int llmt_ce_fwd_bwd(void* logits, const int64_t* labels, float* row_loss, float* row_lse, int rows, int V, int64_t ld,
                     const float* grad_scale_ptr, float grad_scale, int ignore_index, int write_grad, cudaStream_t st);
+int llmt_scale_to_bf16(const void* x, int is_bf16, const float* scale, void* out, int64_t n, cudaStream_t st);
 int llmt_adamw(float* p32, void* p16, const void* g, int g_is_bf16, float* m, float* v, int64_t n, float lr, float b1,
                float b2, float eps, float wd, int step, const float* clip_coef, float grad_scale, int decoupled,
                cudaStream_t st);

@@ -445,7 +445,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
         step = -(-step // 128) * 128
         need_dh, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
         dh = torch.empty_like(h) if need_dh else None
-        dw = torch.zeros(w.shape, dtype=torch.float32, device=w.device) if need_dw else None
+        # the first chunk's product overwrites the buffer, later ones add to it
+        dw = (torch.empty if T > 0 else torch.zeros)(w.shape, dtype=torch.float32, device=w.device) if need_dw else None
         loss = torch.zeros((), dtype=torch.float32, device=h.device)
         first = True
         for s in range(0, T, step):
@@ -467,7 +468,10 @@ class _LinearCrossEntropy(torch.autograd.Function):
     def backward(ctx, g):
         dh, dw = ctx.saved_tensors
         need_dh, need_dw, wdt = ctx.flags
-        return ((dh * g.to(dh.dtype)) if need_dh else None, ((dw * g).to(wdt)) if need_dw else None, None, None)
+        if torch.is_grad_enabled() or wdt != torch.bfloat16:        # create_graph: keep the expressions in the graph
+            return ((dh * g.to(dh.dtype)) if need_dh else None, ((dw * g).to(wdt)) if need_dw else None, None, None)
+        scale = _ext().scale_to_bf16
+        return scale(dh, g) if need_dh else None, scale(dw, g) if need_dw else None, None, None
 
 
 def linear_cross_entropy_sum(h, w, targets, num_chunks: int = 1):
@@ -487,7 +491,9 @@ class _CrossEntropySum(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (d,) = ctx.saved_tensors
-        return d * g.to(d.dtype), None
+        if torch.is_grad_enabled():
+            return d * g.to(d.dtype), None
+        return _ext().scale_to_bf16(d, g), None
 
 
 def cross_entropy_sum(logits, targets):
