@@ -75,3 +75,48 @@ def test_ep_plan_matches_stable_sort(n, E, R):
     pos = rank - start[flat]
     assert torch.equal(drow.long(), send_off.long()[flat] + pos)
     assert torch.equal(drank.long(), flat // (E // R))
+
+
+@pytest.mark.parametrize("n,E", [(0, 4), (1, 1), (5, 16), (1023, 8), (1024, 512), (1025, 100), (32768, 128), (70001, 3)])
+@pytest.mark.parametrize("skew", [False, True])
+def test_plan_segments_kernel_matches_tensor_statement(n, E, skew):
+    """The planning kernels against the tensor expressions of the CPU path: whole numbers, so equal."""
+    from torchllmtuner_b200.models.moe.experts import plan_segments
+    from torchllmtuner_b200.ops.cuda_ext import check_status
+    g = torch.Generator().manual_seed(n + E)
+    flat = torch.randint(0, E, (n,), generator=g)
+    if skew:
+        flat = torch.where(torch.rand(n, generator=g) < 0.9, torch.full_like(flat, E - 1), flat)
+    want = plan_segments(flat, E)
+    got = plan_segments(flat.cuda(), E)
+    check_status("moe_plan")
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
+
+
+@pytest.mark.parametrize("T,E,k,D,F_", [(3, 16, 2, 8, 64), (130, 8, 4, 264, 72), (257, 32, 8, 512, 136), (65, 4, 1, 1032, 64)])
+def test_routed_experts_write_their_padding_rows(T, E, k, D, F_):
+    """Buffers are no longer cleared before use: the same call on poisoned memory gives finite results that match the CPU
+    statement, for narrow rows, a top-k that is no multiple of the combine's eight loads, and empty experts."""
+    from torchllmtuner_b200.models.moe.experts import GroupedExperts, RoutedExperts
+    torch.manual_seed(T)
+    gpu = RoutedExperts(GroupedExperts(E, D, F_, dtype=torch.bfloat16, device="cuda"))
+    cpu = RoutedExperts(GroupedExperts(E, D, F_, dtype=torch.float32))
+    for p, q in zip(gpu.parameters(), cpu.parameters()):
+        torch.nn.init.normal_(p, std=0.05)
+        q.data.copy_(p.detach().float().cpu())
+    x = torch.randn(T, D, device="cuda").bfloat16().requires_grad_()
+    w = torch.rand(T, k, device="cuda", requires_grad=True)
+    idx = torch.randint(0, E, (T, k), device="cuda")
+    xc, wc = x.detach().float().cpu().requires_grad_(), w.detach().cpu().requires_grad_()
+    go = torch.randn(T, D, device="cuda").bfloat16()
+    for _ in range(2):
+        junk = [torch.full((1 << 22,), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+        del junk                                          # the allocator hands this memory to the buffers of the call
+        yg = gpu(x, w, idx)
+        gg = torch.autograd.grad(yg, [x, w, *gpu.parameters()], go)
+    yc = cpu(xc, wc, idx.cpu())
+    gc = torch.autograd.grad(yc, [xc, wc, *cpu.parameters()], go.float().cpu())
+    for a, b in zip((yg, *gg), (yc, *gc)):
+        assert torch.isfinite(a).all()
+        _close(a, b.to("cuda"), 3e-2)

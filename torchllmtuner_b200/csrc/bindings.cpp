@@ -260,7 +260,7 @@ void wait_flags(int64_t flags_ptr, int64_t n, int64_t value, int64_t site, int64
            "llmt_wait_flags");
 }
 
-void grouped_gemm(const Tensor& a, const Tensor& b, Tensor& out, const Tensor& seg_offsets, bool b_mn) {
+void grouped_gemm(const Tensor& a, const Tensor& b, Tensor& out, const Tensor& seg_offsets, bool b_mn, bool accumulate) {
   c10::cuda::CUDAGuard guard(a.device());
   const Mat A = as_mat(a, "a");
   check_bf16(b, "b");
@@ -272,7 +272,7 @@ void grouped_gemm(const Tensor& a, const Tensor& b, Tensor& out, const Tensor& s
   const int64_t N = b_mn ? b.size(2) : b.size(1), K = b_mn ? b.size(1) : b.size(2);
   TORCH_CHECK(A.cols == K && out.size(0) == A.rows && out.size(1) == N && out.stride(1) == 1);
   check_rc(llmt_grouped_gemm_bf16(A.ptr, b.data_ptr(), out.data_ptr(), seg_offsets.data_ptr<int>(), G, (int)A.rows, (int)N,
-                                  (int)K, A.ld, out.stride(0), b_mn, 0, status_ptr(), cur_stream()),
+                                  (int)K, A.ld, out.stride(0), b_mn, 0, accumulate, status_ptr(), cur_stream()),
            "llmt_grouped_gemm_bf16");
 }
 
@@ -646,12 +646,42 @@ Tensor router_topk_bwd(const Tensor& logits, const Tensor& dw, const Tensor& idx
            "llmt_router_topk_bwd");
   return dl;
 }
-// rows must be zero-initialised by the caller (padding rows stay zero)
-void permute_rows(const Tensor& x, const Tensor& dest, Tensor& rows, int64_t k) {
+// flat [n] int64 expert ids -> (dest [n] int64 row of every copy, seg [E + 1] int32, counts [E] int64); copies of one expert
+// keep their order, every segment starts on a multiple of `align` rows.
+std::vector<Tensor> moe_plan(const Tensor& flat, int64_t E, int64_t align) {
+  c10::cuda::CUDAGuard guard(flat.device());
+  TORCH_CHECK(flat.is_cuda() && flat.scalar_type() == at::kLong && flat.is_contiguous(), "flat must be a contiguous int64 CUDA tensor");
+  const int64_t n = flat.numel();
+  Tensor dest = torch::empty({n}, flat.options()), counts = torch::empty({E}, flat.options());
+  Tensor ints = torch::empty({E + 1 + llmt_moe_plan_scratch_ints(n, (int)E)}, flat.options().dtype(torch::kInt));
+  Tensor seg = torch::empty({E + 1}, ints.options());
+  check_rc(llmt_moe_plan(flat.data_ptr<int64_t>(), n, (int)E, (int)align, ints.data_ptr<int>(), dest.data_ptr<int64_t>(), seg.data_ptr<int>(),
+                         counts.data_ptr<int64_t>(), status_ptr(), cur_stream()),
+           "llmt_moe_plan", 3);
+  return {dest, seg, counts};
+}
+struct Padding {
+  const int* seg = nullptr;
+  const int64_t* counts = nullptr;
+  int E = 0;
+};
+static Padding padding_of(const c10::optional<Tensor>& seg, const c10::optional<Tensor>& counts) {
+  if (!seg.has_value()) return {};
+  TORCH_CHECK(counts.has_value() && seg->is_cuda() && seg->scalar_type() == at::kInt && seg->is_contiguous() && counts->is_cuda() &&
+                  counts->scalar_type() == at::kLong && counts->is_contiguous() && seg->numel() == counts->numel() + 1,
+              "seg must be int32 [E + 1] and counts int64 [E]");
+  return {seg->data_ptr<int>(), counts->data_ptr<int64_t>(), (int)counts->numel()};
+}
+// Without seg / counts the rows must be zero-initialised by the caller; with them the padding rows are zeroed here.
+void permute_rows(const Tensor& x, const Tensor& dest, Tensor& rows, int64_t k, const c10::optional<Tensor>& seg,
+                  const c10::optional<Tensor>& counts) {
   c10::cuda::CUDAGuard guard(x.device());
-  check_bf16(x, "x"); check_bf16(rows, "rows");
+  check_bf16(x, "x");
+  check_bf16(rows, "rows");
   TORCH_CHECK(x.is_contiguous() && rows.is_contiguous() && dest.scalar_type() == at::kLong && dest.is_contiguous());
-  check_rc(llmt_permute_rows(x.data_ptr(), dest.data_ptr<int64_t>(), rows.data_ptr(), dest.numel(), (int)k, (int)x.size(1), cur_stream()),
+  const Padding pad = padding_of(seg, counts);
+  check_rc(llmt_permute_rows(x.data_ptr(), dest.data_ptr<int64_t>(), rows.data_ptr(), dest.numel(), (int)k, (int)x.size(1), pad.seg, pad.counts,
+                             pad.E, cur_stream()),
            "llmt_permute_rows");
 }
 Tensor combine_rows(const Tensor& y, const Tensor& dest, const c10::optional<Tensor>& w, int64_t T, int64_t k) {
@@ -664,13 +694,15 @@ Tensor combine_rows(const Tensor& y, const Tensor& dest, const c10::optional<Ten
            "llmt_combine_rows");
   return out;
 }
-std::vector<Tensor> combine_bwd(const Tensor& dout, const Tensor& y, const Tensor& dest, const Tensor& w, int64_t k) {
+std::vector<Tensor> combine_bwd(const Tensor& dout, const Tensor& y, const Tensor& dest, const Tensor& w, int64_t k,
+                                const c10::optional<Tensor>& seg, const c10::optional<Tensor>& counts) {
   c10::cuda::CUDAGuard guard(y.device());
-  Tensor dy = torch::zeros_like(y);
+  const Padding pad = padding_of(seg, counts);
+  Tensor dy = pad.seg != nullptr && dest.numel() > 0 ? torch::empty_like(y) : torch::zeros_like(y);
   Tensor dw = torch::empty({dest.numel()}, y.options().dtype(torch::kFloat));
   Tensor d = dout.contiguous();
   check_rc(llmt_combine_bwd(d.data_ptr(), y.data_ptr(), dest.data_ptr<int64_t>(), w.data_ptr<float>(), dy.data_ptr(), dw.data_ptr<float>(),
-                            dest.numel(), (int)k, (int)y.size(1), cur_stream()),
+                            dest.numel(), (int)k, (int)y.size(1), pad.seg, pad.counts, pad.E, cur_stream()),
            "llmt_combine_bwd");
   return {dy, dw};
 }
@@ -702,9 +734,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("accumulate") = false, py::arg("max_ctas") = 0, py::arg("side") = py::none());
   m.def("router_topk", &router_topk);
   m.def("router_topk_bwd", &router_topk_bwd);
-  m.def("permute_rows", &permute_rows);
+  m.def("moe_plan", &moe_plan);
+  m.def("permute_rows", &permute_rows, py::arg("x"), py::arg("dest"), py::arg("rows"), py::arg("k"), py::arg("seg") = py::none(),
+        py::arg("counts") = py::none());
   m.def("combine_rows", &combine_rows);
-  m.def("combine_bwd", &combine_bwd);
+  m.def("combine_bwd", &combine_bwd, py::arg("dout"), py::arg("y"), py::arg("dest"), py::arg("w"), py::arg("k"), py::arg("seg") = py::none(),
+        py::arg("counts") = py::none());
   m.def("gemm_tp", &gemm_tp, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("b_mn"), py::arg("accumulate"), py::arg("mode"), py::arg("world"),
         py::arg("rank"), py::arg("epoch"), py::arg("peer_src"), py::arg("flags"), py::arg("peer_flags"), py::arg("counters"),
         py::arg("acc") = py::none(), py::arg("out") = py::none(), py::arg("residual") = py::none());
@@ -716,7 +751,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("side_job", &side_job);
   m.def("signal_peers", &signal_peers);
   m.def("wait_flags", &wait_flags, py::arg("flags_ptr"), py::arg("n"), py::arg("value"), py::arg("site"), py::arg("max_polls") = 0);
-  m.def("grouped_gemm", &grouped_gemm);
+  m.def("grouped_gemm", &grouped_gemm, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("seg_offsets"), py::arg("b_mn"),
+        py::arg("accumulate") = false);
   m.def("grouped_wgrad", &grouped_wgrad);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"), py::arg("dres"), py::arg("dw_bf16") = false);

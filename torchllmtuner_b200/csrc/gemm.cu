@@ -646,12 +646,12 @@ extern "C" int llmt_gemm_bf16_tp(const void* A, const void* B, void* C, int M, i
 
 // Grouped forward/dgrad: rows of A (and C) are cut into `num_groups` segments at seg_offsets (device int32,
 // [G+1], multiples of 128, seg_offsets[G] == M_padded); segment g multiplies B[g].
-//   b_mn == 0: B stored [G][N][K];  b_mn == 1: B stored [G][K][N].
+//   b_mn == 0: B stored [G][N][K];  b_mn == 1: B stored [G][K][N] (with `accumulate`: C += ..., added in fp32).
 extern "C" int llmt_grouped_gemm_bf16(const void* A, const void* B, void* C, const int* seg_offsets, int num_groups,
-                                      int M_padded, int N, int K, int64_t lda, int64_t ldc, int b_mn, int out_f32,
+                                      int M_padded, int N, int K, int64_t lda, int64_t ldc, int b_mn, int out_f32, int accumulate,
                                       int* status, cudaStream_t stream) {
   if (M_padded <= 0 || N <= 0 || num_groups <= 0) return 0;
-  if (K <= 0 || (lda & 7) || (M_padded % BM)) return -10;
+  if (K <= 0 || (lda & 7) || (M_padded % BM) || (reinterpret_cast<uintptr_t>(A) & 15)) return -10;
   const bool bn256 = N > 128;
   const uint32_t bn = bn256 ? 256 : 128;
   CUtensorMap ta, tb;
@@ -668,7 +668,11 @@ extern "C" int llmt_grouped_gemm_bf16(const void* A, const void* B, void* C, con
     if (make_tmap_bf16(&tb, B, 3, dims, str, box)) return -12;
   }
   GroupedArgs grp{seg_offsets, num_groups};
-  if (out_f32) return -4;
+  if (out_f32 || (accumulate && !b_mn)) return -4;
+  if (accumulate) {                                    // dx += dy_i W_i of a second projection of the same rows
+    if (bn256) return launch<1, 256, false, true, false, true, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
+    return launch<1, 128, false, true, false, true, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
+  }
   if (bn256) {
     if (b_mn) return launch<1, 256, false, true, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);
     return launch<1, 256, false, false, false, false, 1>(ta, tb, C, M_padded, N, K, ldc, grp, status, 0, stream);

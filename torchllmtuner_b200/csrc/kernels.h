@@ -21,7 +21,7 @@ int llmt_gemm_bf16_tp(const void* A, const void* B, void* C, int M, int N, int K
                       const uint32_t* flags, uint32_t* const* peer_flags, uint32_t* counters, float* acc, void* out,
                       const void* residual, int* status, cudaStream_t stream);
 int llmt_grouped_gemm_bf16(const void* A, const void* B, void* C, const int* seg_offsets, int num_groups, int M_padded,
-                           int N, int K, int64_t lda, int64_t ldc, int b_mn, int out_f32, int* status,
+                           int N, int K, int64_t lda, int64_t ldc, int b_mn, int out_f32, int accumulate, int* status,
                            cudaStream_t stream);
 int llmt_grouped_wgrad_bf16(const void* A, const void* B, void* C, const int* seg_offsets, int num_groups,
                             int rows_padded, int M, int N, int64_t lda, int64_t ldb, int out_f32, int accumulate,
@@ -73,10 +73,14 @@ int llmt_router_topk(const float* logits, const float* bias, float* weights, int
                      int T, int E, int k, int score_fn, int renorm, float route_scale, cudaStream_t st);
 int llmt_router_topk_bwd(const float* logits, const float* dweights, const int64_t* indices, const float* denom, float* dlogits,
                          int T, int E, int k, int score_fn, int renorm, float route_scale, cudaStream_t st);
-int llmt_permute_rows(const void* x, const int64_t* dest, void* rows, int64_t ncopies, int k, int D, cudaStream_t st);
+int64_t llmt_moe_plan_scratch_ints(int64_t n, int E);
+int llmt_moe_plan(const int64_t* flat, int64_t n, int E, int align, int* hist, int64_t* dest, int* seg, int64_t* counts, int* status,
+                  cudaStream_t st);
+int llmt_permute_rows(const void* x, const int64_t* dest, void* rows, int64_t ncopies, int k, int D, const int* seg,
+                      const int64_t* counts, int E, cudaStream_t st);
 int llmt_combine_rows(const void* y, const int64_t* dest, const float* w, void* out, int T, int k, int D, cudaStream_t st);
 int llmt_combine_bwd(const void* dout, const void* y, const int64_t* dest, const float* w, void* dy, float* dw, int64_t ncopies,
-                     int k, int D, cudaStream_t st);
+                     int k, int D, const int* seg, const int64_t* counts, int E, cudaStream_t st);
 
 // ---- peer-memory communication (comm.cu) ----
 int llmt_side_job(int kind, int nsrc, const void* const* src, void* dst, long long n, int accumulate,

@@ -15,6 +15,7 @@ from ...ops import reference as ref
 from ...ops.cuda_ext import load as _ext
 
 SEG_ALIGN = 128
+PLAN_MAX_EXPERTS = 512      # of the planning kernels
 
 
 def padded_capacity(num_copies: int, num_experts: int) -> int:
@@ -25,7 +26,9 @@ def padded_capacity(num_copies: int, num_experts: int) -> int:
 
 def plan_segments(flat_expert: torch.Tensor, num_experts: int):
     """From the expert id of each token copy: (dest_row [n] int64 in the padded layout, seg_offsets [E+1] int32,
-    counts [E] int64). Pure device ops, no host synchronisation."""
+    counts [E] int64). Copies of one expert keep their order. On the device three kernels and no host synchronisation."""
+    if flat_expert.is_cuda and flat_expert.dtype == torch.int64 and 1 <= num_experts <= PLAN_MAX_EXPERTS:
+        return tuple(_ext().moe_plan(flat_expert.contiguous(), num_experts, SEG_ALIGN))
     counts = torch.bincount(flat_expert, minlength=num_experts)
     padded = (counts + (SEG_ALIGN - 1)) // SEG_ALIGN * SEG_ALIGN
     zero = counts.new_zeros(1)
@@ -38,33 +41,58 @@ def plan_segments(flat_expert: torch.Tensor, num_experts: int):
     return dest, seg.to(torch.int32), counts
 
 
+def _rows_view(t: torch.Tensor) -> torch.Tensor:
+    """`t` itself when the grouped kernels can read it (unit inner stride, rows and base on 16-byte boundaries), else a copy.
+    The gradients of gate and up are the two halves of one buffer: copying them cost as much as a grouped product."""
+    if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1] and t.data_ptr() % 16 == 0:
+        return t
+    return t.contiguous()
+
+
 class _GroupedLinear(torch.autograd.Function):
-    """y[seg g] = x[seg g] @ w[g]^T over 128-aligned row segments."""
+    """y_i[seg g] = x[seg g] @ w_i[g]^T over 128-aligned row segments, for one or more weights that read the same rows (gate and
+    up). The input gradient of the second weight is added by the product's epilogue (in fp32, one rounding) instead of by a
+    pass over two finished gradients."""
 
     @staticmethod
-    def forward(ctx, x, w, seg):
-        y = torch.empty(x.shape[0], w.shape[1], dtype=x.dtype, device=x.device)
-        _ext().grouped_gemm(x, w, y, seg, False)
-        ctx.save_for_backward(x, w, seg)
-        return y
+    def forward(ctx, x, seg, *ws):
+        ys = []
+        for w in ws:
+            ys.append(torch.empty(x.shape[0], w.shape[1], dtype=x.dtype, device=x.device))
+            _ext().grouped_gemm(x, w, ys[-1], seg, False)
+        ctx.save_for_backward(x, seg, *ws)
+        return tuple(ys) if len(ys) > 1 else ys[0]
 
     @staticmethod
-    def backward(ctx, dy):
-        x, w, seg = ctx.saved_tensors
-        dy = dy if dy.is_contiguous() else dy.contiguous()
-        dx = dw = None
-        if ctx.needs_input_grad[0]:
-            dx = torch.empty_like(x)
-            _ext().grouped_gemm(dy, w, dx, seg, True)
-        if ctx.needs_input_grad[1]:
-            dw = torch.empty_like(w)
-            _ext().grouped_wgrad(dy, x, dw, seg, False)
-        return dx, dw, None
+    def backward(ctx, *dys):
+        x, seg, *ws = ctx.saved_tensors
+        dx, dws = None, []
+        for i, (dy, w) in enumerate(zip(dys, ws)):
+            dy = _rows_view(dy)
+            if ctx.needs_input_grad[0]:
+                if dx is None:
+                    dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+                    _ext().grouped_gemm(dy, w, dx, seg, True)
+                else:
+                    _ext().grouped_gemm(dy, w, dx, seg, True, True)
+            if ctx.needs_input_grad[2 + i]:
+                dws.append(torch.empty_like(w))
+                _ext().grouped_wgrad(dy, x, dws[-1], seg, False)
+            else:
+                dws.append(None)
+        return (dx, None, *dws)
+
+
+def grouped_linears(x, seg_offsets, *ws):
+    """Several grouped projections of the same rows; one autograd node on the device."""
+    if x.is_cuda and x.dtype == torch.bfloat16:
+        return _GroupedLinear.apply(x, seg_offsets, *ws)
+    return tuple(grouped_linear(x, w, seg_offsets) for w in ws)
 
 
 def grouped_linear(x, w, seg_offsets, counts=None):
     if x.is_cuda and x.dtype == torch.bfloat16:
-        return _GroupedLinear.apply(x, w, seg_offsets)
+        return _GroupedLinear.apply(x, seg_offsets, w)
     # CPU statement over the padded layout
     outs = x.new_zeros(x.shape[0], w.shape[1])
     seg = seg_offsets.tolist()
@@ -76,12 +104,13 @@ def grouped_linear(x, w, seg_offsets, counts=None):
 
 
 class _PermuteRows(torch.autograd.Function):
-    """rows[dest[c]] = x[c // k] into a zeroed padded buffer; backward sums the k copies of every token."""
+    """rows[dest[c]] = x[c // k], padding rows of every segment zero; backward sums the k copies of every token. Rows past the
+    last segment of the statically sized buffer stay unwritten: every consumer stops at that segment's end."""
 
     @staticmethod
-    def forward(ctx, x, dest, cap, k):
-        rows = torch.zeros(cap, x.shape[1], dtype=x.dtype, device=x.device)
-        _ext().permute_rows(x.contiguous(), dest, rows, k)
+    def forward(ctx, x, dest, cap, k, seg, counts):
+        rows = (torch.empty if dest.numel() else torch.zeros)(cap, x.shape[1], dtype=x.dtype, device=x.device)
+        _ext().permute_rows(x.contiguous(), dest, rows, k, seg, counts)
         ctx.save_for_backward(dest)
         ctx.k, ctx.T = k, x.shape[0]
         return rows
@@ -89,24 +118,24 @@ class _PermuteRows(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (dest,) = ctx.saved_tensors
-        return _ext().combine_rows(g.contiguous(), dest, None, ctx.T, ctx.k), None, None, None
+        return _ext().combine_rows(g.contiguous(), dest, None, ctx.T, ctx.k), None, None, None, None, None
 
 
 class _CombineRows(torch.autograd.Function):
     """out[t] = sum_j w[t, j] * y[dest[t * k + j]] in fp32."""
 
     @staticmethod
-    def forward(ctx, y, weights, dest, T, k):
+    def forward(ctx, y, weights, dest, T, k, seg, counts):
         w = weights.float().contiguous()
-        ctx.save_for_backward(y, w, dest)
+        ctx.save_for_backward(y, w, dest, seg, counts)
         ctx.k = k
         return _ext().combine_rows(y.contiguous(), dest, w, T, k)
 
     @staticmethod
     def backward(ctx, g):
-        y, w, dest = ctx.saved_tensors
-        dy, dw = _ext().combine_bwd(g, y.contiguous(), dest, w.reshape(-1), ctx.k)
-        return dy, dw.view_as(w), None, None, None
+        y, w, dest, seg, counts = ctx.saved_tensors
+        dy, dw = _ext().combine_bwd(g, y.contiguous(), dest, w.reshape(-1), ctx.k, seg, counts)
+        return dy, dw.view_as(w), None, None, None, None, None
 
 
 class GroupedExperts(nn.Module):
@@ -144,7 +173,7 @@ class GroupedExperts(nn.Module):
                     h = ops.swiglu(g_, u_) if self.glu_fn is None else self.glu_fn(g_, u_)
                     out[s:t] = ops.linear(h, self.w2_EDF[e])
             return out
-        g, u = self._clamp(grouped_linear(rows, self.w1_EFD, seg_offsets), grouped_linear(rows, self.w3_EFD, seg_offsets))
+        g, u = self._clamp(*grouped_linears(rows, seg_offsets, self.w1_EFD, self.w3_EFD))
         # rows past the last segment of a statically sized receive buffer hold nothing: the kernels skip them
         limit = seg_offsets[-1:] if rows.is_cuda and seg_offsets.dtype == torch.int32 else None
         h = ops.swiglu(g, u, limit) if self.glu_fn is None else self.glu_fn(g, u)
@@ -164,16 +193,16 @@ class LocalTokenDispatcher:
         dest, seg, counts = plan_segments(flat, self.num_experts)
         cap = padded_capacity(T * k, self.num_experts)
         if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0:
-            rows = _PermuteRows.apply(x, dest, cap, k)
+            rows = _PermuteRows.apply(x, dest, cap, k, seg, counts)
         else:
             tok = torch.arange(T * k, device=x.device) // k
             rows = x.new_zeros(cap, x.shape[1]).index_copy(0, dest, x.index_select(0, tok))
-        return rows, seg, {"dest": dest, "T": T, "k": k}
+        return rows, seg, {"dest": dest, "T": T, "k": k, "seg": seg, "counts": counts}
 
     def combine(self, y: torch.Tensor, weights: torch.Tensor, state) -> torch.Tensor:
         T, k = state["T"], state["k"]
         if y.is_cuda and y.dtype == torch.bfloat16 and y.shape[1] % 8 == 0:
-            return _CombineRows.apply(y, weights, state["dest"], T, k)
+            return _CombineRows.apply(y, weights, state["dest"], T, k, state["seg"], state["counts"])
         g = y.index_select(0, state["dest"]).view(T, k, -1)
         return (g.float() * weights.float().unsqueeze(-1)).sum(1).to(y.dtype)
 
