@@ -8,7 +8,7 @@
 // so no operand is ever transposed in memory. The grouped form runs the same tiles over row segments
 // of A (one per expert, 128-row aligned) against a stack of B matrices.
 //
-// CTA = 6 warps: warp 0 issues TMA, warp 1 owns TMEM and issues MMAs, warps 2-5 drain the accumulator.
+// Warp 0 issues TMA, warp 1 owns TMEM and issues MMAs, the next 8 (4 beside comm warps) drain the accumulator.
 // The accumulator is double buffered in TMEM so the epilogue of tile i overlaps the MMAs of tile i+1.
 #include <type_traits>
 #include "comm.cuh"
@@ -18,13 +18,21 @@ namespace llmt {
 
 constexpr int BM = 128;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzle row
-constexpr int kGemmThreads = 192;                       // TMA warp, MMA warp, 4 epilogue warps
-constexpr int kGemmThreadsComm = 192 + kCommThreads;   // plus the comm warps that carry a SideJob
+// COMM: the form launched with a SideJob or a fused tensor-parallel collective: TMA warp, MMA warp, 4 epilogue warps and the
+// comm warps. Without it 8 epilogue warps, two per tensor-memory lane quarter with half of the columns each: one warp per
+// scheduler waits out every tensor-memory and shared-memory latency of a chunk by itself (0.45 us per 64 columns), which
+// shows wherever the k-loop is short: expert weight gradients (K = rows of one expert), small products, the last tile.
+template <bool COMM>
+struct GemmRoles {
+  static constexpr int kEpiWarps = COMM ? 4 : 8;
+  static constexpr int kCommBase = 64 + 32 * kEpiWarps;                       // first comm thread
+  static constexpr int kThreads = kCommBase + (COMM ? kCommThreads : 0);
+};
 
 // CG: CTAs that work on one tile. 1: a 128 x BN tile per CTA. 2: a 256 x BN tile per cluster of two CTAs (cta_group::2): each
 // CTA loads its 128 rows of A and its half of the B tile, the tensor cores of both SMs read both halves of B, and each CTA's
 // tensor memory receives its 128 rows of the product. See pick_tile() for when which is used.
-template <int CG, int BN>
+template <int CG, int BN, bool COMM>
 struct GemmCfg {
   static constexpr int kBRows = BN / CG;           // rows of B that this CTA loads
   static constexpr int kStages = (kBRows == 256) ? 4 : 6;
@@ -32,7 +40,7 @@ struct GemmCfg {
   static constexpr int kBBytes = kBRows * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kTmemCols = 2 * BN;  // two accumulators
-  static constexpr int kEpiBytes = 4 * 4096;  // staging of the epilogue: 32 rows of 128 bytes per warp
+  static constexpr int kEpiBytes = GemmRoles<COMM>::kEpiWarps * 4096;  // staging of the epilogue: 32 rows of 128 bytes per warp
   static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024 /*align slack*/ + 256 /*barriers*/;
 };
 
@@ -41,11 +49,13 @@ struct GroupedArgs {
   int num_groups;
 };
 
-template <int CG, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE>
-__global__ void __launch_bounds__(CG == 2 ? kGemmThreads : kGemmThreadsComm, 1)
+template <int CG, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE, bool COMM>
+__global__ void __launch_bounds__(GemmRoles<COMM>::kThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     void* __restrict__ Cptr, int M, int N, int K, int64_t ldc, GroupedArgs grp, SideJob side, TPFuse tp, int* status) {
-  using Cfg = GemmCfg<CG, BN>;
+  using Cfg = GemmCfg<CG, BN, COMM>;
+  using Roles = GemmRoles<COMM>;
+  static_assert(!COMM || (CG == 1 && MODE == 0), "collectives ride on plain single-CTA products");
   static_assert(CG == 1 || MODE != 1, "segments are 128-row aligned: a 256-row tile would straddle them");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -74,7 +84,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], CG * 128);
+      mbar_init(&tempty[a], CG * 32 * Roles::kEpiWarps);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -122,7 +132,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr int kGroupM = 16 / CG;
   // With a fused tensor-parallel collective (MODE 0 only) the rows are walked chunk by chunk instead: the all-gather
   // form starts with this rank's own chunk, the reduce-scatter form ends with it.
-  const bool tp_on = (MODE == 0) && tp.mode != kTPNone;
+  const bool tp_on = COMM && tp.mode != kTPNone;
   const int tp_mpc = tp_on ? tp.chunk_rows / BM : 1;
   const int tp_tpc = tp_mpc * num_n;
   auto tp_chunk_of = [&](int tt) -> int { return (tp.rank + tt / tp_tpc + (tp.mode == kTPReduceScatter ? 1 : 0)) % tp.world; };
@@ -288,21 +298,23 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
     __syncwarp();
-  } else if (warp >= 6) {
+  } else if (COMM && warp >= 2 + Roles::kEpiWarps) {
     // ------------------------------------------------------------------ comm warps (only launched with a SideJob)
     if (tp_on) {
-      if (tp.mode == kTPAllGather) tp_allgather_comm(tp, threadIdx.x - 192, comm_word, status);
-      else tp_reducescatter_comm(tp, threadIdx.x - 192, comm_word, status);
+      if (tp.mode == kTPAllGather) tp_allgather_comm(tp, threadIdx.x - Roles::kCommBase, comm_word, status);
+      else tp_reducescatter_comm(tp, threadIdx.x - Roles::kCommBase, comm_word, status);
     } else {
-      run_side_job(side, (long long)blockIdx.x * kCommThreads + (threadIdx.x - 192), (long long)gridDim.x * kCommThreads, status);
+      run_side_job(side, (long long)blockIdx.x * kCommThreads + (threadIdx.x - Roles::kCommBase), (long long)gridDim.x * kCommThreads, status);
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..)
     // A thread reads one row of the accumulator, so storing from registers touches 32 rows per instruction with 16 bytes each.
     // Every warp instead turns 32 rows x 128 bytes around in shared memory (16-byte chunks XORed with the row: no bank
     // conflicts) and writes, and when accumulating reads, whole 128-byte lines. What is added is added in fp32.
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
-    uint8_t* stg = epi + quarter * 4096;
+    constexpr int kCols = BN * 4 / Roles::kEpiWarps;       // columns of the tile that this warp drains, from col_w on
+    const int col_w = ((warp - 2) >> 2) * kCols;
+    uint8_t* stg = epi + (warp - 2) * 4096;
     constexpr int kOutBytes = OUT_F32 ? 4 : 2;
     constexpr bool kStageF32 = OUT_F32 || ACCUM;
     constexpr int kChunk = kStageF32 ? 32 : 64;            // columns per 128-byte staging row
@@ -320,20 +332,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int row0 = m0 + quarter * 32;
       if constexpr (ACCUM) {        // fetch this warp's rows of C into L2 while their product is still being computed
         const int pr = min(row0 + lane, row_limit - 1);
-        const uint8_t* line = reinterpret_cast<const uint8_t*>(Cptr) + (c_base + (int64_t)pr * ldc + n0) * kOutBytes;
-        for (int o = 0; o < min(BN, N - n0) * kOutBytes; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + o));
+        const uint8_t* line = reinterpret_cast<const uint8_t*>(Cptr) + (c_base + (int64_t)pr * ldc + n0 + col_w) * kOutBytes;
+        for (int o = 0; o < min(kCols, N - n0 - col_w) * kOutBytes; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + o));
       }
       if (!mbar_wait_bounded(&tfull[acc], acc_phase, abort_flag, status, 400 + acc)) break;
       tc_fence_after();
-      const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      const int n_chunks = (min(BN, N - n0) + kChunk - 1) / kChunk;
+      const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + col_w;
+      const int n_chunks = (min(kCols, N - n0 - col_w) + kChunk - 1) / kChunk;   // <= 0: these columns lie outside
       const bool tile_vec = vec_ok && ((c_base * kOutBytes) & 15) == 0;
 #pragma unroll 1
       for (int c = 0; c < n_chunks; ++c) {
         uint32_t r[kChunk];
         tmem_ld_32x32(t_row + c * kChunk, r);
         if constexpr (kChunk == 64) tmem_ld_32x32(t_row + c * kChunk + 32, r + 32);
-        const int col0 = n0 + c * kChunk;
+        const int col0 = n0 + col_w + c * kChunk;
         if (tile_vec && (N & 7) == 0) {
           constexpr int kPer = kStageF32 ? 4 : 8;          // columns per 16 staged bytes
           const int col = col0 + cc * kPer;
@@ -344,7 +356,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if constexpr (ACCUM) {
             // clamped instead of skipped: eight unconditional loads are in flight together, a branch around each would
             // leave them one after another
-            const int64_t cat = c_base + (col_ok ? col : n0);
+            const int64_t cat = c_base + (col_ok ? col : n0);   // n0 < N
 #pragma unroll
             for (int it = 0; it < 8; ++it)
               old[it] = *reinterpret_cast<const OldT*>(reinterpret_cast<const uint8_t*>(Cptr) +
@@ -500,11 +512,17 @@ static bool use_pair(int64_t M, int64_t N, int max_ctas) {
   return 100 * pair <= 107 * single;
 }
 
-template <int CG, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE>
+template <int CG, int BN, bool A_MN, bool B_MN, bool OUT_F32, bool ACCUM, int MODE, bool COMM = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, int N, int K, int64_t ldc, GroupedArgs grp,
                   int* status, int max_ctas, cudaStream_t stream, const SideJob* side = nullptr, const TPFuse* tpf = nullptr) {
-  using Cfg = GemmCfg<CG, BN>;
-  auto kern = gemm_tcgen05_kernel<CG, BN, A_MN, B_MN, OUT_F32, ACCUM, MODE>;
+  const bool with_tp = tpf != nullptr && tpf->mode != kTPNone;
+  const bool with_side = (side != nullptr && side->kind != kSideNone) || with_tp;
+  if constexpr (CG == 1 && MODE == 0 && !COMM)
+    if (with_side)
+      return launch<CG, BN, A_MN, B_MN, OUT_F32, ACCUM, MODE, true>(ta, tb, C, M, N, K, ldc, grp, status, max_ctas, stream, side, tpf);
+  using Cfg = GemmCfg<CG, BN, COMM>;
+  constexpr int kThreads = GemmRoles<COMM>::kThreads;
+  auto kern = gemm_tcgen05_kernel<CG, BN, A_MN, B_MN, OUT_F32, ACCUM, MODE, COMM>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess) return -2;
@@ -517,7 +535,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, 
   if constexpr (CG == 2) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid * 2);
-    cfg.blockDim = dim3(kGemmThreads);
+    cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute at{};
@@ -529,10 +547,8 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, void* C, int M, 
   }
   SideJob none{};
   TPFuse no_tp{};
-  const bool with_tp = tpf != nullptr && tpf->mode != kTPNone;
-  const bool with_side = (side != nullptr && side->kind != kSideNone) || with_tp;
   if (with_side && max_ctas <= 0) grid = sm_count();   // every SM carries comm warps, even past the last tile
-  kern<<<grid, with_side ? kGemmThreadsComm : kGemmThreads, Cfg::kSmemBytes, stream>>>(
+  kern<<<grid, kThreads, Cfg::kSmemBytes, stream>>>(
       ta, tb, C, M, N, K, ldc, grp, (side != nullptr && !with_tp) ? *side : none, with_tp ? *tpf : no_tp, status);
   return (cudaGetLastError() == cudaSuccess) ? 0 : -3;
 }
@@ -699,7 +715,8 @@ extern "C" int llmt_grouped_wgrad_bf16(const void* A, const void* B, void* C, co
     if (make_tmap_bf16(&tb, B, 2, dims, str, box)) return -12;
   }
   GroupedArgs grp{seg_offsets, num_groups};
-  const int K = rows_padded;
+  const int K = rows_padded;      // single-CTA tiles: with the few k-blocks of one expert the pair form measured slower (164 us
+                                  // against 141 us per 128 x 768 x 2048 gradient over 32768 rows, 62 us to write it)
 #define LLMT_W(BNV, F32, ACC) \
   if (bn256 == (BNV == 256) && (bool)out_f32 == F32 && (bool)accumulate == ACC) \
     return launch<1, BNV, true, true, F32, ACC, 2>(ta, tb, C, M, N, K, (int64_t)N, grp, status, 0, stream);
