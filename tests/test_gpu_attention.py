@@ -234,3 +234,41 @@ def test_attention_pads_widths_without_a_kernel_variant(d, dv, causal):
     for a, b, n in zip(g1, g2, ("dq", "dk", "dv")):
         assert a.shape == b.shape
         _close(a, b, n)
+
+
+@pytest.mark.parametrize("pieces,Tq,Tk,Hq,Hkv,causal", [
+    # two queries: a single visible key makes dS exactly zero (dP = delta), so a one-row piece would compare rounding residues
+    # of 2^-23 |dP| against each other; the second row's gradients set the scale here
+    ([(0, 2, 0, 2, 0)], 2, 2, 1, 1, True),
+    ([(0, 65, 0, 65, 0), (65, 129, 65, 129, 0)], 194, 194, 6, 2, True),          # a group of three: not split over CTAs
+    ([(0, 100, 0, 300, 200)], 100, 300, 4, 1, True),                             # more keys than queries, offset diagonal
+    ([(0, 300, 0, 100, 0)], 300, 100, 4, 2, True),                               # queries past the last key
+    ([(10, 90, 20, 80, 0), (150, 64, 130, 64, 0)], 230, 210, 8, 2, True),        # rows that belong to no piece
+    ([(0, 257, 0, 191, 0)], 257, 191, 8, 1, False),
+    ([(0, 2600, 0, 2600, 0)], 2600, 2600, 16, 4, True)])
+def test_attention_backward_head_256_against_the_row_form(pieces, Tq, Tk, Hq, Hkv, causal):
+    """The backward kernels of head size 256 against the row-chunked form (library products with fp32 results, the path of
+    pieces that share keys) over uneven pieces, offsets and row gaps; gradients repeat bit for bit and rows outside every piece
+    are zero."""
+    from torchllmtuner_b200 import ops
+    from torchllmtuner_b200.ops import reference as ref
+    from torchllmtuner_b200.ops.cuda_ext import check_status, load
+    torch.manual_seed(Tq)
+    q, k, v = (torch.randn(n, h, 256, device="cuda").bfloat16().requires_grad_() for n, h in ((Tq, Hq), (Tk, Hkv), (Tk, Hkv)))
+    meta = ops.AttnMeta.from_pieces(pieces, Tq, Tk, causal, device="cuda")
+    assert len(meta.k_tile_passes) == 1
+    o = ops.attention(q, k, v, meta)
+    _, lse = ops.attention_with_lse(q.detach(), k.detach(), v.detach(), meta)
+    covered = torch.zeros(Tq, dtype=torch.bool, device="cuda")
+    for p in pieces:
+        covered[p[0]:p[0] + p[1]] = True
+    go = torch.randn_like(o)
+    o_ = torch.where(covered[:, None, None], o.detach(), torch.zeros_like(o))
+    got = torch.autograd.grad(o, [q, k, v], go, retain_graph=True)
+    check_status("attn_bwd_wide")
+    want = ref.attention_backward_rows(q.detach(), k.detach(), v.detach(), o_, go, lse, meta.pieces, causal, 256 ** -0.5)
+    for n, a, b in zip(("dq", "dk", "dv"), got, want):
+        _close(a, b.float(), n)
+    assert got[0][~covered].abs().sum() == 0
+    for a, b in zip(got, torch.autograd.grad(o, [q, k, v], go)):
+        assert torch.equal(a, b)

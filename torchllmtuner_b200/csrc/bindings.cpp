@@ -619,6 +619,33 @@ std::vector<Tensor> attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, 
   return {dq, dk, dv};
 }
 
+// Head size 256. `zero_init`: some query or key row belongs to no tile and its gradient is zero.
+std::vector<Tensor> attn_bwd_wide(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& dout, const Tensor& lse,
+                                  const Tensor& q_tiles, const Tensor& k_tiles, double scale, bool causal, bool zero_init) {
+  c10::cuda::CUDAGuard guard(q.device());
+  check_bf16(q, "q"); check_bf16(k, "k"); check_bf16(v, "v"); check_bf16(dout, "dout");
+  for (const Tensor* t : {&q, &k, &v, &dout})
+    TORCH_CHECK(t->dim() == 3 && t->size(2) == 256 && t->stride(2) == 1 && t->stride(1) == 256, "operands need packed heads [T, H, 256]");
+  for (const Tensor* t : {&q_tiles, &k_tiles})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kInt && t->is_contiguous() && t->size(1) == 8, "tile tables must be int32 [n, 8]");
+  TORCH_CHECK(o.is_contiguous() && lse.is_contiguous() && dout.size(0) == q.size(0) && dout.size(1) == q.size(1));
+  const int Tq = (int)q.size(0), Hq = (int)q.size(1), Tk = (int)k.size(0), Hkv = (int)k.size(1);
+  auto make = [&](const Tensor& t) { return zero_init ? torch::zeros(t.sizes(), t.options()) : torch::empty(t.sizes(), t.options()); };
+  Tensor dq = make(q), dk = make(k), dv = make(v);
+  Tensor delta = torch::empty({Hq, Tq}, q.options().dtype(torch::kFloat));
+  const int nq = (int)q_tiles.size(0), nk = (int)k_tiles.size(0);
+  const int nsplit = zero_init ? 1 : llmt_attn_bwd_wide_splits(nk, Hq, Hkv);
+  Tensor part;
+  if (nsplit > 1) part = torch::empty({2, nsplit, Tk, Hkv, 256}, delta.options());
+  check_rc(llmt_attn_bwd_wide(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(),
+                              delta.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), nsplit > 1 ? part.data_ptr<float>() : nullptr,
+                              nsplit, q_tiles.data_ptr<int>(), nq, k_tiles.data_ptr<int>(), nk, Tq, Tk, Hq, Hkv, q.stride(0), k.stride(0),
+                              v.stride(0), o.stride(0), dout.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), (float)scale, causal,
+                              status_ptr(), cur_stream()),
+           "llmt_attn_bwd_wide", nsplit > 1 ? 3 : 2);
+  return {dq, dk, dv};
+}
+
 // ---- MoE
 std::vector<Tensor> router_topk(const Tensor& logits, const c10::optional<Tensor>& bias, int64_t k, int64_t score_fn, bool renorm,
                                 double route_scale) {
@@ -775,6 +802,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_fwd", &attn_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("tiles"), py::arg("scale"), py::arg("causal"),
         py::arg("pair") = false);
   m.def("attn_bwd", &attn_bwd);
+  m.def("attn_bwd_wide", &attn_bwd_wide);
   m.def("read_status", &read_status, py::arg("clear") = true);
   m.def("status_tensor", &status_tensor);
   m.def("launch_count", &launch_count);

@@ -118,6 +118,13 @@ int llmt_attn_bwd_fused(const void* q, const void* k, const void* v, const void*
                         int Tq, int Tk, int Hq, int Hkv, int HD, int64_t q_stride, int64_t k_stride, int64_t v_stride,
                         int64_t o_stride, int64_t do_stride, int64_t dq_stride, int64_t dk_stride, int64_t dv_stride,
                         float scale, int causal, int first, int last, int* status, cudaStream_t st);
+// Head size 256 (attention_bwd_wide.cu): dQ, dK and dV walks in one launch, no atomics.
+int llmt_attn_bwd_wide_splits(int num_k_tiles, int Hq, int Hkv);
+int llmt_attn_bwd_wide(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse, float* delta,
+                       void* dq, void* dk, void* dv, float* part, int nsplit, const int* q_tiles, int num_q_tiles, const int* k_tiles,
+                       int num_k_tiles, int Tq, int Tk, int Hq, int Hkv, int64_t q_stride, int64_t k_stride, int64_t v_stride,
+                       int64_t o_stride, int64_t do_stride, int64_t dq_stride, int64_t dk_stride, int64_t dv_stride, float scale,
+                       int causal, int* status, cudaStream_t st);
 
 #ifdef __cplusplus
 }

@@ -329,7 +329,7 @@ def swiglu(gate, up, row_limit=None):
 
 
 # ----------------------------------------------------------------------------------------------- attention
-DEVICE_ATTENTION_HEAD_DIMS = (64, 128, 256)     # 256: forward kernel, backward rebuilt per chunk of rows from the LSE
+DEVICE_ATTENTION_HEAD_DIMS = (64, 128, 256)     # 256: a backward of three walks; row-chunked where pieces share keys
 
 
 class _Attention(torch.autograd.Function):
@@ -347,8 +347,18 @@ class _Attention(torch.autograd.Function):
         if do.stride(2) != 1 or do.stride(1) != do.shape[2]:
             do = do.contiguous()
         m = ctx.meta
-        if q.shape[-1] not in (64, 128):      # forward kernel only at this head size: rebuild P per chunk of rows from the LSE
+        if q.shape[-1] not in (64, 128):
             ext = _ext()
+            # every key belongs to one piece, and no piece starts with queries that see no key (a query tile's table cannot
+            # hold a diagonal before column 0)
+            if len(m.k_tile_passes) == 1 and all(p[4] >= 0 for p in m.pieces):
+                if do.stride(0) % 8 or do.data_ptr() % 16:
+                    do = do.contiguous()
+                whole = m.covers_all_keys and m.total_k == k.shape[0] and sum(p[1] for p in m.pieces) == q.shape[0]
+                dq, dk, dv = ext.attn_bwd_wide(q, k, v, o, do, lse, m.q_tiles, m.k_tile_passes[0], ctx.scale, m.causal, not whole)
+                return dq, dk, dv, None, None, None
+            # pieces that share keys (context-parallel shards) sum dK / dV over passes: rebuild P per chunk of rows from the
+            # LSE with fp32 accumulators
             dq, dk, dv = ref.attention_backward_rows(q, k, v, o, do, lse, m.pieces, m.causal, ctx.scale,
                                                      probs_fn=ext.attn_rows_probs, ds_fn=ext.attn_rows_ds)
             return dq, dk, dv, None, None, None
