@@ -63,7 +63,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tile_idx = blockIdx.x / Hq;
   const int h = blockIdx.x % Hq;
   const int hk = h / (Hq / Hkv);
@@ -132,46 +132,49 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && n_kv > 0) {
+    if (n_kv > 0) {                                   // warp-uniform control flow, one lane issues (see uniform_warp)
       constexpr uint32_t idS = umma_idesc_bf16(128, kFwdKV, false, false);
       constexpr uint32_t idPV = umma_idesc_bf16(128, HD, false, true);
-      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP);
-      const uint32_t loVm = desc_lo(aV, kFwdKV * 128);
+      const uint32_t loQ = desc_lo(smem_u32(sQ), 16), loK = desc_lo(smem_u32(sK), 16), loVm = desc_lo(smem_u32(sV), kFwdKV * 128),
+                     loP = desc_lo(smem_u32(sP), 16);
+      const bool leader = elect_one();
       bool ok = mbar_wait_bounded(q_full, 0, abort_flag, status, 1200);
-      auto issue_S = [&](int j) -> bool {
-        const int s = j & 1;
+      auto issue_S = [&](auto sc, int j) -> bool {
+        constexpr int s = decltype(sc)::value;
         const uint32_t ph = (j >> 1) & 1;
         if (!mbar_wait_bounded(&kfull[s], ph, abort_flag, status, 1210 + s)) return false;
         if (!mbar_wait_bounded(&sempty[s], ph ^ 1, abort_flag, status, 1220 + s)) return false;
         tc_fence_after();
-        {
-          // descriptors differ only in the start address field: build the two bases once and step the low word
-          const uint64_t dq0 = desc_kmajor_rows(aQ, 0, 128), dk0 = desc_kmajor_rows(aK + s * kKVBytes, 0, kFwdKV);
-          const uint32_t d_s = tS + s * kFwdKV;
+        if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
-            const uint64_t offq = (uint64_t)(((ks >> 2) * (128 * 128) + (ks & 3) * 32) >> 4);
-            const uint64_t offk = (uint64_t)(((ks >> 2) * (kFwdKV * 128) + (ks & 3) * 32) >> 4);
-            umma_bf16_ss(d_s, dq0 + offq, dk0 + offk, idS, ks ? 1u : 0u);
-          }
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_bf16_ss(tS + s * kFwdKV, desc_pack(loQ + koff(ks, 128)), desc_pack(loK + s * (kKVBytes >> 4) + koff(ks, kFwdKV)), idS, ks ? 1u : 0u);
+          umma_commit(&sfull[s]);
+          umma_commit(&kempty[s]);
         }
-        umma_commit(&sfull[s]);
-        umma_commit(&kempty[s]);
         return true;
       };
-      if (ok) ok = issue_S(0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        if (j + 1 < n_kv) { if (!issue_S(j + 1)) break; }
-        const int pb = j & 1;
-        if (!mbar_wait_bounded(&pfull[pb], (j >> 1) & 1, abort_flag, status, 1230 + pb)) break;
-        if (!mbar_wait_bounded(vfull, j & 1, abort_flag, status, 1240)) break;
+      auto step = [&](auto sc, auto nc, int j) -> bool {
+        constexpr int pb = decltype(sc)::value;
+        if (j + 1 < n_kv && !issue_S(nc, j + 1)) return false;
+        if (!mbar_wait_bounded(&pfull[pb], (j >> 1) & 1, abort_flag, status, 1230 + pb)) return false;
+        if (!mbar_wait_bounded(vfull, j & 1, abort_flag, status, 1240)) return false;
         tc_fence_after();
-        const uint32_t loP = desc_lo(aP + pb * kPBytes, 16), acc0 = j ? 1u : 0u;
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < kFwdKV / 16; ++ks)
-          umma_bf16_ss(tO, desc_pack(loP + koff(ks, 128)), desc_pack(loVm + mnoff(ks)), idPV, ks ? 1u : acc0);
-        umma_commit(vempty);
-        umma_commit(&pvdone[pb]);
+          for (int ks = 0; ks < kFwdKV / 16; ++ks)
+            umma_bf16_ss(tO, desc_pack(loP + pb * (kPBytes >> 4) + koff(ks, 128)), desc_pack(loVm + mnoff(ks)), idPV, ks ? 1u : (j ? 1u : 0u));
+          umma_commit(vempty);
+          umma_commit(&pvdone[pb]);
+        }
+        return true;
+      };
+      using I0 = std::integral_constant<int, 0>;
+      using I1 = std::integral_constant<int, 1>;
+      if (ok) ok = issue_S(I0{}, 0);
+      for (int j = 0; j < n_kv && ok; j += 2) {
+        ok = step(I0{}, I1{}, j);
+        if (ok && j + 1 < n_kv) ok = step(I1{}, I0{}, j + 1);
       }
     }
     __syncwarp();

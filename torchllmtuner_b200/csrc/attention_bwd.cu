@@ -29,35 +29,6 @@ namespace llmt {
 
 constexpr int kFusedThreads = 64 + 256 + 128;
 
-// Packed two-lane fp32 arithmetic (one issue slot for two elements).
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  uint64_t ra, rb, rc, rd;
-  float2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rc) : "f"(c.x), "f"(c.y));
-  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(rd) : "l"(ra), "l"(rb), "l"(rc));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  uint64_t ra, rb, rd;
-  float2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-  uint64_t ra, rb, rd;
-  float2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(ra) : "f"(a.x), "f"(a.y));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(rb) : "f"(b.x), "f"(b.y));
-  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(rd) : "l"(ra), "l"(rb));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
-  return d;
-}
 constexpr int kStageBytes = 128 * 32 * 4;   // one 32-column fp32 slice of a dQ tile
 
 template <int HD>
@@ -104,7 +75,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tile_idx = blockIdx.x / Hkv;
   const int hk = blockIdx.x % Hkv;
   const int g = Hq / Hkv;
@@ -172,73 +143,87 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_it > 0) {
+    // warp-uniform control flow, one lane issues (see uniform_warp)
+    if (n_it > 0) {
       constexpr uint32_t idS = umma_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idSh = umma_idesc_bf16(128, 64, false, false);
       constexpr uint32_t idAcc = umma_idesc_bf16(128, HD, false, true);
       constexpr uint32_t idDQ = umma_idesc_bf16(128, HD, true, true);
-      const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), adO = smem_u32(sdO), adS = smem_u32(sdS);
-      const uint32_t loK = desc_lo(aK, 16), loV = desc_lo(aV, 16), loKm = desc_lo(aK, 16384);
+      const uint32_t aK = smem_u32(sK), aQ = smem_u32(sQ), adO = smem_u32(sdO), adS = smem_u32(sdS);
+      const uint32_t loK = desc_lo(aK, 16), loV = desc_lo(smem_u32(sV), 16), loKm = desc_lo(aK, 16384);
+      const uint32_t loQ = desc_lo(aQ, 16), loQm = desc_lo(aQ, 16384);
       const uint32_t lodO = desc_lo(adO, 16), lodOm = desc_lo(adO, 16384);
       const uint32_t lodS = desc_lo(adS, 16), lodSm = desc_lo(adS, 16384);
+      const bool leader = elect_one();
       bool ok = mbar_wait_bounded(kv_full, 0, abort_flag, status, 4200);
       // S^T half hb (queries hb*64 .. +64) = K Q_hb^T; the half's 64 query rows sit 8192 B into each 64-column block of Q
-      auto issue_S = [&](int it, int hb) -> bool {
-        const int b = it & 1;
+      auto issue_S = [&](auto bc, int it, int hb) -> bool {
+        constexpr int b = decltype(bc)::value;
         if (hb == 0) {
           if (!mbar_wait_bounded(&q_full[b], (it >> 1) & 1, abort_flag, status, 4210 + b)) return false;
           tc_fence_after();
         }
-        const uint32_t loQ = desc_lo(aQ + b * kTile + hb * 8192, 16);
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks)
-          umma_bf16_ss(tS + hb * 64, desc_pack(loK + koff(ks, 128)), desc_pack(loQ + koff(ks, 128)), idSh, ks ? 1u : 0u);
-        umma_commit(&s_full[hb]);
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_bf16_ss(tS + hb * 64, desc_pack(loK + koff(ks, 128)), desc_pack(loQ + ((b * kTile + hb * 8192) >> 4) + koff(ks, 128)), idSh,
+                         ks ? 1u : 0u);
+          umma_commit(&s_full[hb]);
+        }
         return true;
       };
       auto issue_dP = [&](int it) -> bool {          // dP^T = V dO^T, into the columns the previous dQ tile has left
         if (!mbar_wait_bounded(do_full, it & 1, abort_flag, status, 4220)) return false;
         if (it > 0 && !mbar_wait_bounded(dq_empty, (it - 1) & 1, abort_flag, status, 4225)) return false;
         tc_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks)
-          umma_bf16_ss(tDP, desc_pack(loV + koff(ks, 128)), desc_pack(lodO + koff(ks, 128)), idS, ks ? 1u : 0u);
-        umma_commit(dp_full);
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_bf16_ss(tDP, desc_pack(loV + koff(ks, 128)), desc_pack(lodO + koff(ks, 128)), idS, ks ? 1u : 0u);
+          umma_commit(dp_full);
+        }
         return true;
       };
-      if (ok) ok = issue_S(0, 0) && issue_S(0, 1) && issue_dP(0);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int b = it & 1;
+      using I0 = std::integral_constant<int, 0>;
+      using I1 = std::integral_constant<int, 1>;
+      auto step = [&](auto bc, auto nc, int it) -> bool {            // tile `it` in Q stage b; the next tile's stage is n
+        constexpr int b = decltype(bc)::value;
         const uint32_t acc0 = it ? 1u : 0u;
         const bool next = it + 1 < n_it;
-        bool fail = false;
 #pragma unroll
         for (int hb = 0; hb < 2; ++hb) {
-          if (!mbar_wait_bounded(&p_full[hb], it & 1, abort_flag, status, 4230 + hb)) { fail = true; break; }
+          if (!mbar_wait_bounded(&p_full[hb], it & 1, abort_flag, status, 4230 + hb)) return false;
           tc_fence_after();
           // dV += P_hb^T dO_hb: 16-query slice ks of the half sits at column (ks >> 1) * 32 + (ks & 1) * 8 of the half
+          if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_bf16_ts(tDV, tS + (uint32_t)(hb * 64 + (ks >> 1) * 32 + (ks & 1) * 8), desc_pack(lodOm + mnoff(hb * 4 + ks)), idAcc,
-                         (hb | ks) ? 1u : acc0);
-          if (hb == 1) umma_commit(do_empty);
-          if (next && !issue_S(it + 1, hb)) { fail = true; break; }     // refill the half just consumed
+            for (int ks = 0; ks < 4; ++ks)
+              umma_bf16_ts(tDV, tS + (uint32_t)(hb * 64 + (ks >> 1) * 32 + (ks & 1) * 8), desc_pack(lodOm + mnoff(hb * 4 + ks)), idAcc,
+                           (hb | ks) ? 1u : acc0);
+            if (hb == 1) umma_commit(do_empty);
+          }
+          if (next && !issue_S(nc, it + 1, hb)) return false;           // refill the half just consumed
         }
-        if (fail) break;
-        if (!mbar_wait_bounded(ds_full, it & 1, abort_flag, status, 4240)) break;
+        if (!mbar_wait_bounded(ds_full, it & 1, abort_flag, status, 4240)) return false;
         tc_fence_after();
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)                // dQ = dS K, first: its read-out gates the next dP^T product
-          umma_bf16_ss(tDP, desc_pack(lodSm + mnoff(ks)), desc_pack(loKm + mnoff(ks)), idDQ, ks ? 1u : 0u);
-        umma_commit(dq_full);
-        const uint32_t loQm = desc_lo(aQ + b * kTile, 16384);
+          for (int ks = 0; ks < 8; ++ks)                // dQ = dS K, first: its read-out gates the next dP^T product
+            umma_bf16_ss(tDP, desc_pack(lodSm + mnoff(ks)), desc_pack(loKm + mnoff(ks)), idDQ, ks ? 1u : 0u);
+          umma_commit(dq_full);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)                // dK += dS^T Q
-          umma_bf16_ss(tDK, desc_pack(lodS + koff(ks, 128)), desc_pack(loQm + mnoff(ks)), idAcc, ks ? 1u : acc0);
-        umma_commit(&q_empty[b]);
-        umma_commit(ds_empty);
-        if (it == n_it - 1) umma_commit(acc_done);
-        if (next && !issue_dP(it + 1)) break;
+          for (int ks = 0; ks < 8; ++ks)                // dK += dS^T Q
+            umma_bf16_ss(tDK, desc_pack(lodS + koff(ks, 128)), desc_pack(loQm + ((b * kTile) >> 4) + mnoff(ks)), idAcc, ks ? 1u : acc0);
+          umma_commit(&q_empty[b]);
+          umma_commit(ds_empty);
+          if (!next) umma_commit(acc_done);
+        }
+        return !next || issue_dP(it + 1);
+      };
+      if (ok) ok = issue_S(I0{}, 0, 0) && issue_S(I0{}, 0, 1) && issue_dP(0);
+      for (int it = 0; it < n_it && ok; it += 2) {
+        ok = step(I0{}, I1{}, it);
+        if (ok && it + 1 < n_it) ok = step(I1{}, I0{}, it + 1);
       }
     }
     __syncwarp();

@@ -65,7 +65,7 @@ __device__ __forceinline__ void wide_walk(const CUtensorMap* mR1, const CUtensor
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* status = a.status;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int g = a.Hq / a.Hkv;
   // rows: first row of the resident tile, its head and live rows; the stream: first row, rows per head and heads to walk
   int row0, nrow, rhead, n_it, per_head = 1, str0, shead0;
@@ -152,50 +152,63 @@ __device__ __forceinline__ void wide_walk(const CUtensorMap* mR1, const CUtensor
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_it > 0) {
+    // warp-uniform control flow, one lane issues (see uniform_warp)
+    if (n_it > 0) {
       constexpr uint32_t idX = umma_idesc_bf16(128, kWideCols, false, false);
       constexpr uint32_t idOut = umma_idesc_bf16(128, kWideHD, false, true);
       const uint32_t loR1 = desc_lo(smem_u32(sR1), 16), loR2 = desc_lo(smem_u32(sR2), 16);
-      const uint32_t aB1 = smem_u32(sB1), aB2 = smem_u32(sB2);
+      const uint32_t lo1 = desc_lo(smem_u32(sB1), 16), lo2 = desc_lo(smem_u32(sB2), 16), lo3 = desc_lo(smem_u32(HAS_Y ? sB1 : sB2), kWideCols * 128);
+      constexpr uint32_t kStep = kWideStr >> 4;
+      const bool leader = elect_one();
       bool ok = mbar_wait_bounded(r_full, 0, abort_flag, status, 4200);
-      // X (and Y) of iteration `it` into buffer it & 1. That buffer's previous content has been consumed: this thread has
+      // X (and Y) of iteration `it` into buffer it & 1. That buffer's previous content has been consumed: this warp has
       // waited for f of iteration it - 2 and issued its product, and products run in the order in which they are issued.
-      auto issue_xy = [&](int it) -> bool {
-        const int s = it & 1;
+      auto issue_xy = [&](auto sc, int it) -> bool {
+        constexpr int s = decltype(sc)::value;
         if (!mbar_wait_bounded(&b1_full[s], (it >> 1) & 1, abort_flag, status, 4210 + s)) return false;
         tc_fence_after();
-        const uint32_t lo1 = desc_lo(aB1 + s * kWideStr, 16);
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < kWideHD / 16; ++ks)
-          umma_bf16_ss(tX + s * kWideCols, desc_pack(loR1 + koff(ks, 128)), desc_pack(lo1 + koff(ks, kWideCols)), idX, ks ? 1u : 0u);
+          for (int ks = 0; ks < kWideHD / 16; ++ks)
+            umma_bf16_ss(tX + s * kWideCols, desc_pack(loR1 + koff(ks, 128)), desc_pack(lo1 + s * kStep + koff(ks, kWideCols)), idX, ks ? 1u : 0u);
+          if constexpr (!HAS_Y) umma_commit(&b1_empty[s]);
+        }
         if constexpr (HAS_Y) {
           if (!mbar_wait_bounded(&b2_full[0], it & 1, abort_flag, status, 4220)) return false;
           tc_fence_after();
-          const uint32_t lo2 = desc_lo(aB2, 16);
+          if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < kWideHD / 16; ++ks)
-            umma_bf16_ss(tY + s * kWideCols, desc_pack(loR2 + koff(ks, 128)), desc_pack(lo2 + koff(ks, kWideCols)), idX, ks ? 1u : 0u);
-          umma_commit(&b2_empty[0]);
-        } else {
-          umma_commit(&b1_empty[s]);
+            for (int ks = 0; ks < kWideHD / 16; ++ks)
+              umma_bf16_ss(tY + s * kWideCols, desc_pack(loR2 + koff(ks, 128)), desc_pack(lo2 + koff(ks, kWideCols)), idX, ks ? 1u : 0u);
+            umma_commit(&b2_empty[0]);
+          }
         }
-        umma_commit(&x_full[s]);
+        if (leader) umma_commit(&x_full[s]);
         return true;
       };
-      if (ok) ok = issue_xy(0);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it & 1;
-        if (it + 1 < n_it && !issue_xy(it + 1)) break;
-        if (!mbar_wait_bounded(&f_full[s], (it >> 1) & 1, abort_flag, status, 4230 + s)) break;
+      auto step = [&](auto sc, auto nc, int it) -> bool {
+        constexpr int s = decltype(sc)::value;
+        if (it + 1 < n_it && !issue_xy(nc, it + 1)) return false;
+        if (!mbar_wait_bounded(&f_full[s], (it >> 1) & 1, abort_flag, status, 4230 + s)) return false;
         if constexpr (!HAS_Y)
-          if (!mbar_wait_bounded(&b2_full[s], (it >> 1) & 1, abort_flag, status, 4240 + s)) break;
+          if (!mbar_wait_bounded(&b2_full[s], (it >> 1) & 1, abort_flag, status, 4240 + s)) return false;
         tc_fence_after();
-        const uint32_t lo3 = desc_lo((HAS_Y ? aB1 : aB2) + s * kWideStr, kWideCols * 128);
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < kWideCols / 16; ++ks)   // f: 8 columns per 16 of the contraction, each half of it over its half of X
-          umma_bf16_ts(tOut, tX + s * kWideCols + (ks >> 1) * 32 + (ks & 1) * 8, desc_pack(lo3 + mnoff(ks)), idOut, (it | ks) ? 1u : 0u);
-        umma_commit(HAS_Y ? &b1_empty[s] : &b2_empty[s]);
-        if (it == n_it - 1) umma_commit(out_done);
+          for (int ks = 0; ks < kWideCols / 16; ++ks)   // f: 8 columns per 16 of the contraction, each half of it over its half of X
+            umma_bf16_ts(tOut, tX + s * kWideCols + (ks >> 1) * 32 + (ks & 1) * 8, desc_pack(lo3 + s * kStep + mnoff(ks)), idOut,
+                         ks ? 1u : (it ? 1u : 0u));
+          umma_commit(HAS_Y ? &b1_empty[s] : &b2_empty[s]);
+          if (it == n_it - 1) umma_commit(out_done);
+        }
+        return true;
+      };
+      using I0 = std::integral_constant<int, 0>;
+      using I1 = std::integral_constant<int, 1>;
+      if (ok) ok = issue_xy(I0{}, 0);
+      for (int it = 0; it < n_it && ok; it += 2) {
+        ok = step(I0{}, I1{}, it);
+        if (ok && it + 1 < n_it) ok = step(I1{}, I0{}, it + 1);
       }
     }
     __syncwarp();

@@ -42,12 +42,12 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* v_full = bars + 5;    // [2]
   uint64_t* v_empty = bars + 7;   // [2]
   uint64_t* s_full = bars + 9;    // [2 heads]
-  uint64_t* p_full = bars + 11;   // [2 heads]
-  uint64_t* pv_done = bars + 13;  // [2 heads]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* p_full = bars + 11;   // [2 heads][2 halves of the keys]
+  uint64_t* pv_done = bars + 15;  // [2 heads]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int pairs = Hq >> 1;
   const int tile_idx = blockIdx.x / pairs;
   const int h0 = (blockIdx.x % pairs) * 2;            // heads h0, h0 + 1 share a key/value head (group size is even)
@@ -61,7 +61,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     mbar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
-      mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 128); mbar_init(&pv_done[s], 1);
+      mbar_init(&s_full[s], 1); mbar_init(&p_full[2 * s], 128); mbar_init(&p_full[2 * s + 1], 128); mbar_init(&pv_done[s], 1);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -112,44 +112,58 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_kv > 0) {
+    // warp-uniform control flow, one lane issues (see uniform_warp)
+    if (n_kv > 0) {
       constexpr uint32_t idS = umma_idesc_bf16(128, kPairKV, false, false);
       constexpr uint32_t idPV = umma_idesc_bf16(128, HD, false, true);
-      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
+      const uint32_t loQ = desc_lo(smem_u32(sQ), 16), loK = desc_lo(smem_u32(sK), 16), loV = desc_lo(smem_u32(sV), 16384);
+      const bool leader = elect_one();
       bool ok = mbar_wait_bounded(q_full, 0, abort_flag, status, 1600);
-      auto issue_S = [&](int j, int g) -> bool {            // S_g = Q_g K(j)^T
-        const int s = j & 1;
-        if (g == 0) {
+      auto issue_S = [&](auto sc, int j, auto gc) -> bool {            // S_g = Q_g K(j)^T
+        constexpr int s = decltype(sc)::value, g = decltype(gc)::value;
+        if constexpr (g == 0) {
           if (!mbar_wait_bounded(&k_full[s], (j >> 1) & 1, abort_flag, status, 1610 + s)) return false;
           tc_fence_after();
         }
-        const uint32_t loQ = desc_lo(aQ + g * kTile, 16), loK = desc_lo(aK + s * kTile, 16);
+        if (leader) {
 #pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks)
-          umma_bf16_ss(tS + g * 128, desc_pack(loQ + koff(ks, 128)), desc_pack(loK + koff(ks, 128)), idS, ks ? 1u : 0u);
-        umma_commit(&s_full[g]);
-        if (g == 1) umma_commit(&k_empty[s]);
+          for (int ks = 0; ks < HD / 16; ++ks)
+            umma_bf16_ss(tS + g * 128, desc_pack(loQ + g * (kTile >> 4) + koff(ks, 128)), desc_pack(loK + s * (kTile >> 4) + koff(ks, 128)), idS,
+                         ks ? 1u : 0u);
+          umma_commit(&s_full[g]);
+          if constexpr (g == 1) umma_commit(&k_empty[s]);
+        }
         return true;
       };
-      if (ok) ok = issue_S(0, 0) && issue_S(0, 1);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int s = j & 1;
-        const bool next = j + 1 < n_kv;
-        bool fail = false;
+      using I0 = std::integral_constant<int, 0>;
+      using I1 = std::integral_constant<int, 1>;
+      auto step = [&](auto sc, auto nc, int j) -> bool {              // tile j in stage s; the next tile's stage is n
+        constexpr int s = decltype(sc)::value;
+        auto head = [&](auto gc) -> bool {
+          constexpr int g = decltype(gc)::value;
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          if (!mbar_wait_bounded(&p_full[g], j & 1, abort_flag, status, 1620 + g)) { fail = true; break; }
-          if (g == 0 && !mbar_wait_bounded(&v_full[s], (j >> 1) & 1, abort_flag, status, 1630 + s)) { fail = true; break; }
-          tc_fence_after();
-          const uint32_t loVm = desc_lo(aV + s * kTile, 16384);
+          for (int hf = 0; hf < 2; ++hf) {                    // O_g += P_g V(j), P_g from tensor memory, 64 keys at a time
+            if (!mbar_wait_bounded(&p_full[2 * g + hf], j & 1, abort_flag, status, 1620 + 2 * g + hf)) return false;
+            if (g == 0 && hf == 0 && !mbar_wait_bounded(&v_full[s], (j >> 1) & 1, abort_flag, status, 1630 + s)) return false;
+            tc_fence_after();
+            if (leader) {
 #pragma unroll
-          for (int ks = 0; ks < kPairKV / 16; ++ks)           // O_g += P_g V(j), P_g from tensor memory
-            umma_bf16_ts(tO + g * HD, tS + g * 128 + ks * 8, desc_pack(loVm + mnoff(ks)), idPV, (j | ks) ? 1u : 0u);
-          umma_commit(&pv_done[g]);
-          if (g == 1) umma_commit(&v_empty[s]);
-          if (next && !issue_S(j + 1, g)) { fail = true; break; }   // refill the S buffer just consumed
-        }
-        if (fail) break;
+              for (int ks = hf * 4; ks < hf * 4 + 4; ++ks)
+                umma_bf16_ts(tO + g * HD, tS + g * 128 + ks * 8, desc_pack(loV + s * (kTile >> 4) + mnoff(ks)), idPV, ks ? 1u : (j ? 1u : 0u));
+            }
+          }
+          if (leader) {
+            umma_commit(&pv_done[g]);
+            if constexpr (g == 1) umma_commit(&v_empty[s]);
+          }
+          return j + 1 >= n_kv || issue_S(nc, j + 1, gc);     // refill the S buffer just consumed
+        };
+        return head(I0{}) && head(I1{});
+      };
+      if (ok) ok = issue_S(I0{}, 0, I0{}) && issue_S(I0{}, 0, I1{});
+      for (int j = 0; j < n_kv && ok; j += 2) {
+        ok = step(I0{}, I1{}, j);
+        if (ok && j + 1 < n_kv) ok = step(I1{}, I0{}, j + 1);
       }
     }
     __syncwarp();
@@ -168,24 +182,22 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_after();
       const int kbase = j * kPairKV;
       const bool need_mask = kbase + kPairKV > (causal ? min(klen, diag0) : klen);
-      // pass 1: running maximum of the row (four 32-column reads; eight independent maxima keep the chains short)
-      float mxs[8];
+      // the whole row of S is read once and stays in registers; three-input maxima, four independent chains
+      uint32_t r[kPairKV];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) mxs[q] = -INFINITY;
+      for (int c = 0; c < kPairKV / 32; ++c) tmem_ld_32x32(tSg + c * 32, r + c * 32);
+      tmem_wait_ld();
+      float mxs[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (need_mask) {
 #pragma unroll
-      for (int c = 0; c < kPairKV / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tSg + c * 32, r);
-        tmem_wait_ld();
-        if (need_mask) {
+        for (int i = 0; i < kPairKV; ++i) if (kbase + i < row_limit) mxs[i & 3] = fmaxf(mxs[i & 3], __uint_as_float(r[i]));
+      } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) if (kbase + c * 32 + i < row_limit) mxs[i & 7] = fmaxf(mxs[i & 7], __uint_as_float(r[i]));
-        } else {
+        for (int i = 0; i < kPairKV; i += 8)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mxs[i & 7] = fmaxf(mxs[i & 7], __uint_as_float(r[i]));
-        }
+          for (int q = 0; q < 4; ++q) mxs[q] = fmax3(mxs[q], __uint_as_float(r[i + 2 * q]), __uint_as_float(r[i + 2 * q + 1]));
       }
-      float mx = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])), fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7])));
+      float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3]));
       mx *= scale_log2;
       const float m_new = fmaxf(m_used, mx);
       const bool need = m_new > m_used + 8.f;  // lazy rescale: only when the running maximum moved by more than 2^8
@@ -207,31 +219,34 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tmem_wait_st();
         }
       }
-      // pass 2: P = exp2(S * c - m), packed bf16 over the columns already read; row sum in fp32
+      // P = exp2(S * c - m), packed bf16 over S; row sum in fp32 before the rounding. Each 64-key half is announced as soon as it
+      // is written, so its product runs under the exponentials of the other half.
       const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
-      float rsum[4] = {0.f, 0.f, 0.f, 0.f};
+      const float2 sc2 = make_float2(scale_log2, scale_log2), nm2 = make_float2(-m_safe, -m_safe);
+      float2 rsum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
       for (int c = 0; c < kPairKV / 32; ++c) {
-        uint32_t r[32], w[16];
-        tmem_ld_32x32(tSg + c * 32, r);
-        tmem_wait_ld();
+        uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0 = ex2(__uint_as_float(r[i]) * scale_log2 - m_safe);
-          float p1 = ex2(__uint_as_float(r[i + 1]) * scale_log2 - m_safe);
+          const int k = c * 32 + i;
+          const float2 t = ffma2(make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), sc2, nm2);
+          float2 p = make_float2(ex2(t.x), ex2(t.y));
           if (need_mask) {
-            if (kbase + c * 32 + i >= row_limit) p0 = 0.f;
-            if (kbase + c * 32 + i + 1 >= row_limit) p1 = 0.f;
+            if (kbase + k >= row_limit) p.x = 0.f;
+            if (kbase + k + 1 >= row_limit) p.y = 0.f;
           }
-          rsum[(i >> 1) & 3] += p0 + p1;
-          w[i >> 1] = pack_bf16x2(p0, p1);
+          rsum[(i >> 1) & 1] = fadd2(rsum[(i >> 1) & 1], p);
+          w[i >> 1] = pack_bf16x2(p.x, p.y);
         }
-        tmem_st_32x16(tSg + c * 16, w);       // columns [16c, 16c + 16) lie behind the read position 32c
+        tmem_st_32x16(tSg + c * 16, w);
+        if (c & 1) {
+          tmem_wait_st();
+          tc_fence_before();
+          mbar_arrive(&p_full[2 * g + (c >> 1)]);
+        }
       }
-      l += (rsum[0] + rsum[1]) + (rsum[2] + rsum[3]);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(&p_full[g]);
+      l += (rsum[0].x + rsum[0].y) + (rsum[1].x + rsum[1].y);
     }
     // ---- finalize
     if (ok && n_kv > 0) ok = mbar_wait_bounded(&pv_done[g], (n_kv - 1) & 1, abort_flag, status, 1720 + g);
