@@ -863,11 +863,8 @@ extern "C" int llmt_attn_bwd(const void* q, const void* k, const void* v, const 
   if ((HD != 64 && HD != 128) || Hq % Hkv || (q_stride & 7) || (k_stride & 7) || (v_stride & 7) || (do_stride & 7) ||
       (dq_stride & 7) || (dk_stride & 7) || (dv_stride & 7))
     return -10;
-  if (pass == 0) {
-    const int64_t items = (int64_t)Tq * Hq;
-    attn_delta_kernel<<<(int)((items + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)o, o_stride, (const __nv_bfloat16*)dout,
-                                                              do_stride, delta, Tq, Hq, HD);
-  }
+  if (pass == 0)
+    if (const int rc = launch_delta(o, o_stride, dout, do_stride, delta, nullptr, Tq, Hq, HD, st)) return rc;
   CUtensorMap tq, tk, tv, tdo;
   if (make_thd_map(&tq, q, Tq, Hq, HD, q_stride) || make_thd_map(&tk, k, Tk, Hkv, HD, k_stride) ||
       make_thd_map(&tv, v, Tk, Hkv, HD, v_stride) || make_thd_map(&tdo, dout, Tq, Hq, HD, do_stride))

@@ -423,9 +423,7 @@ extern "C" int llmt_attn_bwd_wide(const void* q, const void* k, const void* v, c
   if (Hq % Hkv || nsplit < 1 || (Hq / Hkv) % nsplit || (nsplit > 1 && part == nullptr) || (q_stride & 7) || (k_stride & 7) || (v_stride & 7) ||
       (do_stride & 7) || (dq_stride & 7) || (dk_stride & 7) || (dv_stride & 7))
     return -10;
-  const int64_t items = (int64_t)Tq * Hq;
-  attn_delta_kernel<<<(int)((items + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)o, o_stride, (const __nv_bfloat16*)dout, do_stride, delta, Tq, Hq,
-                                                            kWideHD);
+  if (const int rc = launch_delta(o, o_stride, dout, do_stride, delta, nullptr, Tq, Hq, kWideHD, st)) return rc;
   CUtensorMap q128, do128, k128, v128, q64, do64, k64, v64;
   if (make_thd_map(&q128, q, Tq, Hq, kWideHD, q_stride) || make_thd_map(&do128, dout, Tq, Hq, kWideHD, do_stride) ||
       make_thd_map(&k128, k, Tk, Hkv, kWideHD, k_stride) || make_thd_map(&v128, v, Tk, Hkv, kWideHD, v_stride) ||
