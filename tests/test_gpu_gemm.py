@@ -203,3 +203,36 @@ def test_gemm_pair_tiles(M, N, K, layout, accumulate):
         _close(out.contiguous(), ref + keep[1:M + 1, off:off + N].float() if accumulate else ref)
         big[1:M + 1, off:off + N] = keep[1:M + 1, off:off + N]
         assert torch.equal(big, keep)                 # nothing outside the output was touched
+
+
+@pytest.mark.parametrize("need", [(True, True, True), (False, True, False), (True, False, False)])
+@pytest.mark.parametrize("owned", [False, True])
+def test_native_linear_node_matches_the_python_node(need, owned):
+    """The C++ node of `ops.linears` against the Python node: equal bits for any subset of wanted gradients, 3-D rows, under
+    saved-tensor hooks, and when a weight gets an owner's gradient buffer between forward and backward."""
+    from torchllmtuner_b200 import ops
+    from torchllmtuner_b200.ops import functional as F
+    torch.manual_seed(0)
+    x = torch.randn(3, 70, 136, device="cuda").bfloat16().requires_grad_(need[0])
+    ws = [torch.randn(n, 136, device="cuda").bfloat16().requires_grad_(q) for n, q in ((264, need[1]), (64, need[2]))]
+    dys = [torch.randn(3, 70, w.shape[0], device="cuda").bfloat16() for w in ws]
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.shape) or t.clone(), lambda t: t):
+        hooked = ops.linears(x, *ws)
+    got, want = ops.linears(x, *ws), F._MultiLinear.apply(x, *ws)
+    assert len(packed) == 3                                    # the rows and both weights went through the hooks
+    leaves = [t for t in (x, *ws) if t.requires_grad]
+
+    def grads(ys):
+        for w in ws:
+            if owned:                                          # what an FSDP unit does before its block's backward
+                w.main_grad, w.main_grad_initialized = torch.full_like(w, 7.0), False
+        g = torch.autograd.grad(ys, leaves, dys, allow_unused=True, retain_graph=True)
+        return list(g) + [w.main_grad.clone() for w in ws if owned]
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    for a, b in zip(grads(got), grads(want)):
+        assert (a is None and b is None) or torch.equal(a, b)
+    if not owned:
+        for a, b in zip(grads(hooked), grads(want)):
+            assert torch.equal(a, b)

@@ -2,6 +2,8 @@
 // done on the host (dtype, device, contiguity, alignment) are done here so the kernels can assume them.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
 #include "kernels.h"
@@ -734,6 +736,196 @@ std::vector<Tensor> combine_bwd(const Tensor& dout, const Tensor& y, const Tenso
   return {dy, dw};
 }
 
+// ---- autograd nodes of the small hot ops
+// A launch of a small training step takes the device a few microseconds and took the host 20 to 27: the Python frames of
+// apply() and backward(), reshapes, allocations and attribute look-ups around one kernel call. These nodes do the same with the
+// same kernels in C++. What needs Python stays there: a pending peer-memory collective (it rides on the product, so the
+// queue decides) and weights whose gradient accumulates into an owner's buffer (`main_grad`) hand the whole backward to
+// `functional._linears_backward`. Saved tensors go through the usual hooks (activation checkpointing, offload).
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+using OptTensor = c10::optional<Tensor>;
+
+struct PyHooks {
+  PyObject* symm = nullptr;               // module that holds the active collective queue (`_ACTIVE`)
+  PyObject* linears_backward = nullptr;   // functional._linears_backward(x2, ws, dys, need_x, need_ws)
+};
+PyHooks& py_hooks() {
+  static PyHooks h;                       // references are kept for the life of the process
+  return h;
+}
+void set_autograd_hooks(const py::object& symm, const py::object& linears_backward) {
+  PyHooks& h = py_hooks();
+  py::object a = symm, b = linears_backward;
+  Py_XDECREF(h.symm);
+  Py_XDECREF(h.linears_backward);
+  h.symm = a.release().ptr();
+  h.linears_backward = b.release().ptr();
+}
+// With the GIL held: is a collective queue active, or does one of the weights own a gradient buffer?
+bool python_takes_backward(const variable_list& ws) {
+  const PyHooks& h = py_hooks();
+  TORCH_CHECK(h.symm != nullptr && h.linears_backward != nullptr, "set_autograd_hooks was not called");
+  py::object active = py::reinterpret_steal<py::object>(PyObject_GetAttrString(h.symm, "_ACTIVE"));
+  if (!active) throw py::error_already_set();
+  if (!active.is_none()) return true;
+  for (const Tensor& w : ws) {
+    py::object pw = py::reinterpret_steal<py::object>(THPVariable_Wrap(w));
+    if (!pw) throw py::error_already_set();
+    if (!PyObject_HasAttrString(pw.ptr(), "main_grad")) continue;
+    if (!py::object(pw.attr("main_grad")).is_none()) return true;
+  }
+  return false;
+}
+
+Tensor rows_2d(const Tensor& t) {
+  Tensor r = t.dim() == 2 ? t : t.reshape({-1, t.size(-1)});
+  return r.stride(1) == 1 ? r : r.contiguous();
+}
+Tensor like_rows(const Tensor& x, int64_t n) {         // empty tensor of x's shape with the last dimension replaced
+  auto sz = x.sizes().vec();
+  sz.back() = n;
+  return torch::empty(sz, x.options());
+}
+
+// y_i = x W_i^T for one to three weights that read the same rows. dx is summed by the products' epilogues.
+struct NativeLinears : public torch::autograd::Function<NativeLinears> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w0, const OptTensor& w1, const OptTensor& w2) {
+    Tensor x2 = rows_2d(x);
+    variable_list saved{x2, w0}, ys;
+    if (w1.has_value()) saved.push_back(*w1);
+    if (w2.has_value()) saved.push_back(*w2);
+    for (size_t i = 1; i < saved.size(); ++i) {
+      Tensor y = like_rows(x, saved[i].size(0)), y2 = y.view({-1, saved[i].size(0)});
+      gemm(x2, saved[i], y2, false, false, false, 0, c10::nullopt);
+      ys.push_back(y);
+    }
+    ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->save_for_backward(saved);
+    return ys;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list dys) {
+    variable_list saved = ctx->get_saved_variables();
+    const Tensor x2 = saved[0];
+    const variable_list ws(saved.begin() + 1, saved.end());
+    const std::vector<int64_t> shape = ctx->saved_data["shape"].toIntVector();
+    variable_list out(4);
+    const bool need_x = ctx->needs_input_grad(0);
+    variable_list d2;
+    for (const Tensor& d : dys) d2.push_back(rows_2d(d));
+    {
+      py::gil_scoped_acquire gil;
+      try {
+        if (python_takes_backward(ws)) {
+          std::vector<bool> need_w;
+          for (size_t i = 0; i < ws.size(); ++i) need_w.push_back(ctx->needs_input_grad(1 + i));
+          py::object fn = py::reinterpret_borrow<py::object>(py_hooks().linears_backward);
+          auto r = fn(x2, ws, d2, need_x, need_w).cast<std::vector<OptTensor>>();
+          for (size_t i = 0; i < r.size() && i < out.size(); ++i)
+            if (r[i].has_value()) out[i] = i == 0 ? r[i]->reshape(shape) : *r[i];
+          return out;
+        }
+      } catch (py::error_already_set& e) {
+        e.restore();                      // the engine carries a python_error, type and all, to the thread that called backward
+        throw python_error();
+      }
+    }
+    for (size_t i = 0; i < ws.size(); ++i) {
+      if (need_x) {
+        if (i == 0) out[0] = torch::empty(shape, x2.options());
+        Tensor dx = out[0].view({-1, x2.size(1)});
+        gemm(d2[i], ws[i], dx, false, true, i > 0, 0, c10::nullopt);               // dy [M,N] @ W [N,K]
+      }
+      if (ctx->needs_input_grad(1 + i)) {
+        out[1 + i] = torch::empty(ws[i].sizes(), ws[i].options());
+        gemm(d2[i], x2, out[1 + i], true, true, false, 0, c10::nullopt);           // dy^T [N,M] @ x [M,K]
+      }
+    }
+    return out;
+  }
+};
+variable_list linears_node(const Tensor& x, const variable_list& ws) {
+  TORCH_CHECK(ws.size() >= 1 && ws.size() <= 3, "one to three weights");
+  return NativeLinears::apply(x, ws[0], ws.size() > 1 ? OptTensor(ws[1]) : OptTensor(), ws.size() > 2 ? OptTensor(ws[2]) : OptTensor());
+}
+
+struct NativeSwiGLU : public torch::autograd::Function<NativeSwiGLU> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& gate, const Tensor& up, const OptTensor& row_limit) {
+    Tensor g2 = rows_2d(gate), u2 = rows_2d(up);
+    if (g2.stride(0) != u2.stride(0)) { g2 = g2.contiguous(); u2 = u2.contiguous(); }
+    ctx->save_for_backward({g2, u2, row_limit.has_value() ? *row_limit : Tensor()});
+    ctx->saved_data["shape"] = gate.sizes().vec();
+    return swiglu_fwd(g2, u2, row_limit).view(gate.sizes());
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list d) {
+    variable_list s = ctx->get_saved_variables();
+    const Tensor &g2 = s[0], &u2 = s[1];
+    const std::vector<int64_t> shape = ctx->saved_data["shape"].toIntVector();
+    const int64_t F = g2.size(1);
+    Tensor both = torch::empty({g2.size(0), 2 * F}, g2.options());
+    Tensor dg = both.narrow(1, 0, F), du = both.narrow(1, F, F);
+    swiglu_bwd(rows_2d(d[0]), g2, u2, dg, du, s[2].defined() ? OptTensor(s[2]) : OptTensor());
+    return {shape.size() == 2 ? dg : dg.reshape(shape), shape.size() == 2 ? du : du.reshape(shape), Tensor()};
+  }
+};
+
+struct NativeRMSNorm : public torch::autograd::Function<NativeRMSNorm> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, double eps) {
+    Tensor xc = x.contiguous();
+    auto r = rmsnorm_fwd(xc, c10::nullopt, w, eps);
+    ctx->save_for_backward({xc, w, r[1]});
+    return r[0];
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list d) {
+    variable_list s = ctx->get_saved_variables();
+    auto r = rmsnorm_bwd(d[0].contiguous(), s[0], s[1], s[2], c10::nullopt, true);
+    return {r[0], r[1], Tensor()};
+  }
+};
+struct NativeAddRMSNorm : public torch::autograd::Function<NativeAddRMSNorm> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& res, const Tensor& w, double eps) {
+    auto r = rmsnorm_fwd(x.contiguous(), res.contiguous(), w, eps);
+    ctx->save_for_backward({r[2], w, r[1]});
+    return {r[0], r[2]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list d) {
+    variable_list s = ctx->get_saved_variables();
+    auto r = rmsnorm_bwd(d[0].contiguous(), s[0], s[1], s[2], d[1].contiguous(), true);
+    return {r[0], r[0], r[1], Tensor()};
+  }
+};
+
+// q and k of one attention layer: two independent halves in one node.
+struct NativeQKNormRope : public torch::autograd::Function<NativeQKNormRope> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const OptTensor& qw, const OptTensor& kw, const Tensor& cosb,
+                               const Tensor& sinb, double eps) {
+    auto a = qk_norm_rope_fwd(q, qw, cosb, sinb, eps), b = qk_norm_rope_fwd(k, kw, cosb, sinb, eps);
+    ctx->save_for_backward({q, k, qw.has_value() ? *qw : Tensor(), kw.has_value() ? *kw : Tensor(), cosb, sinb, a[1], b[1]});
+    ctx->set_materialize_grads(false);
+    return {a[0], b[0]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list d) {
+    variable_list s = ctx->get_saved_variables(), out(7);
+    for (int i = 0; i < 2; ++i) {
+      if (!d[i].defined()) continue;
+      Tensor dy = d[i];
+      if (dy.stride(2) != 1 || dy.stride(1) != dy.size(2)) dy = dy.contiguous();
+      const Tensor& w = s[2 + i];
+      const bool w16 = w.defined() && w.scalar_type() == at::kBFloat16;
+      auto r = qk_norm_rope_bwd(dy, s[i], w.defined() ? OptTensor(w) : OptTensor(), s[4], s[5], s[6 + i], w16);
+      out[i] = r[0];
+      if (w.defined()) out[2 + i] = w16 ? r[1] : r[1].to(w.scalar_type());
+    }
+    return out;
+  }
+};
+Tensor swiglu_node(const Tensor& g, const Tensor& u, const OptTensor& row_limit) { return NativeSwiGLU::apply(g, u, row_limit); }
+Tensor rmsnorm_node(const Tensor& x, const Tensor& w, double eps) { return NativeRMSNorm::apply(x, w, eps); }
+variable_list add_rmsnorm_node(const Tensor& x, const Tensor& r, const Tensor& w, double eps) { return NativeAddRMSNorm::apply(x, r, w, eps); }
+variable_list qk_norm_rope_node(const Tensor& q, const Tensor& k, const OptTensor& qw, const OptTensor& kw, const Tensor& cosb, const Tensor& sinb, double eps) {
+  return NativeQKNormRope::apply(q, k, qw, kw, cosb, sinb, eps);
+}
+
 // Reads the status word (synchronises the current stream) and clears it. Returns {code, site, block, extra}.
 std::vector<int64_t> read_status(bool clear) {
   Tensor h = status_word().cpu();
@@ -759,6 +951,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("wait_value", &PySideJob::wait_value);
   m.def("gemm", &gemm, "bf16 tcgen05 GEMM", py::arg("a"), py::arg("b"), py::arg("out"), py::arg("a_mn"), py::arg("b_mn"),
         py::arg("accumulate") = false, py::arg("max_ctas") = 0, py::arg("side") = py::none());
+  m.def("set_autograd_hooks", &set_autograd_hooks);
+  m.def("linears_node", &linears_node);
+  m.def("swiglu_node", &swiglu_node);
+  m.def("rmsnorm_node", &rmsnorm_node);
+  m.def("add_rmsnorm_node", &add_rmsnorm_node);
+  m.def("qk_norm_rope_node", &qk_norm_rope_node);
   m.def("router_topk", &router_topk);
   m.def("router_topk_bwd", &router_topk_bwd);
   m.def("moe_plan", &moe_plan);

@@ -18,9 +18,34 @@ from .cuda_ext import load as _ext
 IGNORE_INDEX = ref.IGNORE_INDEX
 
 
+_symm = None
+
+
+def _symm_module():
+    """parallel.symm, imported on first use (it imports the extension's loader, and this module is imported by models first)."""
+    global _symm
+    if _symm is None:
+        from ..parallel import symm
+        _symm = symm
+    return _symm
+
+
 def _comm_queue():
-    from ..parallel import symm
-    return symm._ACTIVE
+    return _symm_module()._ACTIVE
+
+
+_nodes = None
+
+
+def _native():
+    """The extension with its C++ autograd nodes, or None while a peer-memory collective queue is active (products then go
+    through `gemm`, which hands the queue's next job to the kernel)."""
+    global _nodes
+    if _nodes is None:
+        ext = _ext()
+        ext.set_autograd_hooks(_symm_module(), _linears_backward)
+        _nodes = ext
+    return _nodes if _symm._ACTIVE is None else None
 
 
 def _use_cuda(t: torch.Tensor) -> bool:
@@ -178,29 +203,34 @@ class _MultiLinear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *dys):
         x2, *ws = ctx.saved_tensors
-        dx = None
-        if ctx.needs_input_grad[0]:
-            for dy, w in zip(dys, ws):
-                if dy is None:
-                    continue
-                if dx is None:
-                    dx = gemm(_2d(dy), w, b_mn=True)
-                else:
-                    gemm(_2d(dy), w, b_mn=True, out=dx, accumulate=True)
-            dx = None if dx is None else dx.reshape(ctx.xshape)
-        dws = []
-        for i, (dy, w) in enumerate(zip(dys, ws)):
-            if dy is None or not ctx.needs_input_grad[1 + i]:
-                dws.append(None)
+        dx, *dws = _linears_backward(x2, ws, dys, ctx.needs_input_grad[0], ctx.needs_input_grad[1:])
+        return (None if dx is None else dx.reshape(ctx.xshape), *dws)
+
+
+def _linears_backward(x2, ws, dys, need_x, need_ws):
+    """[dx rows, dw_0, ...] of y_i = x2 W_i^T; gradients of weights with an owner's buffer (`main_grad`) go there instead."""
+    dx = None
+    if need_x:
+        for dy, w in zip(dys, ws):
+            if dy is None:
                 continue
-            main = getattr(w, "main_grad", None)
-            if main is not None:
-                gemm(_2d(dy), x2, a_mn=True, b_mn=True, out=main, accumulate=getattr(w, "main_grad_initialized", False))
-                w.main_grad_initialized = True
-                dws.append(None)
+            if dx is None:
+                dx = gemm(_2d(dy), w, b_mn=True)
             else:
-                dws.append(gemm(_2d(dy), x2, a_mn=True, b_mn=True, out_dtype=w.dtype))
-        return (dx, *dws)
+                gemm(_2d(dy), w, b_mn=True, out=dx, accumulate=True)
+    dws = []
+    for dy, w, need in zip(dys, ws, need_ws):
+        if dy is None or not need:
+            dws.append(None)
+            continue
+        main = getattr(w, "main_grad", None)
+        if main is not None:                                                       # accumulate straight into the owner's buffer
+            gemm(_2d(dy), x2, a_mn=True, b_mn=True, out=main, accumulate=getattr(w, "main_grad_initialized", False))
+            w.main_grad_initialized = True
+            dws.append(None)
+        else:
+            dws.append(gemm(_2d(dy), x2, a_mn=True, b_mn=True, out_dtype=w.dtype))
+    return [dx, *dws]
 
 
 def linears(x: torch.Tensor, *ws: torch.Tensor):
@@ -208,7 +238,8 @@ def linears(x: torch.Tensor, *ws: torch.Tensor):
     (CPU, odd shapes, and under per-op checkpointing, whose keep / replay bookkeeping is per projection)."""
     if (_SAC is None and _use_cuda(x) and x.dtype == torch.bfloat16 and len(ws) > 1
             and not any(w.shape[0] % 8 or w.shape[1] % 8 for w in ws)):
-        return _MultiLinear.apply(x, *ws)
+        ext = _native() if len(ws) <= 3 and _all_bf16(ws) else None
+        return tuple(ext.linears_node(x, ws)) if ext is not None else _MultiLinear.apply(x, *ws)
     return tuple(linear(x, w) for w in ws)
 
 
@@ -224,50 +255,29 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
             return y
         kept = frame.take()
         return _Linear.apply(x, w, kept) if kernel else _KeptLinear.apply(x, w, kept)
-    return _Linear.apply(x, w) if kernel else ref.linear(x, w)
+    if not kernel:
+        return ref.linear(x, w)
+    ext = _native() if w.dtype == torch.bfloat16 and w.is_cuda else None
+    return ext.linears_node(x, (w,))[0] if ext is not None else _Linear.apply(x, w)
+
+
+def _all_bf16(ws) -> bool:
+    return all(w.dtype == torch.bfloat16 and w.is_cuda for w in ws)
 
 
 # ----------------------------------------------------------------------------------------------- RMSNorm
-class _RMSNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, eps):
-        xc = _c(x)
-        y, rstd = _ext().rmsnorm_fwd(xc, None, w, eps)
-        ctx.save_for_backward(xc, w, rstd)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, w, rstd = ctx.saved_tensors
-        dx, dw = _ext().rmsnorm_bwd(_c(dy), x, w, rstd, None, True)        # the weight is bf16: the forward checked it
-        return dx, dw, None
-
-
-class _AddRMSNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, res, w, eps):
-        y, rstd, s = _ext().rmsnorm_fwd(_c(x), _c(res), w, eps)
-        ctx.save_for_backward(s, w, rstd)
-        return y, s
-
-    @staticmethod
-    def backward(ctx, dy, ds):
-        s, w, rstd = ctx.saved_tensors
-        dsum, dw = _ext().rmsnorm_bwd(_c(dy), s, w, rstd, _c(ds) if ds is not None else None, True)
-        return dsum, dsum, dw, None
-
-
 def rms_norm(x, weight, eps: float):
-    validate_rms_norm_inputs(x, weight)
+    if not (isinstance(x, torch.Tensor) and isinstance(weight, torch.Tensor) and weight.dim() == 1 and x.shape[-1] == weight.shape[0]):
+        validate_rms_norm_inputs(x, weight)
     if _use_cuda(x) and x.dtype == torch.bfloat16:
-        return _RMSNorm.apply(x, weight, eps)
+        return _ext().rmsnorm_node(x, weight, eps)
     return ref.rms_norm(x, weight, eps)
 
 
 def add_rms_norm(x, residual, weight, eps: float):
     """Returns (rms_norm(x + residual), x + residual) with one pass over the data."""
     if _use_cuda(x) and x.dtype == torch.bfloat16:
-        return _AddRMSNorm.apply(x, residual, weight, eps)
+        return tuple(_ext().add_rmsnorm_node(x, residual, weight, eps))
     return ref.add_rms_norm(x, residual, weight, eps)
 
 
@@ -275,56 +285,19 @@ def add_rms_norm(x, residual, weight, eps: float):
 rope_tables = ref.rope_tables
 
 
-class _QKNormRope(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, cos, sin, eps):
-        y, rstd = _ext().qk_norm_rope_fwd(x, w, cos, sin, eps)
-        ctx.save_for_backward(x, w if w is not None else torch.empty(0), cos, sin, rstd)
-        ctx.has_w = w is not None
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, w, cos, sin, rstd = ctx.saved_tensors
-        if dy.stride(2) != 1 or dy.stride(1) != dy.shape[2]:
-            dy = dy.contiguous()
-        out = _ext().qk_norm_rope_bwd(dy, x, w if ctx.has_w else None, cos, sin, rstd, ctx.has_w and w.dtype == torch.bfloat16)
-        return out[0], (out[1].to(w.dtype) if ctx.has_w else None), None, None, None
-
-
 def qk_norm_rope(q, k, q_weight, k_weight, cos, sin, eps: float):
     """q [T,Hq,d], k [T,Hkv,d] (views with packed heads are fine); cos/sin fp32 [T,d/2]."""
     if _use_cuda(q) and q.dtype == torch.bfloat16:
-        return _QKNormRope.apply(q, q_weight, cos, sin, eps), _QKNormRope.apply(k, k_weight, cos, sin, eps)
+        return tuple(_ext().qk_norm_rope_node(q, k, q_weight, k_weight, cos, sin, eps))
     return ref.qk_norm_rope(q, k, q_weight, k_weight, cos, sin, eps)
 
 
 # ----------------------------------------------------------------------------------------------- SwiGLU
-class _SwiGLU(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, gate, up, row_limit):
-        g2, u2 = _2d(gate), _2d(up)
-        if g2.stride(0) != u2.stride(0):
-            g2, u2 = g2.contiguous(), u2.contiguous()
-        ctx.save_for_backward(g2, u2)
-        ctx.shape, ctx.row_limit = gate.shape, row_limit
-        return _ext().swiglu_fwd(g2, u2, row_limit).reshape(gate.shape)
-
-    @staticmethod
-    def backward(ctx, dout):
-        g2, u2 = ctx.saved_tensors
-        d2 = _2d(dout)
-        both = torch.empty(g2.shape[0], 2 * g2.shape[1], dtype=g2.dtype, device=g2.device)
-        dg, du = both[:, :g2.shape[1]], both[:, g2.shape[1]:]
-        _ext().swiglu_bwd(d2, g2, u2, dg, du, ctx.row_limit)
-        return dg.reshape(ctx.shape), du.reshape(ctx.shape), None
-
-
 def swiglu(gate, up, row_limit=None):
     """silu(gate) * up. `row_limit` (int32 device scalar) bounds the rows that are touched when the operands are
     statically sized buffers whose live row count is only known on the device (expert-parallel receive buffers)."""
     if _use_cuda(gate) and gate.dtype == torch.bfloat16:
-        return _SwiGLU.apply(gate, up, row_limit)
+        return _ext().swiglu_node(gate, up, row_limit)
     return ref.swiglu(gate, up)
 
 
