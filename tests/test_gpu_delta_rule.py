@@ -1,0 +1,70 @@
+"""Kernels of the gated delta rule mixers vs plain PyTorch statements in 32 and 64 bits."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+from tolerances import ELEMENTWISE, REDUCED, assert_close
+
+
+def _close(a, b, name, reduced=False):
+    assert_close(a, b, name=name, **(REDUCED if reduced else ELEMENTWISE))
+
+
+@pytest.mark.parametrize("cuts,C,K", [([0, 1], 8, 4), ([0, 3, 4, 21], 16, 4), ([0, 16, 33], 1032, 2), ([0, 15, 31, 100], 2056, 3), ([0, 700], 264, 4)])
+def test_causal_conv_silu(cuts, C, K):
+    """Documents shorter than the kernel, cuts on and off the 16-row blocks, channel counts that leave threads idle."""
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(C)
+    T = cuts[-1]
+    x, dy = (torch.randn(T, C, device="cuda").bfloat16() for _ in range(2))
+    w = (0.5 * torch.randn(C, K, device="cuda")).bfloat16()
+    pos = torch.cat([torch.arange(b - a, device="cuda") for a, b in zip(cuts[:-1], cuts[1:])])
+    a = [t.clone().requires_grad_() for t in (x, w)]
+    y = ops.causal_conv_silu(*a, pos)
+    g = torch.autograd.grad(y, a, dy)
+    b = [t.double().requires_grad_() for t in (x, w)]
+    z = []
+    for s, e in zip(cuts[:-1], cuts[1:]):
+        p = F.pad(b[0][s:e], (0, 0, K - 1, 0))
+        z.append(sum(p[j:j + e - s] * b[1][:, j] for j in range(K)))
+    want = F.silu(torch.cat(z))
+    gw = torch.autograd.grad(want, b, dy.double())
+    _close(y, want.float(), "y"); _close(g[0], gw[0].float(), "dx"); _close(g[1], gw[1].float(), "dw", True)
+
+
+@pytest.mark.parametrize("T,Hk,Hv,d", [(1, 1, 1, 64), (7, 2, 6, 64), (33, 4, 8, 128), (5, 1, 2, 256)])
+def test_delta_qkv(T, Hk, Hv, d):
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(T)
+    x = torch.randn(T, (2 * Hk + Hv) * d, device="cuda").bfloat16().requires_grad_()
+    got = ops.delta_qkv(x, Hk, Hv, d, d, d ** -0.5, 1e-6)
+    xd = x.detach().double().requires_grad_()
+    q, k, v = xd[:, :Hk * d].view(T, Hk, d), xd[:, Hk * d:2 * Hk * d].view(T, Hk, d), xd[:, 2 * Hk * d:].view(T, Hv, d)
+    q, k = (t * torch.rsqrt(t.square().sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+    want = ((q * d ** -0.5).repeat_interleave(Hv // Hk, 1), k.repeat_interleave(Hv // Hk, 1), v)
+    for a, b in zip(got, want):
+        assert a.dtype == torch.float32 and torch.allclose(a.double(), b, rtol=1e-5, atol=1e-6)
+    dys = [torch.randn_like(t) for t in got]
+    (g,) = torch.autograd.grad(got, x, dys)
+    (gw,) = torch.autograd.grad(want, xd, [t.double() for t in dys])
+    _close(g, gw.float(), "dmixed")
+
+
+@pytest.mark.parametrize("R,D", [(1, 64), (37, 128), (1000, 128), (65, 256)])
+def test_gated_rms_norm(R, D):
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(R)
+    x, gate, dy = (torch.randn(R, D, device="cuda").bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+    a = [t.clone().requires_grad_() for t in (x, gate, w)]
+    y = ops.gated_rms_norm(*a, 1e-6)
+    g = torch.autograd.grad(y, a, dy)
+    b = [t.double().requires_grad_() for t in (x, gate, w)]
+    want = b[0] * torch.rsqrt(b[0].square().mean(-1, keepdim=True) + 1e-6) * b[2] * F.silu(b[1])
+    gw = torch.autograd.grad(want, b, dy.double())
+    _close(y, want.float(), "y")
+    for n, p, q in zip(("dx", "dgate", "dw"), g, gw):
+        _close(p, q.float(), n, n == "dw")
+

@@ -736,6 +736,80 @@ std::vector<Tensor> combine_bwd(const Tensor& dout, const Tensor& y, const Tenso
   return {dy, dw};
 }
 
+// ---- around the gated delta rule
+static void check_conv(const Tensor& x, const Tensor& w, const Tensor& pos) {
+  check_bf16(x, "x");
+  check_bf16(w, "w");
+  TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && w.dim() == 2 && w.is_contiguous() && w.size(0) == x.size(1), "x [T, C], w [C, K]");
+  TORCH_CHECK(pos.is_cuda() && pos.scalar_type() == at::kLong && pos.is_contiguous() && pos.numel() == x.size(0), "positions must be int64 [T]");
+}
+Tensor conv_silu_fwd(const Tensor& x, const Tensor& w, const Tensor& pos) {
+  c10::cuda::CUDAGuard guard(x.device());
+  check_conv(x, w, pos);
+  Tensor y = torch::empty(x.sizes(), x.options());
+  check_rc(llmt_conv_silu_fwd(x.data_ptr(), x.stride(0), w.data_ptr(), pos.data_ptr<int64_t>(), y.data_ptr(), (int)x.size(0), (int)x.size(1),
+                              (int)w.size(1), cur_stream()),
+           "llmt_conv_silu_fwd");
+  return y;
+}
+std::vector<Tensor> conv_silu_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& pos) {
+  c10::cuda::CUDAGuard guard(x.device());
+  check_conv(x, w, pos);
+  check_bf16(dy, "dy");
+  TORCH_CHECK(dy.sizes() == x.sizes() && dy.stride(1) == 1);
+  const int T = (int)x.size(0), C = (int)x.size(1), K = (int)w.size(1);
+  Tensor dx = torch::empty(x.sizes(), x.options()), dw = T > 0 ? torch::empty(w.sizes(), w.options()) : torch::zeros(w.sizes(), w.options());
+  Tensor part = torch::empty({llmt_conv_silu_blocks(T), C, K}, x.options().dtype(at::kFloat));
+  check_rc(llmt_conv_silu_bwd(dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), w.data_ptr(), pos.data_ptr<int64_t>(), dx.data_ptr(),
+                              part.data_ptr<float>(), dw.data_ptr(), T, C, K, cur_stream()),
+           "llmt_conv_silu_bwd", 2);
+  return {dx, dw};
+}
+// mixed [T, (2 Hk + Hv) d] -> q, k [T, Hv, d], v [T, Hv, d] fp32
+std::vector<Tensor> delta_qkv_fwd(const Tensor& mixed, int64_t Hk, int64_t Hv, double qscale, double eps) {
+  c10::cuda::CUDAGuard guard(mixed.device());
+  check_bf16(mixed, "mixed");
+  TORCH_CHECK(mixed.dim() == 2 && mixed.is_contiguous() && Hk > 0 && mixed.size(1) % (2 * Hk + Hv) == 0);
+  const int64_t T = mixed.size(0), d = mixed.size(1) / (2 * Hk + Hv);
+  auto o = mixed.options().dtype(at::kFloat);
+  Tensor q = torch::empty({T, Hv, d}, o), k = torch::empty({T, Hv, d}, o), v = torch::empty({T, Hv, d}, o);
+  check_rc(llmt_delta_qkv_fwd(mixed.data_ptr(), q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), (int)T, (int)Hk, (int)Hv, (int)d,
+                              (float)qscale, (float)eps, cur_stream()),
+           "llmt_delta_qkv_fwd");
+  return {q, k, v};
+}
+Tensor delta_qkv_bwd(const Tensor& dq, const Tensor& dk, const Tensor& dv, const Tensor& mixed, int64_t Hk, int64_t Hv, double qscale, double eps) {
+  c10::cuda::CUDAGuard guard(mixed.device());
+  for (const Tensor* t : {&dq, &dk, &dv}) TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->sizes() == dq.sizes());
+  Tensor dm = torch::empty_like(mixed);
+  check_rc(llmt_delta_qkv_bwd(dq.data_ptr<float>(), dk.data_ptr<float>(), dv.data_ptr<float>(), mixed.data_ptr(), dm.data_ptr(), (int)mixed.size(0),
+                              (int)Hk, (int)Hv, (int)dq.size(2), (float)qscale, (float)eps, cur_stream()),
+           "llmt_delta_qkv_bwd");
+  return dm;
+}
+Tensor gated_norm_fwd(const Tensor& x, const Tensor& gate, const Tensor& w, double eps) {
+  c10::cuda::CUDAGuard guard(x.device());
+  check_bf16(x, "x"); check_bf16(gate, "gate"); check_bf16(w, "w");
+  TORCH_CHECK(x.is_contiguous() && gate.is_contiguous() && w.is_contiguous() && x.sizes() == gate.sizes() && x.size(-1) == w.numel());
+  Tensor y = torch::empty_like(x);
+  check_rc(llmt_gated_norm_fwd(x.data_ptr(), gate.data_ptr(), w.data_ptr(), y.data_ptr(), x.numel() / x.size(-1), (int)x.size(-1), (float)eps,
+                               cur_stream()),
+           "llmt_gated_norm_fwd");
+  return y;
+}
+std::vector<Tensor> gated_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& gate, const Tensor& w, double eps) {
+  c10::cuda::CUDAGuard guard(x.device());
+  check_bf16(dy, "dy");
+  TORCH_CHECK(dy.is_contiguous() && dy.sizes() == x.sizes());
+  const int64_t D = x.size(-1), R = x.numel() / D;
+  Tensor dx = torch::empty_like(x), dg = torch::empty_like(x), dw = R > 0 ? torch::empty_like(w) : torch::zeros_like(w);
+  Tensor part = torch::empty({llmt_gated_norm_bwd_blocks(R, (int)D), D}, x.options().dtype(at::kFloat));
+  check_rc(llmt_gated_norm_bwd(dy.data_ptr(), x.data_ptr(), gate.data_ptr(), w.data_ptr(), dx.data_ptr(), dg.data_ptr(), part.data_ptr<float>(),
+                               dw.data_ptr(), R, (int)D, (float)eps, cur_stream()),
+           "llmt_gated_norm_bwd", 2);
+  return {dx, dg, dw};
+}
+
 // ---- autograd nodes of the small hot ops
 // A launch of a small training step takes the device a few microseconds and took the host 20 to 27: the Python frames of
 // apply() and backward(), reshapes, allocations and attribute look-ups around one kernel call. These nodes do the same with the
@@ -951,6 +1025,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("wait_value", &PySideJob::wait_value);
   m.def("gemm", &gemm, "bf16 tcgen05 GEMM", py::arg("a"), py::arg("b"), py::arg("out"), py::arg("a_mn"), py::arg("b_mn"),
         py::arg("accumulate") = false, py::arg("max_ctas") = 0, py::arg("side") = py::none());
+  m.def("conv_silu_fwd", &conv_silu_fwd);
+  m.def("conv_silu_bwd", &conv_silu_bwd);
+  m.def("delta_qkv_fwd", &delta_qkv_fwd);
+  m.def("delta_qkv_bwd", &delta_qkv_bwd);
+  m.def("gated_norm_fwd", &gated_norm_fwd);
+  m.def("gated_norm_bwd", &gated_norm_bwd);
   m.def("set_autograd_hooks", &set_autograd_hooks);
   m.def("linears_node", &linears_node);
   m.def("swiglu_node", &swiglu_node);

@@ -863,6 +863,13 @@ extern "C" int llmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
   LLMT_CHECK_LAUNCH();
 }
 
+// out[c] = sum over P rows of partial [P][D], into fp32 or bf16.
+extern "C" int llmt_colsum(const float* partial, float* out_f32, void* out_bf16, int P, int D, cudaStream_t st) {
+  if (D <= 0) return 0;
+  colsum_kernel<<<(D + 31) / 32, 1024, 0, st>>>(partial, out_f32, (__nv_bfloat16*)out_bf16, P, D, 0);
+  LLMT_CHECK_LAUNCH();
+}
+
 extern "C" int llmt_qk_norm_rope_fwd(const void* x, int64_t tok_stride, const void* w, const float* cosb, const float* sinb,
                                      void* y, int64_t y_tok_stride, float* rstd, int T, int H, int HD, float eps,
                                      cudaStream_t st) {

@@ -82,6 +82,20 @@ int llmt_combine_rows(const void* y, const int64_t* dest, const float* w, void* 
 int llmt_combine_bwd(const void* dout, const void* y, const int64_t* dest, const float* w, void* dy, float* dw, int64_t ncopies,
                      int k, int D, const int* seg, const int64_t* counts, int E, cudaStream_t st);
 
+// ---- around the gated delta rule (gdn.cu) ----
+int llmt_colsum(const float* partial, float* out_f32, void* out_bf16, int P, int D, cudaStream_t st);
+int llmt_conv_silu_blocks(int T);
+int llmt_conv_silu_fwd(const void* x, int64_t ldx, const void* w, const int64_t* pos, void* y, int T, int C, int K, cudaStream_t st);
+int llmt_conv_silu_bwd(const void* dy, int64_t lddy, const void* x, int64_t ldx, const void* w, const int64_t* pos, void* dx, float* dw_part,
+                       void* dw, int T, int C, int K, cudaStream_t st);
+int llmt_delta_qkv_fwd(const void* mixed, float* q, float* k, float* v, int T, int Hk, int Hv, int D, float qscale, float eps, cudaStream_t st);
+int llmt_delta_qkv_bwd(const float* dq, const float* dk, const float* dv, const void* mixed, void* dmixed, int T, int Hk, int Hv, int D,
+                       float qscale, float eps, cudaStream_t st);
+int llmt_gated_norm_fwd(const void* x, const void* gate, const void* w, void* y, int64_t R, int D, float eps, cudaStream_t st);
+int llmt_gated_norm_bwd_blocks(int64_t R, int D);
+int llmt_gated_norm_bwd(const void* dy, const void* x, const void* gate, const void* w, void* dx, void* dgate, float* dw_part, void* dw,
+                        int64_t R, int D, float eps, cudaStream_t st);
+
 // ---- peer-memory communication (comm.cu) ----
 int llmt_side_job(int kind, int nsrc, const void* const* src, void* dst, long long n, int accumulate,
                   const uint32_t* wait_flags, int n_wait, uint32_t wait_value, int ctas, int* status, cudaStream_t st);

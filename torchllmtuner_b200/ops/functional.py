@@ -8,6 +8,7 @@ import math
 import os
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import reference as ref
 from ..errors import UnsupportedCombinationError
@@ -299,6 +300,76 @@ def swiglu(gate, up, row_limit=None):
     if _use_cuda(gate) and gate.dtype == torch.bfloat16:
         return _ext().swiglu_node(gate, up, row_limit)
     return ref.swiglu(gate, up)
+
+
+# ----------------------------------------------------------------------------------------------- around the delta rule
+class _ConvSiLU(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w, positions):
+        x2 = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
+        w2 = _c(w)
+        ctx.save_for_backward(x2, w2, positions)
+        return _ext().conv_silu_fwd(x2, w2, positions)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dy):
+        x, w, positions = ctx.saved_tensors
+        dy = dy if dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0 else dy.contiguous()
+        return (*_ext().conv_silu_bwd(dy, x, w, positions), None)
+
+
+def causal_conv_silu(x, w, positions):
+    """silu of the depthwise causal convolution of x [T, C] with w [C, K] (last tap on the current row); a tap that would reach
+    before the row's document (index `positions` [T]) contributes nothing. None where the kernel has no form for the inputs."""
+    if not (_use_cuda(x) and x.dtype == w.dtype == torch.bfloat16 and w.shape[1] in (2, 3, 4) and w.shape[0] % 8 == 0
+            and positions.dtype == torch.int64 and positions.is_cuda and positions.dim() == 1 and positions.is_contiguous()):
+        return None
+    return _ConvSiLU.apply(x, w, positions)
+
+
+class _DeltaQKV(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, mixed, key_heads, value_heads, qscale, eps):
+        mixed = _c(mixed)
+        ctx.save_for_backward(mixed)
+        ctx.cfg = (key_heads, value_heads, qscale, eps)
+        return tuple(_ext().delta_qkv_fwd(mixed, *ctx.cfg))
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dq, dk, dv):
+        return _ext().delta_qkv_bwd(_c(dq), _c(dk), _c(dv), ctx.saved_tensors[0], *ctx.cfg), None, None, None, None
+
+
+def delta_qkv(mixed, key_heads: int, value_heads: int, key_dim: int, value_dim: int, qscale: float, eps: float):
+    """Rows [q heads | k heads | v heads] -> fp32 (q, k, v), each [T, value_heads, width]: queries and keys L2-normalised per head
+    (queries scaled) and repeated for the value heads of their group. None where the kernel has no form for the inputs."""
+    if not (_use_cuda(mixed) and mixed.dtype == torch.bfloat16 and key_dim == value_dim and key_dim in (64, 128, 256)):
+        return None
+    return _DeltaQKV.apply(mixed, key_heads, value_heads, qscale, eps)
+
+
+class _GatedRMSNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, gate, w, eps):
+        x, gate = _c(x), _c(gate)
+        ctx.save_for_backward(x, gate, w)
+        ctx.eps = eps
+        return _ext().gated_norm_fwd(x, gate, w, eps)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dy):
+        x, gate, w = ctx.saved_tensors
+        return (*_ext().gated_norm_bwd(_c(dy), x, gate, w, ctx.eps), None)
+
+
+def gated_rms_norm(x, gate, w, eps: float):
+    """rms_norm(x) * w * silu(gate) over the last dimension; None where the kernel has no form for the inputs."""
+    if not (_use_cuda(x) and x.dtype == gate.dtype == w.dtype == torch.bfloat16 and x.shape == gate.shape and x.shape[-1] in (64, 128, 256)):
+        return None
+    return _GatedRMSNorm.apply(x, gate, w, eps)
 
 
 # ----------------------------------------------------------------------------------------------- attention
