@@ -810,6 +810,52 @@ std::vector<Tensor> gated_norm_bwd(const Tensor& dy, const Tensor& x, const Tens
   return {dx, dg, dw};
 }
 
+// q, k, v [T, H, D], beta, g [T, H] fp32 -> (o [T, H, D], what the backward needs: G, W1, W2, P, inv, S, U).
+static void check_delta(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta) {
+  for (const Tensor* t : {&q, &k, &v, &beta})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0,
+                "delta rule operands must be contiguous fp32 CUDA tensors on 16-byte boundaries");
+  TORCH_CHECK(q.dim() == 3 && k.sizes() == q.sizes() && v.sizes() == q.sizes() && beta.numel() == q.size(0) * q.size(1), "q, k, v [T, H, D], beta [T, H]");
+}
+std::vector<Tensor> delta_rule_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& g, bool keep) {
+  c10::cuda::CUDAGuard guard(q.device());
+  check_delta(q, k, v, beta);
+  TORCH_CHECK(g.is_cuda() && g.scalar_type() == at::kFloat && g.is_contiguous() && g.numel() == beta.numel());
+  const int64_t T = q.size(0), H = q.size(1), D = q.size(2), N = (T + 63) / 64;
+  auto o = q.options();
+  Tensor out = torch::empty(q.sizes(), o), G = torch::empty({N, H, 64}, o.dtype(at::kDouble)), W1 = torch::empty({N, H, 64, D}, o), W2 = torch::empty({N, H, 64, D}, o),
+         P = torch::empty({N, H, 64, 64}, o), inv, S, U;
+  if (keep) {
+    inv = torch::empty({N, H, 64, 64}, o);
+    S = torch::empty({N, H, D, D}, o);
+    U = torch::empty(q.sizes(), o);
+  }
+  check_rc(llmt_delta_rule_fwd(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), beta.data_ptr<float>(), g.data_ptr<float>(),
+                               G.data_ptr<double>(), W1.data_ptr<float>(), W2.data_ptr<float>(), P.data_ptr<float>(),
+                               keep ? inv.data_ptr<float>() : nullptr, keep ? S.data_ptr<float>() : nullptr, keep ? U.data_ptr<float>() : nullptr,
+                               out.data_ptr<float>(), (int)T, (int)H, (int)D, cur_stream()),
+           "llmt_delta_rule_fwd", 2);
+  if (!keep) return {out};
+  return {out, G, W1, W2, P, inv, S, U};
+}
+std::vector<Tensor> delta_rule_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& G,
+                                   const Tensor& W1, const Tensor& W2, const Tensor& P, const Tensor& inv, const Tensor& S, const Tensor& U) {
+  c10::cuda::CUDAGuard guard(q.device());
+  check_delta(q, k, v, beta);
+  TORCH_CHECK(dout.scalar_type() == at::kFloat && dout.is_contiguous() && dout.sizes() == q.sizes() && reinterpret_cast<uintptr_t>(dout.data_ptr()) % 16 == 0);
+  TORCH_CHECK(G.is_cuda() && G.scalar_type() == at::kDouble && G.is_contiguous());
+  for (const Tensor* t : {&W1, &W2, &P, &inv, &S, &U}) TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous());
+  Tensor dS = torch::empty_like(S), dU = torch::empty_like(U), dq = torch::empty_like(q), dk = torch::empty_like(q), dv = torch::empty_like(q),
+         db = torch::empty_like(beta), dg = torch::empty_like(beta);
+  check_rc(llmt_delta_rule_bwd(dout.data_ptr<float>(), q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), beta.data_ptr<float>(),
+                               G.data_ptr<double>(), W1.data_ptr<float>(), W2.data_ptr<float>(), P.data_ptr<float>(), inv.data_ptr<float>(),
+                               S.data_ptr<float>(), U.data_ptr<float>(), dS.data_ptr<float>(), dU.data_ptr<float>(), dq.data_ptr<float>(),
+                               dk.data_ptr<float>(), dv.data_ptr<float>(), db.data_ptr<float>(), dg.data_ptr<float>(), (int)q.size(0),
+                               (int)q.size(1), (int)q.size(2), cur_stream()),
+           "llmt_delta_rule_bwd", 2);
+  return {dq, dk, dv, db, dg};
+}
+
 // ---- autograd nodes of the small hot ops
 // A launch of a small training step takes the device a few microseconds and took the host 20 to 27: the Python frames of
 // apply() and backward(), reshapes, allocations and attribute look-ups around one kernel call. These nodes do the same with the
@@ -1025,6 +1071,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("wait_value", &PySideJob::wait_value);
   m.def("gemm", &gemm, "bf16 tcgen05 GEMM", py::arg("a"), py::arg("b"), py::arg("out"), py::arg("a_mn"), py::arg("b_mn"),
         py::arg("accumulate") = false, py::arg("max_ctas") = 0, py::arg("side") = py::none());
+  m.def("delta_rule_fwd", &delta_rule_fwd);
+  m.def("delta_rule_bwd", &delta_rule_bwd);
   m.def("conv_silu_fwd", &conv_silu_fwd);
   m.def("conv_silu_bwd", &conv_silu_bwd);
   m.def("delta_qkv_fwd", &delta_qkv_fwd);

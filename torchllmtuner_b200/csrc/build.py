@@ -20,10 +20,12 @@ PKG = os.path.dirname(HERE)
 BUILD = os.path.join(HERE, "build")
 SO_PATH = os.path.join(PKG, "_C.so")
 STAMP = os.path.join(PKG, "_C.stamp")
-CU_SOURCES = ("gemm.cu", "elementwise.cu", "attention.cu", "attention_fwd_pair.cu", "attention_bwd.cu", "attention_bwd_wide.cu", "moe.cu", "gdn.cu", "comm.cu", "ep_comm.cu", "vocab_parallel.cu", "noalloc.cu")
+CU_SOURCES = ("gemm.cu", "elementwise.cu", "attention.cu", "attention_fwd_pair.cu", "attention_bwd.cu", "attention_bwd_wide.cu", "moe.cu", "gdn.cu", "delta_rule.cu", "comm.cu", "ep_comm.cu", "vocab_parallel.cu", "noalloc.cu")
 HEADERS = ("common.cuh", "comm.cuh", "attn_common.cuh", "kernels.h", "noalloc.h")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--use_fast_math", "-Xptxas", "-v"]
+
+PRECISE_SOURCES = ("delta_rule.cu",)    # fp32 results that stand in for fp32 tensor expressions: no fast-math exponentials and divides
 
 
 def _nvcc() -> str:
@@ -89,7 +91,8 @@ def build(verbose: bool = False, force: bool = False) -> str:
         path = os.path.join(HERE, src)
         obj = os.path.join(BUILD, f"{os.path.splitext(src)[0]}.{_hash([path] + hdr)}{'.dbg' if debug else ''}{tag}.o")
         if not os.path.exists(obj):
-            _run([_nvcc(), *NVCC_FLAGS, *extra, "-I", HERE, "-c", path, "-o", obj], log)
+            flags = [f for f in NVCC_FLAGS if not (src in PRECISE_SOURCES and f == "--use_fast_math")]
+            _run([_nvcc(), *flags, *extra, "-I", HERE, "-c", path, "-o", obj], log)
         return obj
 
     with ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1))) as ex:

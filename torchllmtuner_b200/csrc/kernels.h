@@ -96,6 +96,13 @@ int llmt_gated_norm_bwd_blocks(int64_t R, int D);
 int llmt_gated_norm_bwd(const void* dy, const void* x, const void* gate, const void* w, void* dx, void* dgate, float* dw_part, void* dw,
                         int64_t R, int D, float eps, cudaStream_t st);
 
+// ---- gated delta rule, fp32 (delta_rule.cu) ----
+int llmt_delta_rule_fwd(const float* q, const float* k, const float* v, const float* beta, const float* g, double* G, float* W1, float* W2,
+                        float* P, float* inv, float* S, float* U, float* o, int T, int H, int D, cudaStream_t st);
+int llmt_delta_rule_bwd(const float* dout, const float* q, const float* k, const float* v, const float* beta, const double* G, const float* W1,
+                        const float* W2, const float* P, const float* inv, const float* S, const float* U, float* dS, float* dU, float* dq,
+                        float* dk, float* dv, float* dbeta, float* dg, int T, int H, int D, cudaStream_t st);
+
 // ---- peer-memory communication (comm.cu) ----
 int llmt_side_job(int kind, int nsrc, const void* const* src, void* dst, long long n, int accumulate,
                   const uint32_t* wait_flags, int n_wait, uint32_t wait_value, int ctas, int* status, cudaStream_t st);

@@ -75,7 +75,12 @@ def chunked_delta_rule(q, k, v, beta, log_decay, chunk: int = 64, initial_state=
     with K~_t = exp(G_t) k_t; then O = Q~ S0 + tril(QK) U and S_end = exp(G_C) S0 + (exp(G_C - G) K)^T U.
     Everything that does not depend on S0 is computed for all chunks at once (batched matrix products and one batched
     triangular solve); only the [dk, dv] state update runs chunk after chunk. Decay ratios are only ever formed as
-    exp(G_t - G_i) with i <= t, so nothing overflows however strong the decay."""
+    exp(G_t - G_i) with i <= t, so nothing overflows however strong the decay. On the device the common form (one decay per
+    head, no state in or out) runs as four kernels in the same arithmetic; the chunk length is theirs then."""
+    if initial_state is None and not return_state:
+        o = ops.delta_rule(q, k, v, beta, log_decay)
+        if o is not None:
+            return o
     T, H, dk = q.shape
     dv, C = v.shape[-1], chunk
     pad = (-T) % C

@@ -350,6 +350,40 @@ def delta_qkv(mixed, key_heads: int, value_heads: int, key_dim: int, value_dim: 
     return _DeltaQKV.apply(mixed, key_heads, value_heads, qscale, eps)
 
 
+class _DeltaRule(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, q, k, v, beta, log_decay):
+        q, k, v, beta, g = (_aligned(t) for t in (q, k, v, beta, log_decay.squeeze(-1)))
+        keep = any(ctx.needs_input_grad)
+        o, *saved = _ext().delta_rule_fwd(q, k, v, beta, g, keep)
+        if keep:
+            ctx.save_for_backward(q, k, v, beta, *saved)
+        return o
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, do):
+        dq, dk, dv, db, dg = _ext().delta_rule_bwd(_aligned(do), *ctx.saved_tensors)
+        return dq, dk, dv, db, dg.unsqueeze(-1)
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = _c(t)
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def delta_rule(q, k, v, beta, log_decay):
+    """The gated delta rule with one decay per head and zero initial state: q, k, v [T, H, d], beta [T, H], log_decay [T, H, 1]
+    (<= 0), fp32 -> [T, H, d] (the recurrence of `models.families.delta_rule_scan`). None where the kernels have no form for the
+    inputs."""
+    ts = (q, k, v, beta, log_decay)
+    if not (_use_cuda(q) and all(t.dtype == torch.float32 and t.is_cuda for t in ts) and q.shape == k.shape == v.shape and q.dim() == 3
+            and q.shape[-1] in (64, 128) and q.shape[0] > 0 and tuple(beta.shape) == tuple(q.shape[:2])
+            and tuple(log_decay.shape) == (*q.shape[:2], 1)):
+        return None
+    return _DeltaRule.apply(*ts)
+
+
 class _GatedRMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, gate, w, eps):
