@@ -96,3 +96,27 @@ def test_delta_rule_kernels_match_the_scan_in_64_bits(T, H, d, decay):
         assert torch.equal(p, q)                       # no atomics
     with torch.no_grad():
         assert torch.equal(ops.delta_rule(*x), o)      # the form without a backward
+
+
+def test_second_derivatives_and_transforms_of_the_delta_rule():
+    """What the node cannot do stays with the tensor expressions: a gradient of the gradient, forward-mode derivatives and vmap give
+    what 64 bits give (a second derivative sums a few thousand fp32 terms of its own size: 1e-4 of the largest)."""
+    from torchllmtuner_b200.models.families import chunked_delta_rule
+    g = torch.Generator(device="cuda").manual_seed(5)
+    T, H, d = 70, 2, 64
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x = [F.normalize(r(T, H, d), dim=-1), F.normalize(r(T, H, d), dim=-1), r(T, H, d), torch.rand(T, H, generator=g, device="cuda"),
+         -F.softplus(r(T, H, 1))]
+
+    def second(a):
+        a = [t.clone().requires_grad_() for t in a]
+        first = torch.autograd.grad(chunked_delta_rule(*a).square().sum(), a, create_graph=True)
+        return (*first, *torch.autograd.grad(sum(t.square().sum() for t in first), a))
+
+    tangent = r(T, H, d)
+    forward = lambda a, t: torch.func.jvp(lambda v: chunked_delta_rule(a[0], a[1], v, a[3], a[4]), (a[2],), (t,))  # noqa: E731
+    mapped = lambda a: torch.func.vmap(lambda v: chunked_delta_rule(a[0], a[1], v, a[3], a[4]))(torch.stack((a[2], 2 * a[2])))  # noqa: E731
+    y = [t.double() for t in x]
+    got, want = (*second(x), *forward(x, tangent), mapped(x)), (*second(y), *forward(y, tangent.double()), mapped(y))
+    for p, q in zip(got, want):
+        assert (p.double() - q).abs().max() <= 1e-4 * q.abs().max()

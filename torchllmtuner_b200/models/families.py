@@ -78,9 +78,13 @@ def chunked_delta_rule(q, k, v, beta, log_decay, chunk: int = 64, initial_state=
     exp(G_t - G_i) with i <= t, so nothing overflows however strong the decay. On the device the common form (one decay per
     head, no state in or out) runs as four kernels in the same arithmetic; the chunk length is theirs then."""
     if initial_state is None and not return_state:
-        o = ops.delta_rule(q, k, v, beta, log_decay)
+        o = ops.delta_rule(q, k, v, beta, log_decay, lambda *a: _chunk_expressions(*a, chunk))
         if o is not None:
             return o
+    return _chunk_expressions(q, k, v, beta, log_decay, chunk, initial_state, return_state)
+
+
+def _chunk_expressions(q, k, v, beta, log_decay, chunk: int, initial_state=None, return_state: bool = False):
     T, H, dk = q.shape
     dv, C = v.shape[-1], chunk
     pad = (-T) % C

@@ -162,12 +162,16 @@ class CausalConvolution(nn.Module):
         """x [T, C]; positions [T]: index of each row inside its document. `halo` [B, K-1, C]: under sequence
         parallelism the rows that precede each of the B local spans on the rank before (the position mask still decides
         whether a tap may use them)."""
-        K = self.kernel
+        w = self.weight[:, 0, :]
         if halo is None:
-            y = ops.causal_conv_silu(x, self.weight[:, 0, :], positions)
+            y = ops.causal_conv_silu(x, w, positions, self._expressions)
             if y is not None:
                 return y
-        w = self.weight[:, 0, :].to(x.dtype)                       # [C, K]
+        return self._expressions(x, w, positions, halo)
+
+    def _expressions(self, x, w, positions, halo=None):
+        K = self.kernel
+        w = w.to(x.dtype)                                          # [C, K]
         T, C = x.shape
         out = x * w[:, K - 1]
         if halo is not None:

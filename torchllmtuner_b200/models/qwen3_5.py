@@ -95,11 +95,13 @@ class GatedRMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(dim, dtype=dtype, device=device))
 
     def forward(self, x, gate):
-        y = ops.gated_rms_norm(x, gate, self.weight, self.eps)
-        if y is not None:
-            return y
+        y = ops.gated_rms_norm(x, gate, self.weight, self.eps, self._expressions)
+        return y if y is not None else self._expressions(x, gate, self.weight, self.eps)
+
+    @staticmethod
+    def _expressions(x, gate, w, eps):
         xf = x.float()
-        y = (xf * torch.rsqrt(xf.square().mean(-1, keepdim=True) + self.eps)).to(x.dtype) * self.weight
+        y = (xf * torch.rsqrt(xf.square().mean(-1, keepdim=True) + eps)).to(x.dtype) * w
         return (y * F.silu(gate.float())).to(x.dtype)
 
 
@@ -159,18 +161,8 @@ class GatedDeltaNet(nn.Module):
         mixed = self.in_proj_qkv(x)
         halo = cp.prev_rows(mixed, self.conv1d.kernel - 1) if cp is not None else None
         mixed = self.conv1d(mixed, ctx.positions, halo)
-        qkv = ops.delta_qkv(mixed, self.Hk, self.Hv, self.dk, self.dv, self.dk ** -0.5, 1e-6)
-        if qkv is not None:
-            q, k, v = qkv
-        else:
-            q = mixed[:, :self.key_dim].view(T, self.Hk, self.dk).float()
-            k = mixed[:, self.key_dim:2 * self.key_dim].view(T, self.Hk, self.dk).float()
-            v = mixed[:, 2 * self.key_dim:].view(T, self.Hv, self.dv).float()
-            q = q * torch.rsqrt(q.square().sum(-1, keepdim=True) + 1e-6) * self.dk ** -0.5
-            k = k * torch.rsqrt(k.square().sum(-1, keepdim=True) + 1e-6)
-            rep = self.Hv // self.Hk
-            if rep > 1:
-                q, k = q.repeat_interleave(rep, dim=1), k.repeat_interleave(rep, dim=1)
+        qkv = ops.delta_qkv(mixed, self.Hk, self.Hv, self.dk, self.dv, self.dk ** -0.5, 1e-6, self._qkv_expressions)
+        q, k, v = qkv if qkv is not None else self._qkv_expressions(mixed)
         beta = torch.sigmoid(self.in_proj_b(x).float())
         log_decay = (-self.A_log.float().exp() * F.softplus(self.in_proj_a(x).float() + self.dt_bias.float())).unsqueeze(-1)   # [T, Hv, 1]
         if cp is not None:
@@ -182,6 +174,18 @@ class GatedDeltaNet(nn.Module):
         z = self.in_proj_z(x).view(T * self.Hv, self.dv)
         o = self.norm(o.to(x.dtype).reshape(T * self.Hv, self.dv), z)
         return self.out_proj(o.view(T, self.value_dim))
+
+    def _qkv_expressions(self, mixed):
+        T = mixed.shape[0]
+        q = mixed[:, :self.key_dim].view(T, self.Hk, self.dk).float()
+        k = mixed[:, self.key_dim:2 * self.key_dim].view(T, self.Hk, self.dk).float()
+        v = mixed[:, 2 * self.key_dim:].view(T, self.Hv, self.dv).float()
+        q = q * torch.rsqrt(q.square().sum(-1, keepdim=True) + 1e-6) * self.dk ** -0.5
+        k = k * torch.rsqrt(k.square().sum(-1, keepdim=True) + 1e-6)
+        rep = self.Hv // self.Hk
+        if rep > 1:
+            q, k = q.repeat_interleave(rep, dim=1), k.repeat_interleave(rep, dim=1)
+        return q, k, v
 
 
 class GatedFullAttention(nn.Module):

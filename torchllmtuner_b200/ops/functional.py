@@ -8,7 +8,7 @@ import math
 import os
 
 import torch
-from torch.autograd.function import once_differentiable
+from torch.autograd import forward_ad
 
 from . import reference as ref
 from ..errors import UnsupportedCombinationError
@@ -303,68 +303,96 @@ def swiglu(gate, up, row_limit=None):
 
 
 # ----------------------------------------------------------------------------------------------- around the delta rule
+# Autograd nodes over kernels that took the place of tensor expressions. What the expressions could do and a node cannot stays with
+# them: `statement`, the same computation as tensor expressions, serves second derivatives, and `_has_rules` sends calls under
+# functorch transforms, forward-mode tangents, tracing and dispatch modes, and calls on tensor subclasses, back to the caller.
+def _has_rules(*ts: torch.Tensor) -> bool:
+    return (torch._C._functorch.peek_interpreter_stack() is None and forward_ad._current_level < 0 and not torch.compiler.is_compiling()
+            and not torch.jit.is_tracing() and torch._C._len_torch_dispatch_stack() == 0
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in ts))
+
+
+def _through_statement(ctx, inputs, grads):
+    """Input gradients of `ctx.statement(*inputs)` that carry a graph of their own."""
+    if ctx.statement is None:
+        raise RuntimeError("second derivatives need the computation as tensor expressions (the `statement` argument)")
+    with torch.enable_grad():
+        inputs = [t.view_as(t) for t in inputs]            # distinct graph nodes, also where two inputs are one tensor
+        outs = ctx.statement(*inputs)
+    need = ctx.needs_input_grad[:len(inputs)]
+    got = iter(torch.autograd.grad(outs, [t for t, n in zip(inputs, need) if n], grads, create_graph=True, allow_unused=True))
+    return tuple(next(got) if n else None for n in need) + (None,) * (len(ctx.needs_input_grad) - len(inputs))
+
+
+def _rows16(t: torch.Tensor) -> torch.Tensor:
+    return t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.contiguous()
+
+
 class _ConvSiLU(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, w, positions):
-        x2 = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
-        w2 = _c(w)
-        ctx.save_for_backward(x2, w2, positions)
-        return _ext().conv_silu_fwd(x2, w2, positions)
+    def forward(ctx, x, w, positions, statement):
+        ctx.save_for_backward(x, w, positions)
+        ctx.statement = statement and (lambda x, w: statement(x, w, positions))
+        return _ext().conv_silu_fwd(_rows16(x), _c(w), positions)
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dy):
         x, w, positions = ctx.saved_tensors
-        dy = dy if dy.stride(1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0 else dy.contiguous()
-        return (*_ext().conv_silu_bwd(dy, x, w, positions), None)
+        if torch.is_grad_enabled():
+            return _through_statement(ctx, (x, w), dy)
+        return (*_ext().conv_silu_bwd(_rows16(dy), _rows16(x), _c(w), positions), None, None)
 
 
-def causal_conv_silu(x, w, positions):
+def causal_conv_silu(x, w, positions, statement=None):
     """silu of the depthwise causal convolution of x [T, C] with w [C, K] (last tap on the current row); a tap that would reach
-    before the row's document (index `positions` [T]) contributes nothing. None where the kernel has no form for the inputs."""
+    before the row's document (index `positions` [T]) contributes nothing. None where the kernel has no form for the call."""
     if not (_use_cuda(x) and x.dtype == w.dtype == torch.bfloat16 and w.shape[1] in (2, 3, 4) and w.shape[0] % 8 == 0
-            and positions.dtype == torch.int64 and positions.is_cuda and positions.dim() == 1 and positions.is_contiguous()):
+            and positions.dtype == torch.int64 and positions.is_cuda and positions.dim() == 1 and positions.is_contiguous()
+            and _has_rules(x, w, positions)):
         return None
-    return _ConvSiLU.apply(x, w, positions)
+    return _ConvSiLU.apply(x, w, positions, statement)
 
 
 class _DeltaQKV(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, mixed, key_heads, value_heads, qscale, eps):
-        mixed = _c(mixed)
+    def forward(ctx, mixed, key_heads, value_heads, qscale, eps, statement):
         ctx.save_for_backward(mixed)
-        ctx.cfg = (key_heads, value_heads, qscale, eps)
-        return tuple(_ext().delta_qkv_fwd(mixed, *ctx.cfg))
+        ctx.cfg, ctx.statement = (key_heads, value_heads, qscale, eps), statement
+        return tuple(_ext().delta_qkv_fwd(_c(mixed), *ctx.cfg))
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dq, dk, dv):
-        return _ext().delta_qkv_bwd(_c(dq), _c(dk), _c(dv), ctx.saved_tensors[0], *ctx.cfg), None, None, None, None
+        mixed, = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return _through_statement(ctx, (mixed,), (dq, dk, dv))
+        return _ext().delta_qkv_bwd(_c(dq), _c(dk), _c(dv), _c(mixed), *ctx.cfg), None, None, None, None, None
 
 
-def delta_qkv(mixed, key_heads: int, value_heads: int, key_dim: int, value_dim: int, qscale: float, eps: float):
+def delta_qkv(mixed, key_heads: int, value_heads: int, key_dim: int, value_dim: int, qscale: float, eps: float, statement=None):
     """Rows [q heads | k heads | v heads] -> fp32 (q, k, v), each [T, value_heads, width]: queries and keys L2-normalised per head
-    (queries scaled) and repeated for the value heads of their group. None where the kernel has no form for the inputs."""
-    if not (_use_cuda(mixed) and mixed.dtype == torch.bfloat16 and key_dim == value_dim and key_dim in (64, 128, 256)):
+    (queries scaled) and repeated for the value heads of their group. None where the kernel has no form for the call."""
+    if not (_use_cuda(mixed) and mixed.dtype == torch.bfloat16 and key_dim == value_dim and key_dim in (64, 128, 256) and _has_rules(mixed)):
         return None
-    return _DeltaQKV.apply(mixed, key_heads, value_heads, qscale, eps)
+    return _DeltaQKV.apply(mixed, key_heads, value_heads, qscale, eps, statement)
 
 
 class _DeltaRule(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, beta, log_decay):
-        q, k, v, beta, g = (_aligned(t) for t in (q, k, v, beta, log_decay.squeeze(-1)))
+    def forward(ctx, q, k, v, beta, log_decay, statement):
         keep = any(ctx.needs_input_grad)
-        o, *saved = _ext().delta_rule_fwd(q, k, v, beta, g, keep)
+        o, *saved = _ext().delta_rule_fwd(*(_aligned(t) for t in (q, k, v, beta, log_decay.squeeze(-1))), keep)
         if keep:
-            ctx.save_for_backward(q, k, v, beta, *saved)
+            ctx.save_for_backward(q, k, v, beta, log_decay, *saved)
+            ctx.statement = statement
         return o
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, do):
-        dq, dk, dv, db, dg = _ext().delta_rule_bwd(_aligned(do), *ctx.saved_tensors)
-        return dq, dk, dv, db, dg.unsqueeze(-1)
+        q, k, v, beta, log_decay, *saved = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return _through_statement(ctx, (q, k, v, beta, log_decay), do)
+        dq, dk, dv, db, dg = _ext().delta_rule_bwd(*(_aligned(t) for t in (do, q, k, v, beta, *saved)))
+        return dq, dk, dv, db, dg.unsqueeze(-1), None
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -372,38 +400,39 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
-def delta_rule(q, k, v, beta, log_decay):
+def delta_rule(q, k, v, beta, log_decay, statement=None):
     """The gated delta rule with one decay per head and zero initial state: q, k, v [T, H, d], beta [T, H], log_decay [T, H, 1]
     (<= 0), fp32 -> [T, H, d] (the recurrence of `models.families.delta_rule_scan`). None where the kernels have no form for the
-    inputs."""
+    call."""
     ts = (q, k, v, beta, log_decay)
     if not (_use_cuda(q) and all(t.dtype == torch.float32 and t.is_cuda for t in ts) and q.shape == k.shape == v.shape and q.dim() == 3
             and q.shape[-1] in (64, 128) and q.shape[0] > 0 and tuple(beta.shape) == tuple(q.shape[:2])
-            and tuple(log_decay.shape) == (*q.shape[:2], 1)):
+            and tuple(log_decay.shape) == (*q.shape[:2], 1) and _has_rules(*ts)):
         return None
-    return _DeltaRule.apply(*ts)
+    return _DeltaRule.apply(*ts, statement)
 
 
 class _GatedRMSNorm(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, gate, w, eps):
-        x, gate = _c(x), _c(gate)
+    def forward(ctx, x, gate, w, eps, statement):
         ctx.save_for_backward(x, gate, w)
-        ctx.eps = eps
-        return _ext().gated_norm_fwd(x, gate, w, eps)
+        ctx.eps, ctx.statement = eps, statement and (lambda x, gate, w: statement(x, gate, w, eps))
+        return _ext().gated_norm_fwd(_c(x), _c(gate), w, eps)
 
     @staticmethod
-    @once_differentiable
     def backward(ctx, dy):
         x, gate, w = ctx.saved_tensors
-        return (*_ext().gated_norm_bwd(_c(dy), x, gate, w, ctx.eps), None)
+        if torch.is_grad_enabled():
+            return _through_statement(ctx, (x, gate, w), dy)
+        return (*_ext().gated_norm_bwd(_c(dy), _c(x), _c(gate), w, ctx.eps), None, None)
 
 
-def gated_rms_norm(x, gate, w, eps: float):
-    """rms_norm(x) * w * silu(gate) over the last dimension; None where the kernel has no form for the inputs."""
-    if not (_use_cuda(x) and x.dtype == gate.dtype == w.dtype == torch.bfloat16 and x.shape == gate.shape and x.shape[-1] in (64, 128, 256)):
+def gated_rms_norm(x, gate, w, eps: float, statement=None):
+    """rms_norm(x) * w * silu(gate) over the last dimension; None where the kernel has no form for the call."""
+    if not (_use_cuda(x) and x.dtype == gate.dtype == w.dtype == torch.bfloat16 and x.shape == gate.shape and x.shape[-1] in (64, 128, 256)
+            and _has_rules(x, gate, w)):
         return None
-    return _GatedRMSNorm.apply(x, gate, w, eps)
+    return _GatedRMSNorm.apply(x, gate, w, eps, statement)
 
 
 # ----------------------------------------------------------------------------------------------- attention
