@@ -87,7 +87,8 @@ def main() -> None:
         out.update(seq=S, heads=[H, Hk], head_dim=d, ms=ms, tflops_causal=tf, frac_of_peak=tf / ptf)
     elif a.op == "delta_rule":
         # gated delta rule, forward + backward in fp32: --heads, --head-dim, --chunk; --channel-decay for a decay per key channel;
-        # --loop forces the chunk-after-chunk form the scan form replaces
+        # --loop forces the chunk-after-chunk form the scan form replaces (head sizes 64 and 128 with one decay per head run as
+        # kernels whatever the form and the chunk)
         import torch.nn.functional as F
         from ..models import families as fam
         S, H, d = a.seq, a.heads, a.head_dim
@@ -101,7 +102,8 @@ def main() -> None:
         def step():
             torch.autograd.grad(fam.chunked_delta_rule(*x, a.chunk).square().sum(), x)
         ms = timeit(step, a.iters, a.warmup)
-        out.update(seq=S, heads=H, head_dim=d, chunk=a.chunk, channel_decay=a.channel_decay, form="loop" if a.loop else "scan", ms_fwd_bwd=ms)
+        form = "kernels" if not a.channel_decay and d in (64, 128) else "loop" if a.loop else "scan"
+        out.update(seq=S, heads=H, head_dim=d, chunk=a.chunk, channel_decay=a.channel_decay, form=form, ms_fwd_bwd=ms)
     elif a.op == "rmsnorm":
         x = torch.randn(a.rows, a.cols, device=dev).bfloat16(); w = torch.ones(a.cols, device=dev).bfloat16()
         ms = timeit(lambda: ops.rms_norm(x, w, 1e-6), a.iters, a.warmup)
