@@ -826,7 +826,7 @@ std::vector<Tensor> delta_rule_fwd(const Tensor& q, const Tensor& k, const Tenso
   Tensor out = torch::empty(q.sizes(), o), G = torch::empty({N, H, 64}, o.dtype(at::kDouble)), W1 = torch::empty({N, H, 64, D}, o), W2 = torch::empty({N, H, 64, D}, o),
          P = torch::empty({N, H, 64, 64}, o), inv, S, U;
   if (keep) {
-    inv = torch::empty({N, H, 64, 64}, o);
+    inv = torch::empty({2, N, H, 64, 64}, o);
     S = torch::empty({N, H, D, D}, o);
     U = torch::empty(q.sizes(), o);
   }
