@@ -1,0 +1,48 @@
+"""What the autograd nodes hand to the kernels: 16-byte loads need rows on 16-byte boundaries, whatever views a caller passes. The kernel
+library is replaced by a recorder, so a wrong address shows here and never reaches a device."""
+import pytest
+import torch
+
+from torchllmtuner_b200.ops import functional as F
+
+
+class Recorder:
+    """Stands in for the extension: answers with zeros and keeps the operands of every call."""
+
+    def __init__(self, **answers):
+        self.answers, self.seen = answers, {}
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.seen[name] = [a for a in args if isinstance(a, torch.Tensor)]
+            return self.answers[name](*args)
+        return call
+
+    def misaligned(self):
+        return [(n, i) for n, ts in self.seen.items() for i, t in enumerate(ts) if t.dtype != torch.int64 and t.data_ptr() % 16]
+
+
+def shifted(*shape, dtype=torch.bfloat16, by=1):
+    """A contiguous tensor whose first element is `by` elements past a 16-byte boundary."""
+    n = 1
+    for s in shape:
+        n *= s
+    flat = torch.randn(n + 16).to(dtype)
+    start = next(i for i in range(16) if flat[i:].data_ptr() % 16 == by * flat.element_size())
+    t = flat[start:start + n].view(shape)
+    assert t.is_contiguous() and t.data_ptr() % 16
+    return t
+
+
+def zeros(*like):
+    return lambda *args: tuple(torch.zeros_like(args[i]) for i in like)
+
+
+def test_gated_norm_operands(monkeypatch):
+    ext = Recorder(gated_norm_fwd=lambda x, gate, w, eps: torch.zeros_like(x), gated_norm_bwd=zeros(1, 2, 3))
+    monkeypatch.setattr(F, "_ext", lambda: ext)
+    x, gate, w = shifted(5, 64).requires_grad_(), shifted(5, 64).requires_grad_(), torch.randn(64, 2).bfloat16()[:, 0].requires_grad_()
+    F._GatedRMSNorm.apply(x, gate, w, 1e-6, None).backward(shifted(5, 64))
+    assert set(ext.seen) == {"gated_norm_fwd", "gated_norm_bwd"} and not ext.misaligned()
+    assert all(t.is_contiguous() for ts in ext.seen.values() for t in ts)
+    assert torch.equal(ext.seen["gated_norm_fwd"][0], x)

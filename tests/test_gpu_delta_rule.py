@@ -69,6 +69,34 @@ def test_gated_rms_norm(R, D):
         _close(p, q.float(), n, n == "dw")
 
 
+def _shifted(t):
+    """The same values in contiguous memory one element past a 16-byte boundary."""
+    flat = torch.empty(t.numel() + 16, dtype=t.dtype, device=t.device)
+    v = flat[1:t.numel() + 1].view(t.shape)
+    v.copy_(t)
+    assert v.is_contiguous() and v.data_ptr() % 16
+    return v
+
+
+def _same_from_shifted(op, ins, dys):
+    """`op` on operands and upstream gradients off the 16-byte boundary gives the bits that it gives for aligned ones."""
+    def run(ins, dys):
+        ins = [t.detach().requires_grad_() for t in ins]
+        ys = op(*ins)
+        ys = ys if isinstance(ys, tuple) else (ys,)
+        return (*ys, *torch.autograd.grad(ys, ins, dys))
+    want, got = run(ins, dys), run([_shifted(t) for t in ins], [_shifted(t) for t in dys])
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_gated_rms_norm_off_the_16_byte_boundary():
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(1)
+    x, gate, dy = (torch.randn(37, 128, device="cuda").bfloat16() for _ in range(3))
+    w = torch.randn(128, device="cuda").bfloat16()
+    _same_from_shifted(lambda *a: ops.gated_rms_norm(*a, 1e-6), (x, gate, w), (dy,))
+
+
 @pytest.mark.parametrize("T,H,d", [(1, 1, 64), (63, 2, 128), (64, 3, 64), (65, 2, 128), (300, 2, 64), (700, 1, 128)])
 @pytest.mark.parametrize("decay", [0.05, 3.0])
 def test_delta_rule_kernels_match_the_scan_in_64_bits(T, H, d, decay):

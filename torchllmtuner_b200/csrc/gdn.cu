@@ -372,6 +372,7 @@ extern "C" int llmt_delta_qkv_bwd(const float* dq, const float* dk, const float*
 }
 extern "C" int llmt_gated_norm_fwd(const void* x, const void* gate, const void* w, void* y, int64_t R, int D, float eps, cudaStream_t st) {
   if (R <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) return -10;
   const int64_t per = 8 * 256 / D;
   if (by_width(D, [&](auto g) {
         gated_norm_fwd_kernel<decltype(g)::value><<<(unsigned)((R + per - 1) / per), 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)gate,
@@ -388,6 +389,9 @@ extern "C" int llmt_gated_norm_bwd_blocks(int64_t R, int D) {
 extern "C" int llmt_gated_norm_bwd(const void* dy, const void* x, const void* gate, const void* w, void* dx, void* dgate, float* dw_part, void* dw,
                                    int64_t R, int D, float eps, cudaStream_t st) {
   if (R <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(w) |
+       reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dgate)) & 15)
+    return -10;
   const int blocks = llmt_gated_norm_bwd_blocks(R, D);
   if (by_width(D, [&](auto g) {
         gated_norm_bwd_kernel<decltype(g)::value><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gate,

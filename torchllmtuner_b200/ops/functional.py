@@ -324,6 +324,11 @@ def _through_statement(ctx, inputs, grads):
     return tuple(next(got) if n else None for n in need) + (None,) * (len(ctx.needs_input_grad) - len(inputs))
 
 
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """`t` in contiguous memory on a 16-byte boundary. Not `.contiguous()`: that returns a contiguous view off the boundary unchanged."""
+    return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 def _rows16(t: torch.Tensor) -> torch.Tensor:
     return t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.contiguous()
 
@@ -395,11 +400,6 @@ class _DeltaRule(torch.autograd.Function):
         return dq, dk, dv, db, dg.unsqueeze(-1), None
 
 
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    t = _c(t)
-    return t if t.data_ptr() % 16 == 0 else t.clone()
-
-
 def delta_rule(q, k, v, beta, log_decay, statement=None):
     """The gated delta rule with one decay per head and zero initial state: q, k, v [T, H, d], beta [T, H], log_decay [T, H, 1]
     (<= 0), fp32 -> [T, H, d] (the recurrence of `models.families.delta_rule_scan`). None where the kernels have no form for the
@@ -417,20 +417,20 @@ class _GatedRMSNorm(torch.autograd.Function):
     def forward(ctx, x, gate, w, eps, statement):
         ctx.save_for_backward(x, gate, w)
         ctx.eps, ctx.statement = eps, statement and (lambda x, gate, w: statement(x, gate, w, eps))
-        return _ext().gated_norm_fwd(_c(x), _c(gate), w, eps)
+        return _ext().gated_norm_fwd(_aligned(x), _aligned(gate), _aligned(w), eps)
 
     @staticmethod
     def backward(ctx, dy):
         x, gate, w = ctx.saved_tensors
         if torch.is_grad_enabled():
             return _through_statement(ctx, (x, gate, w), dy)
-        return (*_ext().gated_norm_bwd(_c(dy), _c(x), _c(gate), w, ctx.eps), None, None)
+        return (*_ext().gated_norm_bwd(*(_aligned(t) for t in (dy, x, gate, w)), ctx.eps), None, None)
 
 
 def gated_rms_norm(x, gate, w, eps: float, statement=None):
     """rms_norm(x) * w * silu(gate) over the last dimension; None where the kernel has no form for the call."""
     if not (_use_cuda(x) and x.dtype == gate.dtype == w.dtype == torch.bfloat16 and x.shape == gate.shape and x.shape[-1] in (64, 128, 256)
-            and _has_rules(x, gate, w)):
+            and w.shape == x.shape[-1:] and _has_rules(x, gate, w)):
         return None
     return _GatedRMSNorm.apply(x, gate, w, eps, statement)
 
