@@ -46,3 +46,12 @@ def test_gated_norm_operands(monkeypatch):
     assert set(ext.seen) == {"gated_norm_fwd", "gated_norm_bwd"} and not ext.misaligned()
     assert all(t.is_contiguous() for ts in ext.seen.values() for t in ts)
     assert torch.equal(ext.seen["gated_norm_fwd"][0], x)
+
+
+def test_convolution_operands(monkeypatch):
+    ext = Recorder(conv_silu_fwd=lambda x, w, pos: torch.zeros_like(x), conv_silu_bwd=lambda dy, x, w, pos: (torch.zeros_like(x), torch.zeros_like(w)))
+    monkeypatch.setattr(F, "_ext", lambda: ext)
+    for x in (shifted(5, 16), torch.randn(1, 17).bfloat16()[:, :16], torch.randn(16, 5).bfloat16().t()):      # off the boundary, odd row stride, column-major
+        F._ConvSiLU.apply(x.requires_grad_(), torch.randn(16, 4).bfloat16().requires_grad_(), torch.arange(x.shape[0]), None).backward(shifted(*x.shape))
+        assert set(ext.seen) == {"conv_silu_fwd", "conv_silu_bwd"} and not ext.misaligned()
+        assert all(t.stride(1) == 1 and t.stride(0) % 8 == 0 for t in (ext.seen["conv_silu_fwd"][0], *ext.seen["conv_silu_bwd"][:2]))

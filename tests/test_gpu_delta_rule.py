@@ -97,6 +97,14 @@ def test_gated_rms_norm_off_the_16_byte_boundary():
     _same_from_shifted(lambda *a: ops.gated_rms_norm(*a, 1e-6), (x, gate, w), (dy,))
 
 
+def test_causal_conv_silu_off_the_16_byte_boundary():
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(2)
+    x, dy = (torch.randn(37, 264, device="cuda").bfloat16() for _ in range(2))
+    w, pos = torch.randn(264, 4, device="cuda").bfloat16(), torch.arange(37, device="cuda")
+    _same_from_shifted(lambda x, w: ops.causal_conv_silu(x, w, pos), (x, w), (dy,))
+
+
 @pytest.mark.parametrize("T,H,d", [(1, 1, 64), (63, 2, 128), (64, 3, 64), (65, 2, 128), (300, 2, 64), (700, 1, 128)])
 @pytest.mark.parametrize("decay", [0.05, 3.0])
 def test_delta_rule_kernels_match_the_scan_in_64_bits(T, H, d, decay):

@@ -330,7 +330,7 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
 
 
 def _rows16(t: torch.Tensor) -> torch.Tensor:
-    return t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.contiguous()
+    return t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
 
 
 class _ConvSiLU(torch.autograd.Function):
