@@ -55,3 +55,12 @@ def test_convolution_operands(monkeypatch):
         F._ConvSiLU.apply(x.requires_grad_(), torch.randn(16, 4).bfloat16().requires_grad_(), torch.arange(x.shape[0]), None).backward(shifted(*x.shape))
         assert set(ext.seen) == {"conv_silu_fwd", "conv_silu_bwd"} and not ext.misaligned()
         assert all(t.stride(1) == 1 and t.stride(0) % 8 == 0 for t in (ext.seen["conv_silu_fwd"][0], *ext.seen["conv_silu_bwd"][:2]))
+
+
+def test_delta_qkv_operands(monkeypatch):
+    ext = Recorder(delta_qkv_fwd=lambda m, Hk, Hv, scale, eps: [torch.zeros(m.shape[0], Hv, 64) for _ in range(3)],
+                   delta_qkv_bwd=lambda dq, dk, dv, m, *cfg: torch.zeros_like(m))
+    monkeypatch.setattr(F, "_ext", lambda: ext)
+    ys = F._DeltaQKV.apply(shifted(5, 4 * 64).requires_grad_(), 1, 2, 0.125, 1e-6, None)
+    torch.autograd.backward(ys, [shifted(5, 2, 64, dtype=torch.float32) for _ in ys])
+    assert set(ext.seen) == {"delta_qkv_fwd", "delta_qkv_bwd"} and not ext.misaligned()

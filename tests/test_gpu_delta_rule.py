@@ -105,6 +105,13 @@ def test_causal_conv_silu_off_the_16_byte_boundary():
     _same_from_shifted(lambda x, w: ops.causal_conv_silu(x, w, pos), (x, w), (dy,))
 
 
+def test_delta_qkv_off_the_16_byte_boundary():
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(3)
+    x, dys = torch.randn(37, 8 * 64, device="cuda").bfloat16(), [torch.randn(37, 4, 64, device="cuda") for _ in range(3)]
+    _same_from_shifted(lambda x: ops.delta_qkv(x, 2, 4, 64, 64, 0.125, 1e-6), (x,), dys)
+
+
 @pytest.mark.parametrize("T,H,d", [(1, 1, 64), (63, 2, 128), (64, 3, 64), (65, 2, 128), (300, 2, 64), (700, 1, 128)])
 @pytest.mark.parametrize("decay", [0.05, 3.0])
 def test_delta_rule_kernels_match_the_scan_in_64_bits(T, H, d, decay):

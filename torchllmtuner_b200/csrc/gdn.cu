@@ -361,7 +361,9 @@ extern "C" int llmt_delta_qkv_fwd(const void* mixed, float* q, float* k, float* 
 extern "C" int llmt_delta_qkv_bwd(const float* dq, const float* dk, const float* dv, const void* mixed, void* dmixed, int T, int Hk, int Hv, int D,
                                   float qscale, float eps, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (Hk < 1 || Hv % Hk || ((reinterpret_cast<uintptr_t>(mixed) | reinterpret_cast<uintptr_t>(dmixed)) & 15)) return -10;
+  if (Hk < 1 || Hv % Hk || ((reinterpret_cast<uintptr_t>(mixed) | reinterpret_cast<uintptr_t>(dmixed) | reinterpret_cast<uintptr_t>(dq) |
+                             reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15))
+    return -10;
   const int64_t items = (int64_t)T * (2 * Hk + Hv), per = 8 * 256 / D;
   if (by_width(D, [&](auto g) {
         delta_qkv_bwd_kernel<decltype(g)::value><<<(unsigned)((items + per - 1) / per), 256, 0, st>>>(dq, dk, dv, (const __nv_bfloat16*)mixed,

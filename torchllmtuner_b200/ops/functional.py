@@ -363,14 +363,14 @@ class _DeltaQKV(torch.autograd.Function):
     def forward(ctx, mixed, key_heads, value_heads, qscale, eps, statement):
         ctx.save_for_backward(mixed)
         ctx.cfg, ctx.statement = (key_heads, value_heads, qscale, eps), statement
-        return tuple(_ext().delta_qkv_fwd(_c(mixed), *ctx.cfg))
+        return tuple(_ext().delta_qkv_fwd(_aligned(mixed), *ctx.cfg))
 
     @staticmethod
     def backward(ctx, dq, dk, dv):
         mixed, = ctx.saved_tensors
         if torch.is_grad_enabled():
             return _through_statement(ctx, (mixed,), (dq, dk, dv))
-        return _ext().delta_qkv_bwd(_c(dq), _c(dk), _c(dv), _c(mixed), *ctx.cfg), None, None, None, None, None
+        return _ext().delta_qkv_bwd(*(_aligned(t) for t in (dq, dk, dv, mixed)), *ctx.cfg), None, None, None, None, None
 
 
 def delta_qkv(mixed, key_heads: int, value_heads: int, key_dim: int, value_dim: int, qscale: float, eps: float, statement=None):
