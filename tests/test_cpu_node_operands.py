@@ -64,3 +64,17 @@ def test_delta_qkv_operands(monkeypatch):
     ys = F._DeltaQKV.apply(shifted(5, 4 * 64).requires_grad_(), 1, 2, 0.125, 1e-6, None)
     torch.autograd.backward(ys, [shifted(5, 2, 64, dtype=torch.float32) for _ in ys])
     assert set(ext.seen) == {"delta_qkv_fwd", "delta_qkv_bwd"} and not ext.misaligned()
+
+
+def test_wide_attention_upstream_gradient(monkeypatch):
+    from torchllmtuner_b200.ops import AttnMeta
+    ext = Recorder(attn_bwd_wide=lambda q, k, v, *rest: (torch.zeros_like(q), torch.zeros_like(k), torch.zeros_like(v)))
+    monkeypatch.setattr(F, "_ext", lambda: ext)
+    meta = AttnMeta.build([0, 5], device="cpu")
+    meta.q_tiles, meta.k_tile_passes = torch.zeros(1, 8, dtype=torch.int32), [torch.zeros(1, 8, dtype=torch.int32)]
+    q, k, v = (torch.randn(5, 1, 256).bfloat16().requires_grad_() for _ in range(3))
+    kept = (torch.randn(5, 1, 256).bfloat16(), torch.randn(1, 5))
+    for do in (shifted(5, 1, 256), torch.randn(5, 1, 260).bfloat16()[..., :256]):        # off the boundary, odd row stride
+        o, _ = F._Attention.apply(q, k, v, meta, 0.0625, kept)
+        o.backward(do)
+        assert not ext.misaligned() and ext.seen["attn_bwd_wide"][4].stride() == (256, 256, 1) and torch.equal(ext.seen["attn_bwd_wide"][4], do)

@@ -272,3 +272,16 @@ def test_attention_backward_head_256_against_the_row_form(pieces, Tq, Tk, Hq, Hk
     assert got[0][~covered].abs().sum() == 0
     for a, b in zip(got, torch.autograd.grad(o, [q, k, v], go)):
         assert torch.equal(a, b)
+
+
+def test_attention_backward_head_256_takes_upstream_gradients_off_the_16_byte_boundary():
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(4)
+    q, k, v = (torch.randn(140, h, 256, device="cuda").bfloat16().requires_grad_() for h in (4, 2, 2))
+    o = ops.attention(q, k, v, ops.AttnMeta.build([0, 140], device="cuda"))
+    go = torch.randn_like(o)
+    flat = torch.empty(go.numel() + 16, dtype=go.dtype, device="cuda")
+    off = flat[1:go.numel() + 1].view(go.shape).copy_(go)
+    assert off.is_contiguous() and off.data_ptr() % 16
+    for a, b in zip(torch.autograd.grad(o, [q, k, v], go, retain_graph=True), torch.autograd.grad(o, [q, k, v], off)):
+        assert torch.equal(a, b)

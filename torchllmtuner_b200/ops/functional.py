@@ -459,8 +459,8 @@ class _Attention(torch.autograd.Function):
             # every key belongs to one piece, and no piece starts with queries that see no key (a query tile's table cannot
             # hold a diagonal before column 0)
             if len(m.k_tile_passes) == 1 and all(p[4] >= 0 for p in m.pieces):
-                if do.stride(0) % 8 or do.data_ptr() % 16:
-                    do = do.contiguous()
+                if do.stride(0) % 8 or do.stride(1) != 256 or do.data_ptr() % 16:
+                    do = do.clone(memory_format=torch.contiguous_format)
                 whole = m.covers_all_keys and m.total_k == k.shape[0] and sum(p[1] for p in m.pieces) == q.shape[0]
                 dq, dk, dv = ext.attn_bwd_wide(q, k, v, o, do, lse, m.q_tiles, m.k_tile_passes[0], ctx.scale, m.causal, not whole)
                 return dq, dk, dv, None, None, None
