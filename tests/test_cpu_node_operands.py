@@ -7,19 +7,17 @@ from torchllmtuner_b200.ops import functional as F
 
 
 class Recorder:
-    """Stands in for the extension: answers with zeros and keeps the operands of every call."""
+    """Stands in for the extension: answers with zeros, keeps the operands of the last call of each name and the places of all that were off a boundary."""
 
     def __init__(self, **answers):
-        self.answers, self.seen = answers, {}
+        self.answers, self.seen, self.off = answers, {}, []
 
     def __getattr__(self, name):
         def call(*args):
             self.seen[name] = [a for a in args if isinstance(a, torch.Tensor)]
+            self.off += [(name, i) for i, t in enumerate(self.seen[name]) if t.dtype != torch.int64 and t.data_ptr() % 16]
             return self.answers[name](*args)
         return call
-
-    def misaligned(self):
-        return [(n, i) for n, ts in self.seen.items() for i, t in enumerate(ts) if t.dtype != torch.int64 and t.data_ptr() % 16]
 
 
 def shifted(*shape, dtype=torch.bfloat16, by=1):
@@ -43,7 +41,7 @@ def test_gated_norm_operands(monkeypatch):
     monkeypatch.setattr(F, "_ext", lambda: ext)
     x, gate, w = shifted(5, 64).requires_grad_(), shifted(5, 64).requires_grad_(), torch.randn(64, 2).bfloat16()[:, 0].requires_grad_()
     F._GatedRMSNorm.apply(x, gate, w, 1e-6, None).backward(shifted(5, 64))
-    assert set(ext.seen) == {"gated_norm_fwd", "gated_norm_bwd"} and not ext.misaligned()
+    assert set(ext.seen) == {"gated_norm_fwd", "gated_norm_bwd"} and not ext.off
     assert all(t.is_contiguous() for ts in ext.seen.values() for t in ts)
     assert torch.equal(ext.seen["gated_norm_fwd"][0], x)
 
@@ -53,7 +51,7 @@ def test_convolution_operands(monkeypatch):
     monkeypatch.setattr(F, "_ext", lambda: ext)
     for x in (shifted(5, 16), torch.randn(1, 17).bfloat16()[:, :16], torch.randn(16, 5).bfloat16().t()):      # off the boundary, odd row stride, column-major
         F._ConvSiLU.apply(x.requires_grad_(), torch.randn(16, 4).bfloat16().requires_grad_(), torch.arange(x.shape[0]), None).backward(shifted(*x.shape))
-        assert set(ext.seen) == {"conv_silu_fwd", "conv_silu_bwd"} and not ext.misaligned()
+        assert set(ext.seen) == {"conv_silu_fwd", "conv_silu_bwd"} and not ext.off
         assert all(t.stride(1) == 1 and t.stride(0) % 8 == 0 for t in (ext.seen["conv_silu_fwd"][0], *ext.seen["conv_silu_bwd"][:2]))
 
 
@@ -63,7 +61,7 @@ def test_delta_qkv_operands(monkeypatch):
     monkeypatch.setattr(F, "_ext", lambda: ext)
     ys = F._DeltaQKV.apply(shifted(5, 4 * 64).requires_grad_(), 1, 2, 0.125, 1e-6, None)
     torch.autograd.backward(ys, [shifted(5, 2, 64, dtype=torch.float32) for _ in ys])
-    assert set(ext.seen) == {"delta_qkv_fwd", "delta_qkv_bwd"} and not ext.misaligned()
+    assert set(ext.seen) == {"delta_qkv_fwd", "delta_qkv_bwd"} and not ext.off
 
 
 def test_wide_attention_upstream_gradient(monkeypatch):
@@ -77,4 +75,14 @@ def test_wide_attention_upstream_gradient(monkeypatch):
     for do in (shifted(5, 1, 256), torch.randn(5, 1, 260).bfloat16()[..., :256]):        # off the boundary, odd row stride
         o, _ = F._Attention.apply(q, k, v, meta, 0.0625, kept)
         o.backward(do)
-        assert not ext.misaligned() and ext.seen["attn_bwd_wide"][4].stride() == (256, 256, 1) and torch.equal(ext.seen["attn_bwd_wide"][4], do)
+        assert not ext.off and ext.seen["attn_bwd_wide"][4].stride() == (256, 256, 1) and torch.equal(ext.seen["attn_bwd_wide"][4], do)
+
+
+def test_grouped_projection_upstream_gradients(monkeypatch):
+    from torchllmtuner_b200.models.moe import experts
+    ext = Recorder(grouped_gemm=lambda *a: None, grouped_wgrad=lambda *a: None)
+    monkeypatch.setattr(experts, "_ext", lambda: ext)
+    x, ws = torch.randn(128, 16).bfloat16().requires_grad_(), [torch.randn(1, 24, 16).bfloat16().requires_grad_() for _ in range(2)]
+    ys = experts._GroupedLinear.apply(x, torch.tensor([0, 128], dtype=torch.int32), *ws)
+    torch.autograd.backward(ys, [shifted(128, 24), torch.randn(128, 49).bfloat16()[:, :24]])
+    assert set(ext.seen) == {"grouped_gemm", "grouped_wgrad"} and not ext.off

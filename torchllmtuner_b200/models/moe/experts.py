@@ -46,7 +46,7 @@ def _rows_view(t: torch.Tensor) -> torch.Tensor:
     The gradients of gate and up are the two halves of one buffer: copying them cost as much as a grouped product."""
     if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1] and t.data_ptr() % 16 == 0:
         return t
-    return t.contiguous()
+    return t.clone(memory_format=torch.contiguous_format)
 
 
 class _GroupedLinear(torch.autograd.Function):
