@@ -97,6 +97,24 @@ def test_gated_rms_norm_off_the_16_byte_boundary():
     _same_from_shifted(lambda *a: ops.gated_rms_norm(*a, 1e-6), (x, gate, w), (dy,))
 
 
+@pytest.mark.parametrize("T,C", [(65536, 16), (65537, 16), (1048640, 8)])
+def test_causal_conv_silu_on_long_rows(T, C):
+    """Rows on both sides of the length from which a block walks more than 16 of them, and more than 65535 blocks of 16 would cover:
+    against the convolution of the library in fp32, cut into documents of 1000 rows."""
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(5)
+    x, dy = (torch.randn(T, C, device="cuda").bfloat16() for _ in range(2))
+    w, pos = torch.randn(C, 4, device="cuda").bfloat16(), torch.arange(T, device="cuda") % 1000
+    a = [t.clone().requires_grad_() for t in (x, w)]
+    y = ops.causal_conv_silu(*a, pos)
+    g = torch.autograd.grad(y, a, dy)
+    b = [t.float().requires_grad_() for t in (x, w)]
+    z = sum(torch.where((pos >= j)[:, None], F.pad(b[0], (0, 0, j, 0))[:T], 0.0) * b[1][:, 3 - j] for j in range(4))
+    want = F.silu(z)
+    gw = torch.autograd.grad(want, b, dy.float())
+    _close(y, want, "y"); _close(g[0], gw[0], "dx"); _close(g[1], gw[1], "dw", True)
+
+
 def test_causal_conv_silu_off_the_16_byte_boundary():
     from torchllmtuner_b200 import ops
     torch.manual_seed(2)

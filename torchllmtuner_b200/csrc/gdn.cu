@@ -24,12 +24,14 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf
 
 // ------------------------------------------------------------------------------------------ causal convolution + SiLU
 // z[t, c] = sum_j x[t - j, c] * w[c, K - 1 - j] over the taps j <= pos[t] (the index of row t in its document); y = silu(z).
-// Bound by memory: a thread owns 8 channels and walks kConvTok rows with the last K rows in registers, so every row is read
-// once (plus K - 1 rows per block). 2048 x 8192, K = 4: 25 us forward, 86 us backward (67 and 100 MB; as tensor expressions about 1.1 ms together).
-constexpr int kConvTok = 16;
+// Bound by memory: a thread owns 8 channels and walks the `tok` rows of its block with the last K rows in registers, so every row is
+// read once (plus K - 1 rows per block). 2048 x 8192, K = 4: 25 us forward, 86 us backward (67 and 100 MB; as tensor expressions about 1.1 ms together).
+// 16 rows per block; rows of more than 16 x kConvBlocks tokens get longer blocks, which bounds the grid (gridDim.y ends at 65535) and the
+// partial sums of the weight gradient.
+constexpr int kConvTok = 16, kConvBlocks = 4096;
 template <int K>
 __global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w,
-                                                            const int64_t* __restrict__ pos, __nv_bfloat16* __restrict__ y, int T, int C) {
+                                                            const int64_t* __restrict__ pos, __nv_bfloat16* __restrict__ y, int T, int C, int tok) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
   if (c >= C) return;
   float wt[8][K];
@@ -37,7 +39,7 @@ __global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const __nv_bfloat16*
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < K; ++j) wt[i][j] = __bfloat162float(w[(int64_t)(c + i) * K + K - 1 - j]);   // wt[.][j]: tap j rows back
-  const int t0 = blockIdx.y * kConvTok, t1 = min(T, t0 + kConvTok);
+  const int t0 = blockIdx.y * tok, t1 = min(T, t0 + tok);
   uint4 win[K];                                        // win[j]: row t - j
 #pragma unroll
   for (int j = 1; j < K; ++j) win[j - 1] = t0 - j >= 0 ? *reinterpret_cast<const uint4*>(x + (int64_t)(t0 - j) * ldx + c) : make_uint4(0, 0, 0, 0);
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const __nv_bfloat16*
 template <int K>
 __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, int64_t lddy, const __nv_bfloat16* __restrict__ x,
                                                             int64_t ldx, const __nv_bfloat16* __restrict__ w, const int64_t* __restrict__ pos,
-                                                            __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int T, int C) {
+                                                            __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int T, int C, int tok) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
   if (c >= C) return;
   float wt[8][K], dw[8][K];
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const __nv_bfloat16*
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < K; ++j) { wt[i][j] = __bfloat162float(w[(int64_t)(c + i) * K + K - 1 - j]); dw[i][j] = 0.f; }
-  const int t0 = blockIdx.y * kConvTok, t1 = min(T, t0 + kConvTok), last = min(T, t1 + K - 1) - 1;
+  const int t0 = blockIdx.y * tok, t1 = min(T, t0 + tok), last = min(T, t1 + K - 1) - 1;
   const uint4 zero = make_uint4(0, 0, 0, 0);
   uint4 win[K];                                        // win[j]: row t - j
 #pragma unroll
@@ -305,7 +307,14 @@ int sm_count();   // gemm.cu
 using namespace llmt;
 #define LLMT_CHECK_LAUNCH() return (cudaGetLastError() == cudaSuccess) ? 0 : -3
 
-extern "C" int llmt_conv_silu_blocks(int T) { return (T + kConvTok - 1) / kConvTok; }
+static inline int conv_tok(int T) {            // rows per block, a multiple of kConvTok
+  const int64_t per = ((int64_t)T + kConvBlocks - 1) / kConvBlocks;
+  return per <= kConvTok ? kConvTok : (int)((per + kConvTok - 1) / kConvTok * kConvTok);
+}
+extern "C" int llmt_conv_silu_blocks(int T) {
+  const int tok = conv_tok(T);
+  return (int)(((int64_t)T + tok - 1) / tok);
+}
 template <typename F>
 static inline int by_taps(int K, F&& f) {
   switch (K) {
@@ -320,7 +329,7 @@ extern "C" int llmt_conv_silu_fwd(const void* x, int64_t ldx, const void* w, con
   if (C % 8 || ldx % 8 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15)) return -10;
   const dim3 grid((C / 8 + 127) / 128, llmt_conv_silu_blocks(T));
   if (by_taps(K, [&](auto k) {
-        conv_silu_fwd_kernel<decltype(k)::value><<<grid, 128, 0, st>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, pos, (__nv_bfloat16*)y, T, C);
+        conv_silu_fwd_kernel<decltype(k)::value><<<grid, 128, 0, st>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, pos, (__nv_bfloat16*)y, T, C, conv_tok(T));
       }))
     return -10;
   LLMT_CHECK_LAUNCH();
@@ -333,7 +342,7 @@ extern "C" int llmt_conv_silu_bwd(const void* dy, int64_t lddy, const void* x, i
   const dim3 grid((C / 8 + 127) / 128, llmt_conv_silu_blocks(T));
   if (by_taps(K, [&](auto k) {
         conv_silu_bwd_kernel<decltype(k)::value><<<grid, 128, 0, st>>>((const __nv_bfloat16*)dy, lddy, (const __nv_bfloat16*)x, ldx,
-                                                                       (const __nv_bfloat16*)w, pos, (__nv_bfloat16*)dx, dw_part, T, C);
+                                                                       (const __nv_bfloat16*)w, pos, (__nv_bfloat16*)dx, dw_part, T, C, conv_tok(T));
       }))
     return -10;
   llmt_colsum(dw_part, nullptr, dw, grid.y, C * K, st);
