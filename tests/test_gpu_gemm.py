@@ -236,3 +236,40 @@ def test_native_linear_node_matches_the_python_node(need, owned):
     if not owned:
         for a, b in zip(grads(hooked), grads(want)):
             assert torch.equal(a, b)
+
+
+def test_launches_of_two_threads_are_all_counted():
+    """A backward runs in autograd's thread without the GIL while another Python thread launches: the count of both together is the sum
+    of what each adds alone."""
+    import threading
+    from torchllmtuner_b200 import ops
+    from torchllmtuner_b200.ops.cuda_ext import load
+    ext, w = load(), torch.ones(64, device="cuda", dtype=torch.bfloat16)
+
+    def graph():
+        y = torch.ones(1, 64, device="cuda", dtype=torch.bfloat16).requires_grad_()
+        for _ in range(2000):
+            y = ops.rms_norm(y, w, 1e-6)
+        return y
+
+    def counted(f):
+        before = ext.launch_count()
+        f()
+        return ext.launch_count() - before
+
+    def forwards(n):
+        with torch.no_grad():
+            for _ in range(n):
+                ops.rms_norm(x, w, 1e-6)
+    x = torch.ones(1, 64, device="cuda", dtype=torch.bfloat16)
+    ys = [graph() for _ in range(11)]
+    alone = counted(lambda: ys.pop().sum().backward())
+    assert alone >= 2000 and counted(lambda: forwards(10)) == 10
+    other = threading.Thread(target=forwards, args=(60000,))
+
+    def both():
+        other.start()
+        while ys:
+            ys.pop().sum().backward()
+        other.join()
+    assert counted(both) == 10 * alone + 60000

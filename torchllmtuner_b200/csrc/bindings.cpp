@@ -6,6 +6,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
+#include <atomic>
+
 #include "kernels.h"
 
 namespace {
@@ -18,11 +20,12 @@ inline void check_bf16(const Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");
   TORCH_CHECK(t.scalar_type() == at::kBFloat16, name, " must be bfloat16");
 }
-// Number of kernels of this library launched so far (the caller-side count; each binding adds what it enqueues).
-static int64_t g_launches = 0;
+// Number of kernels of this library launched so far (the caller-side count; each binding adds what it enqueues). Atomic: the C++
+// autograd nodes run their backward in autograd's thread without the GIL, beside launches of Python threads.
+static std::atomic<int64_t> g_launches{0};
 inline void check_rc(int rc, const char* what, int launches = 1) {
   TORCH_CHECK(rc == 0, what, " failed with code ", rc);
-  g_launches += launches;
+  g_launches.fetch_add(launches, std::memory_order_relaxed);
 }
 
 Tensor& status_word() {
@@ -84,7 +87,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& out, bool a_mn, bool b_mn, b
   TORCH_CHECK(rc == 0, "llmt_gemm_bf16 failed with code ", rc, " (M=", M, " N=", N, " K=", K, " lda=", A.ld, " ldb=", B.ld,
               " ldc=", out.stride(0), " a_mn=", a_mn, " b_mn=", b_mn, " a%16=", reinterpret_cast<uintptr_t>(A.ptr) % 16,
               " b%16=", reinterpret_cast<uintptr_t>(B.ptr) % 16, ")");
-  g_launches += 1;
+  g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
 // GEMM fused with a tensor-parallel row collective over peer memory (csrc/comm.cuh). mode 1: `a` is the local gathered
@@ -1054,7 +1057,7 @@ std::vector<int64_t> read_status(bool clear) {
   return r;
 }
 Tensor status_tensor() { return status_word(); }
-int64_t launch_count() { return g_launches; }
+int64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 }  // namespace
 
