@@ -594,12 +594,14 @@ __global__ void __launch_bounds__(NT, 2048 / NT) ce_fwd_bwd_kernel(__nv_bfloat16
     float f[8];
     unpack8(u, f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = __expf(f[j] - lse) * gsc;
-    if (at == lab_vec) {
+    for (int j = 0; j < 8; ++j) f[j] = __expf(f[j] - lse);
+    if (at == lab_vec) {                             // before the factor: p - 1 is exact where p is close to 1
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        if (j == lab_j) f[j] -= gsc;
+        if (j == lab_j) f[j] -= 1.f;
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] *= gsc;
     store8(p + (int64_t)at * 8, f);
   };
   i = threadIdx.x;
