@@ -273,3 +273,19 @@ def test_cross_entropy_gradient_of_a_confident_row():
     a, b = (t.gather(1, label[:, None]).double() for t in (one, third))
     assert (a < 0).sum() > len(d) // 2                      # confident, and not yet exactly 1
     assert ((b - a / 3).abs() <= 2.0 ** -7.9 * (a / 3).abs()).all()
+
+
+def test_qk_norm_rope_outputs_are_differentiated_apart():
+    """A backward through the queries frees their graph and leaves that of the keys."""
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(0)
+    q, k = (torch.randn(37, h, 64, device="cuda").bfloat16().requires_grad_() for h in (4, 2))
+    ws = [torch.randn(64, device="cuda").bfloat16().requires_grad_() for _ in range(2)]
+    ang = torch.rand(37, 32, device="cuda")
+    dys = [torch.randn_like(t) for t in (q, k)]
+    call = lambda: ops.qk_norm_rope(q, k, *ws, ang.cos(), ang.sin(), 1e-6)  # noqa: E731
+    want = torch.autograd.grad(call(), (q, k, *ws), dys)
+    yq, yk = call()
+    got = (torch.autograd.grad(yq, (q, ws[0]), dys[0]), torch.autograd.grad(yk, (k, ws[1]), dys[1]))
+    for a, b in zip((got[0][0], got[1][0], got[0][1], got[1][1]), want):
+        assert torch.equal(a, b)

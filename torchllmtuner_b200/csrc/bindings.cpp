@@ -1018,27 +1018,22 @@ struct NativeAddRMSNorm : public torch::autograd::Function<NativeAddRMSNorm> {
   }
 };
 
-// q and k of one attention layer: two independent halves in one node.
+// One node for q and one for k: either output can be differentiated (and its graph freed) without the other.
 struct NativeQKNormRope : public torch::autograd::Function<NativeQKNormRope> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const OptTensor& qw, const OptTensor& kw, const Tensor& cosb,
-                               const Tensor& sinb, double eps) {
-    auto a = qk_norm_rope_fwd(q, qw, cosb, sinb, eps), b = qk_norm_rope_fwd(k, kw, cosb, sinb, eps);
-    ctx->save_for_backward({q, k, qw.has_value() ? *qw : Tensor(), kw.has_value() ? *kw : Tensor(), cosb, sinb, a[1], b[1]});
-    ctx->set_materialize_grads(false);
-    return {a[0], b[0]};
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& w, const Tensor& cosb, const Tensor& sinb, double eps) {
+    auto r = qk_norm_rope_fwd(x, w, cosb, sinb, eps);
+    ctx->save_for_backward({x, w.has_value() ? *w : Tensor(), cosb, sinb, r[1]});
+    return r[0];
   }
   static variable_list backward(AutogradContext* ctx, variable_list d) {
-    variable_list s = ctx->get_saved_variables(), out(7);
-    for (int i = 0; i < 2; ++i) {
-      if (!d[i].defined()) continue;
-      Tensor dy = d[i];
-      if (dy.stride(2) != 1 || dy.stride(1) != dy.size(2)) dy = dy.contiguous();
-      const Tensor& w = s[2 + i];
-      const bool w16 = w.defined() && w.scalar_type() == at::kBFloat16;
-      auto r = qk_norm_rope_bwd(dy, s[i], w.defined() ? OptTensor(w) : OptTensor(), s[4], s[5], s[6 + i], w16);
-      out[i] = r[0];
-      if (w.defined()) out[2 + i] = w16 ? r[1] : r[1].to(w.scalar_type());
-    }
+    variable_list s = ctx->get_saved_variables(), out(5);
+    Tensor dy = d[0];
+    if (dy.stride(2) != 1 || dy.stride(1) != dy.size(2)) dy = dy.contiguous();
+    const Tensor& w = s[1];
+    const bool w16 = w.defined() && w.scalar_type() == at::kBFloat16;
+    auto r = qk_norm_rope_bwd(dy, s[0], w.defined() ? OptTensor(w) : OptTensor(), s[2], s[3], s[4], w16);
+    out[0] = r[0];
+    if (w.defined()) out[1] = w16 ? r[1] : r[1].to(w.scalar_type());
     return out;
   }
 };
@@ -1046,7 +1041,7 @@ Tensor swiglu_node(const Tensor& g, const Tensor& u, const OptTensor& row_limit)
 Tensor rmsnorm_node(const Tensor& x, const Tensor& w, double eps) { return NativeRMSNorm::apply(x, w, eps); }
 variable_list add_rmsnorm_node(const Tensor& x, const Tensor& r, const Tensor& w, double eps) { return NativeAddRMSNorm::apply(x, r, w, eps); }
 variable_list qk_norm_rope_node(const Tensor& q, const Tensor& k, const OptTensor& qw, const OptTensor& kw, const Tensor& cosb, const Tensor& sinb, double eps) {
-  return NativeQKNormRope::apply(q, k, qw, kw, cosb, sinb, eps);
+  return {NativeQKNormRope::apply(q, qw, cosb, sinb, eps), NativeQKNormRope::apply(k, kw, cosb, sinb, eps)};
 }
 
 // Reads the status word (synchronises the current stream) and clears it. Returns {code, site, block, extra}.
