@@ -245,7 +245,9 @@ def test_attention_pads_widths_without_a_kernel_variant(d, dv, causal):
     ([(0, 300, 0, 100, 0)], 300, 100, 4, 2, True),                               # queries past the last key
     ([(10, 90, 20, 80, 0), (150, 64, 130, 64, 0)], 230, 210, 8, 2, True),        # rows that belong to no piece
     ([(0, 257, 0, 191, 0)], 257, 191, 8, 1, False),
-    ([(0, 2600, 0, 2600, 0)], 2600, 2600, 16, 4, True)])
+    ([(0, 2600, 0, 2600, 0)], 2600, 2600, 16, 4, True),
+    # a group of four over 4, 2, 2 and 1 CTAs on 148 SMs: key tiles x key/value heads on both sides of 3/4 and 3/2 of the SMs
+    *(([(128 * i, 128, 128 * i, 128, 0) for i in range(n)], 128 * n, 128 * n, 8, 2, True) for n in (55, 56, 110, 111))])
 def test_attention_backward_head_256_against_the_row_form(pieces, Tq, Tk, Hq, Hkv, causal):
     """The backward kernels of head size 256 against the row-chunked form (library products with fp32 results, the path of
     pieces that share keys) over uneven pieces, offsets and row gaps; gradients repeat bit for bit and rows outside every piece

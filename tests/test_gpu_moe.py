@@ -11,7 +11,11 @@ def _close(a, b, tol=3e-2):
 
 
 @pytest.mark.parametrize("T,E,k,fn,renorm,use_bias", [(300, 128, 8, "softmax", True, True), (64, 8, 2, "sigmoid", True, False),
-                                                      (1000, 256, 6, "softmax", False, False), (17, 64, 4, "sigmoid", False, True)])
+                                                      (1000, 256, 6, "softmax", False, False), (17, 64, 4, "sigmoid", False, True),
+                                                      # both sides of 128 and 256 experts (4, 8 or 16 per lane), and the most
+                                                      (33, 127, 8, "softmax", True, True), (33, 129, 8, "sigmoid", True, True),
+                                                      (33, 255, 8, "softmax", True, False), (33, 257, 8, "softmax", True, True),
+                                                      (33, 512, 16, "sigmoid", True, True)])
 def test_router_topk_matches_reference(T, E, k, fn, renorm, use_bias):
     from torchllmtuner_b200.models.moe.routing import _RouterTopK
     from torchllmtuner_b200.ops import reference as ref
@@ -94,12 +98,46 @@ def test_plan_segments_kernel_matches_tensor_statement(n, E, skew):
         assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
 
 
+def _poison(*sizes):
+    """Free bf16 blocks of these element counts full of NaN: buffers of those sizes that a call allocates next consist of them. Requests
+    up to 1 MB come from another pool of the allocator than larger ones, so the sizes have to be the call's own."""
+    junk = [torch.full((n,), float("nan"), device="cuda", dtype=torch.bfloat16) for n in sizes for _ in range(12)]
+    del junk
+    for n in sizes:
+        assert torch.empty(n, device="cuda", dtype=torch.bfloat16).isnan().all()
+
+
+@pytest.mark.parametrize("T,E,k,D", [(3, 16, 2, 8), (130, 8, 4, 264), (257, 32, 8, 512), (65, 4, 1, 1032), (512, 4, 1, 64)])
+def test_padding_rows_are_written(T, E, k, D):
+    """The dispatch copy and the combine's backward on buffers full of NaN: every copy arrives, every padding row of a segment is zero
+    and rows past the last segment are not touched."""
+    from torchllmtuner_b200.models.moe.experts import padded_capacity, plan_segments
+    from torchllmtuner_b200.ops.cuda_ext import load
+    torch.manual_seed(D)
+    x, w = torch.randn(T, D, device="cuda").bfloat16(), torch.rand(T * k, device="cuda")
+    flat = torch.randint(0, E - 1, (T * k,), device="cuda")            # the last expert has no copies
+    dest, seg, counts = plan_segments(flat, E)
+    cap, end = padded_capacity(T * k, E), int(seg[-1])
+    padding = torch.ones(cap, dtype=torch.bool, device="cuda")
+    padding[dest] = False
+    padding[end:] = False
+    rows = torch.full((cap, D), float("nan"), device="cuda", dtype=torch.bfloat16)
+    load().permute_rows(x, dest, rows, k, seg, counts)
+    assert torch.equal(rows[dest], x.repeat_interleave(k, 0)) and (rows[padding] == 0).all() and rows[end:].isnan().all()
+    y = torch.randn(cap, D, device="cuda").bfloat16()
+    _poison(cap * D)
+    dy, dw = load().combine_bwd(x, y, dest, w, k, seg, counts)
+    want = (w[:, None] * x.repeat_interleave(k, 0).float()).bfloat16()
+    assert torch.equal(dy[dest], want) and (dy[padding] == 0).all() and dw.isfinite().all()
+
+
 @pytest.mark.parametrize("T,E,k,D,F_", [(3, 16, 2, 8, 64), (130, 8, 4, 264, 72), (257, 32, 8, 512, 136), (65, 4, 1, 1032, 64)])
 def test_routed_experts_write_their_padding_rows(T, E, k, D, F_):
     """Buffers are no longer cleared before use: the same call on poisoned memory gives finite results that match the CPU
     statement, for narrow rows, a top-k that is no multiple of the combine's eight loads, and empty experts."""
-    from torchllmtuner_b200.models.moe.experts import GroupedExperts, RoutedExperts
+    from torchllmtuner_b200.models.moe.experts import GroupedExperts, RoutedExperts, padded_capacity
     torch.manual_seed(T)
+    cap = padded_capacity(T * k, E)
     gpu = RoutedExperts(GroupedExperts(E, D, F_, dtype=torch.bfloat16, device="cuda"))
     cpu = RoutedExperts(GroupedExperts(E, D, F_, dtype=torch.float32))
     for p, q in zip(gpu.parameters(), cpu.parameters()):
@@ -111,8 +149,7 @@ def test_routed_experts_write_their_padding_rows(T, E, k, D, F_):
     xc, wc = x.detach().float().cpu().requires_grad_(), w.detach().cpu().requires_grad_()
     go = torch.randn(T, D, device="cuda").bfloat16()
     for _ in range(2):
-        junk = [torch.full((1 << 22,), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(4)]
-        del junk                                          # the allocator hands this memory to the buffers of the call
+        _poison(cap * D, cap * F_, 2 * cap * F_)
         yg = gpu(x, w, idx)
         gg = torch.autograd.grad(yg, [x, w, *gpu.parameters()], go)
     yc = cpu(xc, wc, idx.cpu())
