@@ -47,12 +47,6 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(rd));
   return d;
 }
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-
 // Warp index that the compiler knows to be the same in all lanes. The warp that issues the products walks its loop as a whole
 // and lets one lane issue: with uniform control flow, descriptors and barrier addresses are computed in uniform registers,
 // where tcgen05.mma takes them. In a single-thread branch every operand is moved there instruction by instruction, and beside
@@ -61,14 +55,6 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 // 461 -> 368; nothing else changed.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
-// 16-column slice `ks` of a K-major tile stored as 64-column halves of [128 rows][128 B].
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t base, int ks) {
-  return umma_desc_sw128(base + (ks >> 2) * 16384 + (ks & 3) * 32, 16, 1024);
-}
-// 16-row slice `ks` of the same physical tile read as an MN-major operand (rows = reduction index).
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t base, int ks) {
-  return umma_desc_sw128(base + ks * 2048, 16384, 1024);
-}
 // Store 32 consecutive bf16 (packed in 16 words) of row `row`, columns [col0, col0+32) into a swizzled K-major tile.
 __device__ __forceinline__ void store_row32_swz(uint8_t* tile, int row, int col0, const uint32_t* w) {
   uint8_t* base = tile + (col0 >> 6) * 16384 + row * 128;
@@ -86,16 +72,8 @@ struct AttnSmem {
   static constexpr int kP = 128 * 128 * 2;     // P / dS tile
 };
 
-// 16-column slice `ks` of a K-major tile with `rows` rows stored as 64-column halves of [rows][128 B].
-__device__ __forceinline__ uint64_t desc_kmajor_rows(uint32_t base, int ks, int rows) {
-  return umma_desc_sw128(base + (ks >> 2) * (rows * 128) + (ks & 3) * 32, 16, 1024);
-}
-// 16-row slice `ks` of a tile with `rows` rows read as an MN-major operand (64-column blocks `rows * 128` B apart).
-__device__ __forceinline__ uint64_t desc_mnmajor_rows(uint32_t base, int ks, int rows) {
-  return umma_desc_sw128(base + ks * 2048, rows * 128, 1024);
-}
-
-// offset (in 16-byte units) of 16-column slice `ks` of a K-major tile with `rows` rows / of 16-row slice `ks` read MN-major
+// offset (in 16-byte units) of 16-column slice `ks` of a K-major tile with `rows` rows, stored as 64-column halves of [rows][128 B] / of
+// 16-row slice `ks` of the same tile read as an MN-major operand (rows = reduction index)
 __host__ __device__ constexpr uint32_t koff(int ks, int rows) { return (uint32_t)(((ks >> 2) * (rows * 128) + (ks & 3) * 32) >> 4); }
 __host__ __device__ constexpr uint32_t mnoff(int ks) { return (uint32_t)((ks * 2048) >> 4); }
 
