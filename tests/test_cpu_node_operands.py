@@ -86,3 +86,51 @@ def test_grouped_projection_upstream_gradients(monkeypatch):
     ys = experts._GroupedLinear.apply(x, torch.tensor([0, 128], dtype=torch.int32), *ws)
     torch.autograd.backward(ys, [shifted(128, 24), torch.randn(128, 49).bfloat16()[:, :24]])
     assert set(ext.seen) == {"grouped_gemm", "grouped_wgrad"} and not ext.off
+
+
+def _batched(call, *ins):
+    """Gradients of three upstream gradients at once against one after another."""
+    ins = [t.detach().requires_grad_() for t in ins]
+    ys = call(*ins)
+    ys = ys if isinstance(ys, tuple) else (ys,)
+    dys = [torch.randn(3, *y.shape).to(y.dtype) for y in ys]
+    return torch.autograd.grad(ys, ins, dys, is_grads_batched=True, retain_graph=True), ins, [[d[i] for d in dys] for i in range(3)]
+
+
+def test_batched_upstream_gradients_take_the_expressions(monkeypatch):
+    """`is_grads_batched` hands a backward tensors without memory: no kernel is called with one, and the result is that of the expressions."""
+    from torchllmtuner_b200.models.families import _chunk_expressions
+    from torchllmtuner_b200.models.qwen3_5 import GatedRMSNorm
+    zero = lambda t: lambda *a: torch.zeros_like(t)  # noqa: E731
+    x, z, w = torch.randn(5, 64), torch.randn(5, 64), torch.randn(64)
+    q, k, v = (torch.randn(70, 2, 64) for _ in range(3))
+    beta, decay = torch.rand(70, 2), -torch.rand(70, 2, 1)
+    norm = lambda x, z, w: GatedRMSNorm._expressions(x, z, w, 1e-6)  # noqa: E731
+    conv = lambda x, w, pos: (x * w[:, 0]).sin()  # noqa: E731
+    rule = lambda *a: _chunk_expressions(*a, 64)  # noqa: E731
+    split = lambda m: (m[:, :64].sin(), m[:, 64:128].cos(), m[:, 128:])  # noqa: E731
+    nodes = {"norm": ((x, z, w), dict(gated_norm_fwd=zero(x)), lambda *a: F._GatedRMSNorm.apply(*a, 1e-6, lambda *b: GatedRMSNorm._expressions(*b)), norm),
+             "conv": ((x, torch.randn(64, 4)), dict(conv_silu_fwd=zero(x)), lambda x, w: F._ConvSiLU.apply(x, w, torch.arange(5), conv), lambda x, w: conv(x, w, None)),
+             "qkv": ((torch.randn(5, 192),), dict(delta_qkv_fwd=lambda *a: [torch.zeros(5, 64) for _ in range(3)]),
+                     lambda m: F._DeltaQKV.apply(m, 1, 1, 1.0, 1e-6, split), split),
+             "rule": ((q, k, v, beta, decay), dict(delta_rule_fwd=lambda *a: [torch.zeros_like(v)]), lambda *a: F._DeltaRule.apply(*a, rule), rule)}
+    for name, (ins, answers, call, statement) in nodes.items():
+        ext = Recorder(**answers)
+        monkeypatch.setattr(F, "_ext", lambda: ext)
+        got, leaves, dys = _batched(call, *ins)
+        for i in range(3):
+            for a, b in zip(got, torch.autograd.grad(statement(*leaves), leaves, dys[i])):
+                assert torch.allclose(a[i], b, rtol=1e-4, atol=1e-5), name
+        assert set(ext.seen) == set(answers)
+
+
+def test_batched_gradients_of_the_losses_take_the_expressions(monkeypatch):
+    ext = Recorder(ce_fwd_bwd=lambda work, *a: (torch.ones(work.shape[0]), None), gemm=lambda a, b, out, *rest: out.fill_(2.0))
+    monkeypatch.setattr(F, "_ext", lambda: ext)
+    target = torch.zeros(8, dtype=torch.int64)
+    for call, ins in ((lambda t: F._CrossEntropySum.apply(t, target), (torch.randn(8, 16).bfloat16(),)),
+                      (lambda h, w: F._LinearCrossEntropy.apply(h, w, target, 1), (torch.randn(8, 16).bfloat16(), torch.randn(24, 16).bfloat16()))):
+        got, leaves, dys = _batched(call, *ins)
+        for i in range(3):
+            for a, b, t in zip(got, torch.autograd.grad(call(*leaves), leaves, dys[i], create_graph=True), leaves):
+                assert a[i].shape == t.shape and torch.equal(a[i], b)

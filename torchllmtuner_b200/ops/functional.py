@@ -304,7 +304,7 @@ def swiglu(gate, up, row_limit=None):
 
 # ----------------------------------------------------------------------------------------------- around the delta rule
 # Autograd nodes over kernels that took the place of tensor expressions. What the expressions could do and a node cannot stays with
-# them: `statement`, the same computation as tensor expressions, serves second derivatives, and `_has_rules` sends calls under
+# them: `statement`, the same computation as tensor expressions, serves second derivatives and batched gradients, and `_has_rules` sends calls under
 # functorch transforms, forward-mode tangents, tracing and dispatch modes, and calls on tensor subclasses, back to the caller.
 def _has_rules(*ts: torch.Tensor) -> bool:
     return (torch._C._functorch.peek_interpreter_stack() is None and forward_ad._current_level < 0 and not torch.compiler.is_compiling()
@@ -312,15 +312,29 @@ def _has_rules(*ts: torch.Tensor) -> bool:
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in ts))
 
 
+def _beyond_kernels(*grads: torch.Tensor) -> bool:
+    """Does this backward need tensor expressions: to build a graph of its own, or because the upstream gradients are batches of a vmap
+    over them (`is_grads_batched`, a vectorised jacobian), which have no memory that a kernel could read?"""
+    if torch.is_grad_enabled():
+        return True
+    try:
+        for g in grads:
+            g.data_ptr()
+    except RuntimeError:
+        return True
+    return False
+
+
 def _through_statement(ctx, inputs, grads):
-    """Input gradients of `ctx.statement(*inputs)` that carry a graph of their own."""
+    """Input gradients of `ctx.statement(*inputs)`, with a graph of their own where one is being built."""
     if ctx.statement is None:
-        raise RuntimeError("second derivatives need the computation as tensor expressions (the `statement` argument)")
+        raise RuntimeError("second derivatives and batched gradients need the computation as tensor expressions (the `statement` argument)")
+    graph = torch.is_grad_enabled()
     with torch.enable_grad():
         inputs = [t.view_as(t) for t in inputs]            # distinct graph nodes, also where two inputs are one tensor
         outs = ctx.statement(*inputs)
     need = ctx.needs_input_grad[:len(inputs)]
-    got = iter(torch.autograd.grad(outs, [t for t, n in zip(inputs, need) if n], grads, create_graph=True, allow_unused=True))
+    got = iter(torch.autograd.grad(outs, [t for t, n in zip(inputs, need) if n], grads, create_graph=graph, allow_unused=True))
     return tuple(next(got) if n else None for n in need) + (None,) * (len(ctx.needs_input_grad) - len(inputs))
 
 
@@ -343,7 +357,7 @@ class _ConvSiLU(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, positions = ctx.saved_tensors
-        if torch.is_grad_enabled():
+        if _beyond_kernels(dy):
             return _through_statement(ctx, (x, w), dy)
         return (*_ext().conv_silu_bwd(_rows16(dy), _rows16(x), _c(w), positions), None, None)
 
@@ -368,7 +382,7 @@ class _DeltaQKV(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dq, dk, dv):
         mixed, = ctx.saved_tensors
-        if torch.is_grad_enabled():
+        if _beyond_kernels(dq, dk, dv):
             return _through_statement(ctx, (mixed,), (dq, dk, dv))
         return _ext().delta_qkv_bwd(*(_aligned(t) for t in (dq, dk, dv, mixed)), *ctx.cfg), None, None, None, None, None
 
@@ -394,7 +408,7 @@ class _DeltaRule(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do):
         q, k, v, beta, log_decay, *saved = ctx.saved_tensors
-        if torch.is_grad_enabled():
+        if _beyond_kernels(do):
             return _through_statement(ctx, (q, k, v, beta, log_decay), do)
         dq, dk, dv, db, dg = _ext().delta_rule_bwd(*(_aligned(t) for t in (do, q, k, v, beta, *saved)))
         return dq, dk, dv, db, dg.unsqueeze(-1), None
@@ -422,7 +436,7 @@ class _GatedRMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, gate, w = ctx.saved_tensors
-        if torch.is_grad_enabled():
+        if _beyond_kernels(dy):
             return _through_statement(ctx, (x, gate, w), dy)
         return (*_ext().gated_norm_bwd(*(_aligned(t) for t in (dy, x, gate, w)), ctx.eps), None, None)
 
@@ -579,7 +593,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
     def backward(ctx, g):
         dh, dw = ctx.saved_tensors
         need_dh, need_dw, wdt = ctx.flags
-        if torch.is_grad_enabled() or wdt != torch.bfloat16:        # create_graph: keep the expressions in the graph
+        if wdt != torch.bfloat16 or _beyond_kernels(g):
             return ((dh * g.to(dh.dtype)) if need_dh else None, ((dw * g).to(wdt)) if need_dw else None, None, None)
         scale = _ext().scale_to_bf16
         return scale(dh, g) if need_dh else None, scale(dw, g) if need_dw else None, None, None
@@ -602,7 +616,7 @@ class _CrossEntropySum(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (d,) = ctx.saved_tensors
-        if torch.is_grad_enabled():
+        if _beyond_kernels(g):
             return d * g.to(d.dtype), None
         return _ext().scale_to_bf16(d, g), None
 
