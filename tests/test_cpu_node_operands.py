@@ -134,3 +134,12 @@ def test_batched_gradients_of_the_losses_take_the_expressions(monkeypatch):
         for i in range(3):
             for a, b, t in zip(got, torch.autograd.grad(call(*leaves), leaves, dys[i], create_graph=True), leaves):
                 assert a[i].shape == t.shape and torch.equal(a[i], b)
+
+
+@pytest.mark.parametrize("owner,name", [(torch._C._functorch, "peek_interpreter_stack"), (torch._C, "_len_torch_dispatch_stack"),
+                                        (torch.autograd.forward_ad, "_current_level")])
+def test_a_torch_without_the_private_queries_takes_the_expressions(monkeypatch, owner, name):
+    assert F._has_rules(torch.ones(1))
+    monkeypatch.delattr(owner, name)
+    monkeypatch.setattr(F, "_NO_TRANSFORM", F._transform_probes())
+    assert not F._has_rules(torch.ones(1))

@@ -306,9 +306,22 @@ def swiglu(gate, up, row_limit=None):
 # Autograd nodes over kernels that took the place of tensor expressions. What the expressions could do and a node cannot stays with
 # them: `statement`, the same computation as tensor expressions, serves second derivatives and batched gradients, and `_has_rules` sends calls under
 # functorch transforms, forward-mode tangents, tracing and dispatch modes, and calls on tensor subclasses, back to the caller.
+def _transform_probes():
+    """What torch has no public query for: the functorch interpreter stack, the forward-mode level and the dispatch-mode stack. None on a
+    torch that names them differently: all calls then take the expressions, slower and never wrong."""
+    try:
+        stack, modes = torch._C._functorch.peek_interpreter_stack, torch._C._len_torch_dispatch_stack
+        forward_ad._current_level
+    except AttributeError:
+        return None
+    return lambda: stack() is None and modes() == 0 and forward_ad._current_level < 0
+
+
+_NO_TRANSFORM = _transform_probes()
+
+
 def _has_rules(*ts: torch.Tensor) -> bool:
-    return (torch._C._functorch.peek_interpreter_stack() is None and forward_ad._current_level < 0 and not torch.compiler.is_compiling()
-            and not torch.jit.is_tracing() and torch._C._len_torch_dispatch_stack() == 0
+    return (_NO_TRANSFORM is not None and _NO_TRANSFORM() and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in ts))
 
 
