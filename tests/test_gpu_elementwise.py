@@ -289,3 +289,21 @@ def test_qk_norm_rope_outputs_are_differentiated_apart():
     got = (torch.autograd.grad(yq, (q, ws[0]), dys[0]), torch.autograd.grad(yk, (k, ws[1]), dys[1]))
     for a, b in zip((got[0][0], got[1][0], got[0][1], got[1][1]), want):
         assert torch.equal(a, b)
+
+
+def test_traced_ops_follow_their_inputs():
+    """A trace calls the ops again on new inputs, forward and backward: nothing that an op computed while it was recorded is a constant."""
+    from torchllmtuner_b200 import ops
+    torch.manual_seed(0)
+    new = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    w, W, qw, ang = new(128), new(64, 128), new(64), torch.rand(16, 32, device="cuda")
+    calls = [(lambda x, y: ops.rms_norm(x + y, w, 1e-6), (16, 128)), (lambda x, y: ops.add_rms_norm(x, y, w, 1e-6), (16, 128)),
+             (lambda x, y: ops.swiglu(x, y), (16, 128)), (lambda x, y: ops.linear(x + y, W), (16, 128)), (lambda x, y: ops.linears(x + y, W, W), (16, 128)),
+             (lambda x, y: ops.qk_norm_rope(x, y, qw, None, ang.cos(), ang.sin(), 1e-6), (16, 2, 64))]
+    for call, shape in calls:
+        traced = torch.jit.trace(call, (new(*shape), new(*shape)), check_trace=False)
+        ins = [new(*shape).requires_grad_() for _ in range(2)]
+        ys = [t if isinstance(t, tuple) else (t,) for t in (traced(*ins), call(*ins))]
+        dys = [torch.randn_like(t) for t in ys[0]]
+        for a, b in zip((*ys[0], *torch.autograd.grad(ys[0], ins, dys)), (*ys[1], *torch.autograd.grad(ys[1], ins, dys))):
+            assert torch.equal(a, b)

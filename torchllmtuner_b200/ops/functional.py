@@ -40,13 +40,42 @@ _nodes = None
 
 def _native():
     """The extension with its C++ autograd nodes, or None while a peer-memory collective queue is active (products then go
-    through `gemm`, which hands the queue's next job to the kernel)."""
+    through `gemm`, which hands the queue's next job to the kernel) and under `torch.jit.trace` (see `_PythonNode`)."""
     global _nodes
     if _nodes is None:
         ext = _ext()
         ext.set_autograd_hooks(_symm_module(), _linears_backward)
         _nodes = ext
-    return _nodes if _symm._ACTIVE is None else None
+    return _nodes if _symm._ACTIVE is None and not torch.jit.is_tracing() else None
+
+
+class _PythonNode(torch.autograd.Function):
+    """A C++ node as one Python op. `torch.jit.trace` records a Python op by reference and calls it again whenever the trace runs; of a C++
+    node it would record the tensors that it returned, as constants. The backward computes the forward again."""
+
+    @staticmethod
+    def forward(ctx, node, *args):
+        ctx.node, ctx.rest = node, [None if isinstance(a, torch.Tensor) else a for a in args]
+        ctx.at = [i for i, a in enumerate(args) if isinstance(a, torch.Tensor)]
+        ctx.save_for_backward(*(args[i] for i in ctx.at))
+        out = node(*args)
+        return out if isinstance(out, torch.Tensor) else tuple(out)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        need = ctx.needs_input_grad[1:]
+        args = list(ctx.rest)
+        for i, t in zip(ctx.at, ctx.saved_tensors):
+            args[i] = t.detach().requires_grad_(need[i])
+        with torch.enable_grad():
+            outs = ctx.node(*args)
+        outs = (outs,) if isinstance(outs, torch.Tensor) else tuple(outs)
+        got = iter(torch.autograd.grad(outs, [a for a, n in zip(args, need) if n], dys, allow_unused=True))
+        return (None, *(next(got) if n else None for n in need))
+
+
+def _run_node(node, *args):
+    return _PythonNode.apply(node, *args) if torch.jit.is_tracing() else node(*args)
 
 
 def _use_cuda(t: torch.Tensor) -> bool:
@@ -271,14 +300,14 @@ def rms_norm(x, weight, eps: float):
     if not (isinstance(x, torch.Tensor) and isinstance(weight, torch.Tensor) and weight.dim() == 1 and x.shape[-1] == weight.shape[0]):
         validate_rms_norm_inputs(x, weight)
     if _use_cuda(x) and x.dtype == torch.bfloat16:
-        return _ext().rmsnorm_node(x, weight, eps)
+        return _run_node(_ext().rmsnorm_node, x, weight, eps)
     return ref.rms_norm(x, weight, eps)
 
 
 def add_rms_norm(x, residual, weight, eps: float):
     """Returns (rms_norm(x + residual), x + residual) with one pass over the data."""
     if _use_cuda(x) and x.dtype == torch.bfloat16:
-        return tuple(_ext().add_rmsnorm_node(x, residual, weight, eps))
+        return tuple(_run_node(_ext().add_rmsnorm_node, x, residual, weight, eps))
     return ref.add_rms_norm(x, residual, weight, eps)
 
 
@@ -289,7 +318,7 @@ rope_tables = ref.rope_tables
 def qk_norm_rope(q, k, q_weight, k_weight, cos, sin, eps: float):
     """q [T,Hq,d], k [T,Hkv,d] (views with packed heads are fine); cos/sin fp32 [T,d/2]."""
     if _use_cuda(q) and q.dtype == torch.bfloat16:
-        return tuple(_ext().qk_norm_rope_node(q, k, q_weight, k_weight, cos, sin, eps))
+        return tuple(_run_node(_ext().qk_norm_rope_node, q, k, q_weight, k_weight, cos, sin, eps))
     return ref.qk_norm_rope(q, k, q_weight, k_weight, cos, sin, eps)
 
 
@@ -298,7 +327,7 @@ def swiglu(gate, up, row_limit=None):
     """silu(gate) * up. `row_limit` (int32 device scalar) bounds the rows that are touched when the operands are
     statically sized buffers whose live row count is only known on the device (expert-parallel receive buffers)."""
     if _use_cuda(gate) and gate.dtype == torch.bfloat16:
-        return _ext().swiglu_node(gate, up, row_limit)
+        return _run_node(_ext().swiglu_node, gate, up, row_limit)
     return ref.swiglu(gate, up)
 
 
