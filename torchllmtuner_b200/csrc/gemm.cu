@@ -31,7 +31,7 @@ struct GemmRoles {
 
 // CG: CTAs that work on one tile. 1: a 128 x BN tile per CTA. 2: a 256 x BN tile per cluster of two CTAs (cta_group::2): each
 // CTA loads its 128 rows of A and its half of the B tile, the tensor cores of both SMs read both halves of B, and each CTA's
-// tensor memory receives its 128 rows of the product. See pick_tile() for when which is used.
+// tensor memory receives its 128 rows of the product. See use_pair() for when which is used.
 template <int CG, int BN, bool COMM>
 struct GemmCfg {
   static constexpr int kBRows = BN / CG;           // rows of B that this CTA loads

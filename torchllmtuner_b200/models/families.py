@@ -34,7 +34,9 @@ class HybridConfig(Qwen3Config):
     delta_heads: int = 4
     delta_head_dim: int = 32
     delta_channel_decay: bool = False          # True: KDA (per-channel decay), False: gated delta-net (per-head decay)
-    delta_chunk_size: int = 0                  # tokens per chunk of the chunk-parallel delta rule; 0: 64 (per-head decay) / 16 (KDA)
+    # tokens per chunk of the chunk-parallel delta rule as tensor expressions; 0: 64 (per-head decay) / 16 (KDA). The device kernels (one
+    # decay per head, head size 64 or 128) have chunks of 64
+    delta_chunk_size: int = 0
     attention_output_gate: bool = True
     kv_lora_rank: int = 64                     # latent attention
     qk_rope_dim: int = 32
@@ -76,7 +78,8 @@ def chunked_delta_rule(q, k, v, beta, log_decay, chunk: int = 64, initial_state=
     Everything that does not depend on S0 is computed for all chunks at once (batched matrix products and one batched
     triangular solve); only the [dk, dv] state update runs chunk after chunk. Decay ratios are only ever formed as
     exp(G_t - G_i) with i <= t, so nothing overflows however strong the decay. On the device the common form (one decay per
-    head, no state in or out) runs as four kernels in the same arithmetic; the chunk length is theirs then."""
+    head, no state in or out) runs as four kernels in the same arithmetic, whose chunks have 64 tokens: `chunk` then changes
+    nothing there (it never changes the result, only its rounding, time and memory)."""
     if initial_state is None and not return_state:
         o = ops.delta_rule(q, k, v, beta, log_decay, lambda *a: _chunk_expressions(*a, chunk))
         if o is not None:

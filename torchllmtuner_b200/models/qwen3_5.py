@@ -41,7 +41,7 @@ class Qwen35Config(Qwen3Config):
     linear_key_head_dim: int = 16
     linear_value_head_dim: int = 16
     linear_conv_kernel_dim: int = 4
-    linear_chunk_size: int = 64
+    linear_chunk_size: int = 64     # of the delta rule as tensor expressions; the device kernels (head size 64 or 128) have chunks of 64
     partial_rotary_factor: float = 0.25
     mrope_section: list[int] = field(default_factory=list)      # frequencies per axis (time, height, width); default: near-equal thirds
     attn_output_gate: bool = True
