@@ -99,12 +99,18 @@ def test_plan_segments_kernel_matches_tensor_statement(n, E, skew):
 
 
 def _poison(*sizes):
-    """Free bf16 blocks of these element counts full of NaN: buffers of those sizes that a call allocates next consist of them. Requests
-    up to 1 MB come from another pool of the allocator than larger ones, so the sizes have to be the call's own."""
-    junk = [torch.full((n,), float("nan"), device="cuda", dtype=torch.bfloat16) for n in sizes for _ in range(12)]
-    del junk
-    for n in sizes:
-        assert torch.empty(n, device="cuda", dtype=torch.bfloat16).isnan().all()
+    """Fill the allocator's free memory with NaN, so that whatever a call allocates next consists of them (bf16 element counts in `sizes`
+    are checked). Requests up to 1 MB come from another pool than larger ones, and both keep gaps between live tensors: blocks of
+    every size down to the allocator's 512 bytes fill them."""
+    def fill():
+        torch.cuda.empty_cache()
+        junk = [torch.full((1 << b,), float("nan"), device="cuda", dtype=torch.bfloat16) for b in range(24, 7, -1) for _ in range(24)]
+        del junk
+    fill()
+    probes = [torch.empty(n, device="cuda", dtype=torch.bfloat16) for n in sizes]
+    assert all(t.isnan().all() for t in probes)
+    del probes
+    fill()                                               # the check's own temporaries were free memory
 
 
 @pytest.mark.parametrize("T,E,k,D", [(3, 16, 2, 8), (130, 8, 4, 264), (257, 32, 8, 512), (65, 4, 1, 1032), (512, 4, 1, 64)])
