@@ -258,6 +258,21 @@ def test_scale_to_bf16(n, dtype):
     assert torch.equal(load().scale_to_bf16(x, g), (x.float() * g).bfloat16())
 
 
+@pytest.mark.parametrize("T,D", [(5, 256), (5, 264), (9472, 264), (9473, 264), (9473, 512), (3000, 1344)])
+def test_rmsnorm_forward_at_the_edges_of_its_rule(T, D):
+    """Widths of one vector per lane and one more, row counts on both sides of one wave of eight-row blocks on 148 SMs, and a
+    width between two groups."""
+    from torchllmtuner_b200 import ops
+    from torchllmtuner_b200.ops import reference as ref
+    torch.manual_seed(T + D)
+    x, r = (torch.randn(T, D, device="cuda").bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+    _close(ops.rms_norm(x, w, 1e-6), ref.rms_norm(x.float(), w.float(), 1e-6), name="y")
+    y, s = ops.add_rms_norm(x, r, w, 1e-6)
+    want, ws = ref.add_rms_norm(x.float(), r.float(), w.float(), 1e-6)
+    _close(y, want, name="y"), _close(s, ws, name="sum")
+
+
 def test_cross_entropy_gradient_of_a_confident_row():
     """Where the label's probability is close to 1, p - 1 is exact in fp32 and the gradient is that times the factor: the gradients of a
     factor of 1 and of 1/3 agree up to the rounding of each to bf16 (8 bits of significand: 2^-8 relative each, 2^-7 together). Rounding p times the factor first would leave an

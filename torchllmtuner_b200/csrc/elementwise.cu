@@ -53,8 +53,8 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
 
 // ------------------------------------------------------------------------------------------ RMSNorm
 // A row is owned by TR threads (a warp up to the whole block), each holding NV groups of 8 columns:
-// col = (v * TR + t) * 8, so that narrow rows (a 512-wide model: 64 vectors) leave no thread idle. Bound by memory; TR is the
-// smallest group that covers the row with NV = 2 (two 16-byte loads per operand in flight per thread, TR = 32 needs no barrier).
+// col = (v * TR + t) * 8, so that narrow rows (a 512-wide model: 64 vectors) leave no thread idle. Bound by memory; NV and TR by
+// width in fwd_by_row_width and bwd_by_row_width (TR = 32 needs no barrier).
 // The forward gives a group a block of its own (or a warp of an eight-row block): named barriers with a computed id reserve
 // all sixteen of a block and then only four blocks fit an SM (57 us against 42 us at 8192 x 4096). The backward, which has two
 // blocks per SM anyway, puts 256 / TR groups into a block to keep the number of weight-gradient partials down.
@@ -816,15 +816,33 @@ using namespace llmt;
 
 #define LLMT_CHECK_LAUNCH() return (cudaGetLastError() == cudaSuccess) ? 0 : -3
 
-// The row kernels by width: the smallest thread group that covers a row with two vectors per thread. WIDE is the pair for
-// rows above 4096: the forward takes four vectors on 256 threads, the backward (which would spill) two on 512.
-template <int WIDE_NV, int WIDE_TR, typename F>
-static inline void by_row_width(int D, F&& f) {
-  if (D <= 512) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 32>{});
-  else if (D <= 1024) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 64>{});
-  else if (D <= 2048) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 128>{});
-  else if (D <= 4096) f(std::integral_constant<int, 2>{}, std::integral_constant<int, 256>{});
-  else f(std::integral_constant<int, WIDE_NV>{}, std::integral_constant<int, WIDE_TR>{});
+// The forward by width: the smallest thread group that covers a row with one vector per thread, up to 256 threads (two or four
+// vectors beyond). A row's time is the chain load - reduce - store, which a second vector lengthens, and the two-vector groups of 64 and
+// 128 threads take 40 registers, so that only 12 of 16 blocks of the grid are resident. us without / with the residual, two vectors on
+// half the threads -> one vector: 2048 x 704 3.4 / 4.0 -> 3.0 / 3.7, 2048 x 1344 5.1 / 7.5 -> 4.2 / 5.7, 13434 x 1024 13.6 / 20.7 ->
+// 11.8 / 20.2, 13434 x 2048 25.6 / 45.8 -> 22.2 / 38.2. Rows of 257 to 512 are the exception once there is more than a wave of
+// blocks of eight rows: 13434 x 512 5.9 / 10.1 us with a warp per row against 6.2 / 10.9, but 2048 x 512 3.0 / 3.6 against 2.6 / 3.6.
+template <typename F>
+static inline void fwd_by_row_width(int T, int D, F&& f) {
+  using std::integral_constant;
+  if (D <= 256) f(integral_constant<int, 1>{}, integral_constant<int, 32>{});
+  else if (D <= 512 && T > 64 * sm_count()) f(integral_constant<int, 2>{}, integral_constant<int, 32>{});
+  else if (D <= 512) f(integral_constant<int, 1>{}, integral_constant<int, 64>{});
+  else if (D <= 1024) f(integral_constant<int, 1>{}, integral_constant<int, 128>{});
+  else if (D <= 2048) f(integral_constant<int, 1>{}, integral_constant<int, 256>{});
+  else if (D <= 4096) f(integral_constant<int, 2>{}, integral_constant<int, 256>{});
+  else f(integral_constant<int, 4>{}, integral_constant<int, 256>{});
+}
+// The backward by width: the smallest thread group that covers a row with two vectors per thread (it prefetches the next row, so its
+// chain is hidden, and fewer groups mean fewer partial sums); above 4096 two vectors on 512 threads, as four would spill.
+template <typename F>
+static inline void bwd_by_row_width(int D, F&& f) {
+  using std::integral_constant;
+  if (D <= 512) f(integral_constant<int, 2>{}, integral_constant<int, 32>{});
+  else if (D <= 1024) f(integral_constant<int, 2>{}, integral_constant<int, 64>{});
+  else if (D <= 2048) f(integral_constant<int, 2>{}, integral_constant<int, 128>{});
+  else if (D <= 4096) f(integral_constant<int, 2>{}, integral_constant<int, 256>{});
+  else f(integral_constant<int, 2>{}, integral_constant<int, 512>{});
 }
 
 extern "C" int llmt_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* sum_out, float* rstd, int T,
@@ -833,7 +851,7 @@ extern "C" int llmt_rmsnorm_fwd(const void* x, const void* res, const void* w, v
   if (D % 8 || D > 8 * kRowThreads * 4) return -10;
   auto X = (const __nv_bfloat16*)x; auto R = (const __nv_bfloat16*)res; auto W = (const __nv_bfloat16*)w;
   auto Y = (__nv_bfloat16*)y; auto S = (__nv_bfloat16*)sum_out;
-  by_row_width<4, 256>(D, [&](auto nv, auto tr) {
+  fwd_by_row_width(T, D, [&](auto nv, auto tr) {
     constexpr int TR = decltype(tr)::value, NT = TR > 32 ? TR : kRowThreads, RPB = NT / TR;
     const int blocks = (T + RPB - 1) / RPB, cap = sm_count() * (2048 / NT);
     rmsnorm_fwd_kernel<decltype(nv)::value, TR><<<blocks < cap ? blocks : cap, NT, 0, st>>>(X, R, W, Y, S, rstd, T, D, eps);
@@ -855,7 +873,7 @@ extern "C" int llmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
   auto DY = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
   auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
   int grid = 0;
-  by_row_width<2, 512>(D, [&](auto nv, auto tr) {
+  bwd_by_row_width(D, [&](auto nv, auto tr) {
     constexpr int NV = decltype(nv)::value, TR = decltype(tr)::value, NT = RowBlock<TR>::kThreads, RPB = RowBlock<TR>::kRows;
     const int blocks = (T + RPB - 1) / RPB, most = llmt_rmsnorm_bwd_partials(T), cap = NT > 256 ? (most + 1) / 2 : most;
     grid = blocks < cap ? blocks : cap;
