@@ -211,7 +211,9 @@ def test_rmsnorm_at_the_edges_of_the_row_groups(T, D):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("n", [1, 7, 8, 255, 257, 4097, 303104, 303105, 5000003, 20000008])
+@pytest.mark.parametrize("n", [1, 7, 8, 255, 257, 4097, 303104, 303105, 5000003, 20000008,
+                               # 1 to 31 steps of 303104 elements and a few more: every combination of batch sizes
+                               *(303104 * k + 4 * k + 3 for k in (1, 2, 3, 5, 7, 10, 15, 16, 23, 31))])
 def test_sq_norm_has_the_same_bits_on_any_alignment(n, dtype):
     """The kernel for 16-byte aligned data and the one for any slice add the same terms in the same order: equal bits. Thousands of
     fp32 terms per partial sum stay within 1e-5 of the 64-bit sum."""

@@ -749,21 +749,26 @@ __global__ void __launch_bounds__(256, 1) sqnorm_partial_vec_kernel(const T* __r
     for (int e = 0; e < 8; ++e) s[e] += f[e] * f[e];
   };
   int64_t i = (int64_t)vb * 256 + lane * 8;
-  for (; i + (U - 1) * nt + 8 <= n; i += U * nt) {
-    uint4 u[U][kWords];
+  auto batch = [&](auto nc) -> bool {                  // N vectors, all in flight before the first is added; false: fewer are left
+    constexpr int N = decltype(nc)::value;
+    if (i + (N - 1) * nt + 8 > n) return false;
+    uint4 u[N][kWords];
 #pragma unroll
-    for (int k = 0; k < U; ++k)
+    for (int k = 0; k < N; ++k)
 #pragma unroll
       for (int w = 0; w < kWords; ++w) u[k][w] = ld_stream(reinterpret_cast<const uint4*>(x + i + k * nt) + w);
 #pragma unroll
-    for (int k = 0; k < U; ++k) add(u[k]);
-  }
-  for (; i + 8 <= n; i += nt) {
-    uint4 u[kWords];
-#pragma unroll
-    for (int w = 0; w < kWords; ++w) u[w] = ld_stream(reinterpret_cast<const uint4*>(x + i) + w);
-    add(u);
-  }
+    for (int k = 0; k < N; ++k) add(u[k]);
+    i += N * nt;
+    return true;
+  };
+  while (batch(std::integral_constant<int, U>{})) {}
+  // the rest in halving batches: one vector after another, up to U - 1 of them were as long a chain as the whole of a mid-sized tensor
+  // (4.6 M bf16 values 11.7 us, against 8.6 with the scalar loads below)
+  if constexpr (U > 8) batch(std::integral_constant<int, 8>{});
+  batch(std::integral_constant<int, 4>{});
+  batch(std::integral_constant<int, 2>{});
+  batch(std::integral_constant<int, 1>{});
 #pragma unroll
   for (int e = 0; e < 8; ++e)
     if (i + e < n) {
