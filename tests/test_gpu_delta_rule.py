@@ -159,6 +159,29 @@ def test_delta_rule_kernels_match_the_scan_in_64_bits(T, H, d, decay):
         assert torch.equal(ops.delta_rule(*x), o)      # the form without a backward
 
 
+@pytest.mark.parametrize("H,d", [(2, 64), (1, 128)])
+def test_long_documents_of_few_heads_take_the_expressions(H, d):
+    """Both sides of the rule that sends a long document with few heads to the tensor expressions, and the two forms against each other
+    beyond it (each within 2e-5 of 64 bits at the lengths above; the states of a thousand chunks decay, so length adds nothing)."""
+    from torchllmtuner_b200 import ops
+    from torchllmtuner_b200.models.families import chunked_delta_rule
+    from torchllmtuner_b200.ops.functional import _DeltaRule
+    g = torch.Generator(device="cuda").manual_seed(d)
+    T = (1 << 22) // d + 1
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x = [F.normalize(r(T, H, d), dim=-1), F.normalize(r(T, H, d), dim=-1), r(T, H, d), torch.rand(T, H, generator=g, device="cuda"), -F.softplus(r(T, H, 1))]
+    x = [t.requires_grad_() for t in x]
+    assert ops.delta_rule(*x) is None and ops.delta_rule(*(t[:-1] for t in x)) is not None
+    with torch.no_grad():
+        assert ops.delta_rule(*(t[:-1] for t in x)) is None and ops.delta_rule(*(t[:(1 << 21) // d] for t in x)) is not None
+    many = [t.detach().repeat_interleave(4, 1).requires_grad_() for t in x]
+    assert ops.delta_rule(*many) is not None
+    do = r(T, H, d)
+    a, b = _DeltaRule.apply(*x, None), chunked_delta_rule(*x)
+    for p, q in zip((a, *torch.autograd.grad(a, x, do)), (b, *torch.autograd.grad(b, x, do))):
+        assert (p - q).norm() <= 4e-5 * q.norm()
+
+
 def test_second_derivatives_and_transforms_of_the_delta_rule():
     """What the node cannot do stays with the tensor expressions: a gradient of the gradient, forward-mode derivatives and vmap give
     what 64 bits give (a second derivative sums a few thousand fp32 terms of its own size: 1e-4 of the largest)."""

@@ -456,14 +456,25 @@ class _DeltaRule(torch.autograd.Function):
         return dq, dk, dv, db, dg.unsqueeze(-1), None
 
 
+def _long_chain(T: int, H: int, D: int, grad: bool) -> bool:
+    """Few heads and a long document: the scan kernels walk the chunks one after another on H x D / 32 SMs (5.2 us a chunk at head size 64,
+    8.1 at 128, the same again backwards), while the tensor expressions scan over chunk states in about 2 sqrt(chunks) steps. Forward +
+    backward ms, kernels / expressions: 65536 tokens 1 x 64 10.9 / 9.9, 4 x 64 12.0 / 12.7, 2 x 128 17.3 / 12.1, 4 x 128 18.6 / 19.8;
+    131072 tokens 4 x 64 23.9 / 19.4, 8 x 64 26.5 / 33.6, 3 x 128 35.8 / 29.9, 4 x 128 37.0 / 38.9; 32768 tokens 2 x 128 8.7 / 8.8.
+    Forward alone crosses at half the length: 32768 tokens 4 x 64 2.8 / 2.5, 16384 tokens 2 x 128 2.1 / 1.9."""
+    return H <= (4 if D == 64 else 3) and T * D > (1 << 22 if grad else 1 << 21)
+
+
 def delta_rule(q, k, v, beta, log_decay, statement=None):
     """The gated delta rule with one decay per head and zero initial state: q, k, v [T, H, d], beta [T, H], log_decay [T, H, 1]
     (<= 0), fp32 -> [T, H, d] (the recurrence of `models.families.delta_rule_scan`). None where the kernels have no form for the
-    call."""
+    call or the tensor expressions are faster."""
     ts = (q, k, v, beta, log_decay)
     if not (_use_cuda(q) and all(t.dtype == torch.float32 and t.is_cuda for t in ts) and q.shape == k.shape == v.shape and q.dim() == 3
             and q.shape[-1] in (64, 128) and q.shape[0] > 0 and tuple(beta.shape) == tuple(q.shape[:2])
             and tuple(log_decay.shape) == (*q.shape[:2], 1) and _has_rules(*ts)):
+        return None
+    if _long_chain(*q.shape, torch.is_grad_enabled() and any(t.requires_grad for t in ts)):
         return None
     return _DeltaRule.apply(*ts, statement)
 
