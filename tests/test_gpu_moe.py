@@ -98,23 +98,18 @@ def test_plan_segments_kernel_matches_tensor_statement(n, E, skew):
         assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
 
 
-def _poison(*sizes):
-    """Fill the allocator's free memory with NaN, so that whatever a call allocates next consists of them (bf16 element counts in `sizes`
-    are checked). Requests up to 1 MB come from another pool than larger ones, and both keep gaps between live tensors: blocks of
-    every size down to the allocator's 512 bytes fill them."""
-    def fill():
-        torch.cuda.empty_cache()
-        junk = [torch.full((1 << b,), float("nan"), device="cuda", dtype=torch.bfloat16) for b in range(24, 7, -1) for _ in range(24)]
-        del junk
-    fill()
-    probes = [torch.empty(n, device="cuda", dtype=torch.bfloat16) for n in sizes]
-    assert all(t.isnan().all() for t in probes)
-    del probes
-    fill()                                               # the check's own temporaries were free memory
+@pytest.fixture
+def poisoned():
+    """Every buffer that is allocated without a value is full of NaN (torch's deterministic mode does that)."""
+    before, warn = torch.are_deterministic_algorithms_enabled(), torch.is_deterministic_algorithms_warn_only_enabled()
+    torch.use_deterministic_algorithms(True, warn_only=True)
+    assert torch.utils.deterministic.fill_uninitialized_memory and torch.empty(64, device="cuda", dtype=torch.bfloat16).isnan().all()
+    yield
+    torch.use_deterministic_algorithms(before, warn_only=warn)
 
 
 @pytest.mark.parametrize("T,E,k,D", [(3, 16, 2, 8), (130, 8, 4, 264), (257, 32, 8, 512), (65, 4, 1, 1032), (512, 4, 1, 64)])
-def test_padding_rows_are_written(T, E, k, D):
+def test_padding_rows_are_written(poisoned, T, E, k, D):
     """The dispatch copy and the combine's backward on buffers full of NaN: every copy arrives, every padding row of a segment is zero
     and rows past the last segment are not touched."""
     from torchllmtuner_b200.models.moe.experts import padded_capacity, plan_segments
@@ -131,19 +126,17 @@ def test_padding_rows_are_written(T, E, k, D):
     load().permute_rows(x, dest, rows, k, seg, counts)
     assert torch.equal(rows[dest], x.repeat_interleave(k, 0)) and (rows[padding] == 0).all() and rows[end:].isnan().all()
     y = torch.randn(cap, D, device="cuda").bfloat16()
-    _poison(cap * D)
     dy, dw = load().combine_bwd(x, y, dest, w, k, seg, counts)
     want = (w[:, None] * x.repeat_interleave(k, 0).float()).bfloat16()
     assert torch.equal(dy[dest], want) and (dy[padding] == 0).all() and dw.isfinite().all()
 
 
 @pytest.mark.parametrize("T,E,k,D,F_", [(3, 16, 2, 8, 64), (130, 8, 4, 264, 72), (257, 32, 8, 512, 136), (65, 4, 1, 1032, 64)])
-def test_routed_experts_write_their_padding_rows(T, E, k, D, F_):
+def test_routed_experts_write_their_padding_rows(poisoned, T, E, k, D, F_):
     """Buffers are no longer cleared before use: the same call on poisoned memory gives finite results that match the CPU
     statement, for narrow rows, a top-k that is no multiple of the combine's eight loads, and empty experts."""
-    from torchllmtuner_b200.models.moe.experts import GroupedExperts, RoutedExperts, padded_capacity
+    from torchllmtuner_b200.models.moe.experts import GroupedExperts, RoutedExperts
     torch.manual_seed(T)
-    cap = padded_capacity(T * k, E)
     gpu = RoutedExperts(GroupedExperts(E, D, F_, dtype=torch.bfloat16, device="cuda"))
     cpu = RoutedExperts(GroupedExperts(E, D, F_, dtype=torch.float32))
     for p, q in zip(gpu.parameters(), cpu.parameters()):
@@ -154,10 +147,8 @@ def test_routed_experts_write_their_padding_rows(T, E, k, D, F_):
     idx = torch.randint(0, E, (T, k), device="cuda")
     xc, wc = x.detach().float().cpu().requires_grad_(), w.detach().cpu().requires_grad_()
     go = torch.randn(T, D, device="cuda").bfloat16()
-    for _ in range(2):
-        _poison(cap * D, cap * F_, 2 * cap * F_)
-        yg = gpu(x, w, idx)
-        gg = torch.autograd.grad(yg, [x, w, *gpu.parameters()], go)
+    yg = gpu(x, w, idx)
+    gg = torch.autograd.grad(yg, [x, w, *gpu.parameters()], go)
     yc = cpu(xc, wc, idx.cpu())
     gc = torch.autograd.grad(yc, [xc, wc, *cpu.parameters()], go.float().cpu())
     for a, b in zip((yg, *gg), (yc, *gc)):
