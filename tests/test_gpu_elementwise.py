@@ -251,6 +251,29 @@ def test_cross_entropy_kernel_at_its_size_limits(rows, V, mask):
     _close(x, dref.float(), name="dlogits")
 
 
+@pytest.mark.parametrize("rows", [2, 600])
+@pytest.mark.parametrize("V", [4096, 4104, 8192, 8200, 16384, 16392, 76800, 76808])
+def test_cross_entropy_kernel_on_both_sides_of_its_rule(rows, V):
+    """Thread counts depend on the width, on whether there are more rows than SMs and on whether gradients are written: loss and gradients
+    against 64 bits, and the loss alone leaves the logits as they are."""
+    from torchllmtuner_b200.ops.cuda_ext import load
+    torch.manual_seed(V)
+    x, y = torch.randn(rows, V, device="cuda").mul_(3).bfloat16(), torch.randint(0, V, (rows,), device="cuda")
+    lf = x.double()
+    lse_ref = lf.logsumexp(-1)
+    want = lse_ref - lf.gather(1, y[:, None])[:, 0]
+    for grad in (False, True):
+        buf = x.clone()
+        loss, lse = load().ce_fwd_bwd(buf, y, 0.5, None, -100, grad)
+        assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5) and torch.allclose(lse.double(), lse_ref, rtol=1e-5, atol=1e-5)
+        if grad:
+            d = (lf - lse_ref[:, None]).exp_()
+            d[torch.arange(rows, device="cuda"), y] -= 1
+            _close(buf, d.mul_(0.5).float(), name="dlogits")
+        else:
+            assert torch.equal(buf, x)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n", [1, 7, 8, 1000003])
 def test_scale_to_bf16(n, dtype):

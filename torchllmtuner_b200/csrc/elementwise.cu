@@ -986,12 +986,17 @@ extern "C" int llmt_ce_fwd_bwd(void* logits, const int64_t* labels, float* row_l
     ce_fwd_bwd_kernel<NT><<<rows, NT, (size_t)cached * 16, st>>>(L, labels, row_loss, row_lse, V, ld, grad_scale_ptr, grad_scale, ignore_index,
                                                                  write_grad, cached);
   };
-  // Rows in flight times their size decides: up to 150 KB a row, four blocks of 512 threads per SM stay inside L2 (592 rows);
-  // beyond that two blocks of 1024 with 64 KB of each row in shared memory do. Measured us, 256 / 512 / 1024 threads at
-  // 1024 x 4096: 11 / - / -, 4096 x 32000: - / 98 / 115, 2048 x 50000: - / 82 / 90, 2048 x 151936: - / 281 / 252.
-  if (V <= 8192) go(std::integral_constant<int, 256>{}, 1024);
-  else if (V <= 76800) go(std::integral_constant<int, 512>{}, 2560);
-  else go(std::integral_constant<int, 1024>{}, 4096);
+  // With more rows than SMs, rows in flight times their size decides: up to 150 KB a row, four blocks of 512 threads per SM stay
+  // inside L2 (592 rows); beyond that two blocks of 1024 with 64 KB of each row in shared memory do. Without gradients nothing is
+  // read twice: 512 threads there too. Measured us, 256 / 512 / 1024 threads at 1000 x 4096: 6.8 / 8.6 / 13, 4000 x 32000: 98 / 96 / 114,
+  // 2000 x 50000: 95 / 80 / 89, 2000 x 151936: 300 / 274 / 247; no gradients 4000 x 76808: 101 / 103 / 121.
+  // Up to one row per SM it is the chain of one row: 110 x 4096 2.8 / 2.9 / 3.1, 40 x 11728 4.4 / 3.8 / 4.2, 40 x 20536 6.3 / 5.5 / 4.9,
+  // 110 x 76800 25 / 17 / 13.
+  const bool few = rows <= sm_count();
+  using std::integral_constant;
+  if (V <= (few ? 4096 : 8192)) go(integral_constant<int, 256>{}, 1024);
+  else if (V <= (few ? 16384 : 76800) || !(few || write_grad)) go(integral_constant<int, 512>{}, 2560);
+  else go(integral_constant<int, 1024>{}, 4096);
   LLMT_CHECK_LAUNCH();
 }
 
