@@ -97,6 +97,23 @@ def test_gated_rms_norm_off_the_16_byte_boundary():
     _same_from_shifted(lambda *a: ops.gated_rms_norm(*a, 1e-6), (x, gate, w), (dy,))
 
 
+def test_causal_conv_silu_on_any_positions():
+    """Positions that no packed row has (negative, beyond the row's own index, jumping): the node takes what the tensor expressions take."""
+    from torchllmtuner_b200.models.kimi_k3 import CausalConvolution
+    torch.manual_seed(6)
+    x, dy = (torch.randn(50, 16, device="cuda").bfloat16() for _ in range(2))
+    conv = CausalConvolution(16, 4, dtype=torch.float32, device="cuda")
+    torch.nn.init.normal_(conv.weight)
+    conv.weight.data.copy_(conv.weight.data.bfloat16())
+    low = CausalConvolution(16, 4, dtype=torch.bfloat16, device="cuda")
+    low.load_state_dict(conv.state_dict())
+    pos = torch.randint(-2, 5, (50,), device="cuda")
+    a, b = x.clone().requires_grad_(), x.float().requires_grad_()
+    y, want = low(a, pos), conv(b, pos)
+    g, gw = torch.autograd.grad(y, [a, low.weight], dy), torch.autograd.grad(want, [b, conv.weight], dy.float())
+    _close(y, want, "y"); _close(g[0], gw[0], "dx"); _close(g[1], gw[1], "dw", True)
+
+
 @pytest.mark.parametrize("T,C", [(65536, 16), (65537, 16), (1048640, 8)])
 def test_causal_conv_silu_on_long_rows(T, C):
     """Rows on both sides of the length from which a block walks more than 16 of them, and more than 65535 blocks of 16 would cover:

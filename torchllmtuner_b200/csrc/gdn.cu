@@ -23,7 +23,7 @@ __device__ __forceinline__ uint4 down8(const float* f) {
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
 // ------------------------------------------------------------------------------------------ causal convolution + SiLU
-// z[t, c] = sum_j x[t - j, c] * w[c, K - 1 - j] over the taps j <= pos[t] (the index of row t in its document); y = silu(z).
+// z[t, c] = sum_j x[t - j, c] * w[c, K - 1 - j] over j = 0 and the taps j <= pos[t] (the index of row t in its document); y = silu(z).
 // Bound by memory: a thread owns 8 channels and walks the `tok` rows of its block with the last K rows in registers, so every row is
 // read once (plus K - 1 rows per block). 2048 x 8192, K = 4: 25 us forward, 86 us backward (67 and 100 MB; as tensor expressions about 1.1 ms together).
 // 16 rows per block; rows of more than 16 x kConvBlocks tokens get longer blocks, which bounds the grid (gridDim.y ends at 65535) and the
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const __nv_bfloat16*
     float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      if (p < j) continue;
+      if (j > 0 && p < j) continue;
       float f[8];
       up8(win[j], f);
 #pragma unroll
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const __nv_bfloat16*
     up8(*reinterpret_cast<const uint4*>(dy + (int64_t)t * lddy + c), d);
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      if (ps[0] < j) continue;
+      if (j > 0 && ps[0] < j) continue;
       float f[8];
       up8(win[j], f);
 #pragma unroll
@@ -118,14 +118,14 @@ __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const __nv_bfloat16*
       float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int j = 0; j < K; ++j) {
-        if (ps[j] < j) continue;                       // also rows beyond the last one (pos -1)
+        if (j > 0 && ps[j] < j) continue;              // also rows beyond the last one (pos -1)
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] += dz[j][i] * wt[i][j];
       }
       *reinterpret_cast<uint4*>(dx + (int64_t)t * C + c) = down8(o);
 #pragma unroll
       for (int j = 0; j < K; ++j) {
-        if (ps[0] < j) continue;
+        if (j > 0 && ps[0] < j) continue;
         float f[8];
         up8(win[j], f);
 #pragma unroll
