@@ -60,23 +60,40 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
 // blocks per SM anyway, puts 256 / TR groups into a block to keep the number of weight-gradient partials down.
 // 8192 x 4096 bf16 with the residual: forward 42 us, backward 50 us + 3.5 us for the column sums (before: 95 + 14 us, one row
 // after another without the prefetch); the 268 MB that each reads and writes take 42 us at copy speed.
-template <int TR, bool ONE_GROUP>
-__device__ __forceinline__ float row_sum(float v, float* red, int& buf) {
-  v = warp_sum(v);
-  if constexpr (TR > 32) {
-    // one barrier per row: the partial sums alternate between two buffers, and no warp can be two rows ahead
-    constexpr int NW = TR / 32;
-    const int grp = threadIdx.x / TR, t = threadIdx.x % TR;
-    float* r = red + buf * ((TR > kRowThreads ? TR : kRowThreads) / 32) + grp * NW;
-    if ((t & 31) == 0) r[t >> 5] = v;
-    if constexpr (ONE_GROUP) __syncthreads();
-    else named_bar_sync(1 + grp, TR);
-    v = r[0];
+// The order of a row's additions is that of 256 threads with one vector each up to 2048 columns (two or four beyond), whatever group
+// computes it: a group whose threads hold PARTS vectors of such a row keeps their sums apart, and the partial sums of the warps meet in
+// a tree. Bits then do not depend on the group, and a rounding that differs here travels through a whole network of bf16 layers.
+template <int TR, int NV>
+__host__ __device__ constexpr int row_parts() { return TR * NV <= kRowThreads ? NV : 1; }
+template <int TR, int PARTS, bool ONE_GROUP>
+__device__ __forceinline__ float row_sum(const float (&v)[PARTS], float* red, int& buf) {
+  constexpr int NW = TR / 32, N = NW * PARTS;
+  const int t = threadIdx.x % TR;
+  float s = v[0];
+  if constexpr (PARTS == 2) {                          // two warp sums for six shuffles: each half of the warp finishes one of them
+    const bool hi = threadIdx.x & 16;
+    s = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 16);
 #pragma unroll
-    for (int i = 1; i < NW; ++i) v += r[i];
-    buf ^= 1;
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  } else {
+    static_assert(PARTS == 1, "one or two vectors whose sums are kept apart");
+    s = warp_sum(s);
   }
-  return v;
+  if constexpr (TR == 32) return PARTS == 2 ? s + __shfl_xor_sync(0xffffffffu, s, 16) : s;
+  // one barrier per row: the partial sums alternate between two buffers, and no warp can be two rows ahead
+  float* r = red + buf * (PARTS * (TR > kRowThreads ? TR : kRowThreads) / 32) + threadIdx.x / TR * N;
+  if ((t & (32 / PARTS - 1)) == 0) r[(PARTS == 2 ? (t >> 4 & 1) * NW : 0) + (t >> 5)] = s;
+  if constexpr (ONE_GROUP) __syncthreads();
+  else named_bar_sync(1 + threadIdx.x / TR, TR);
+  float a[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) a[i] = r[i];
+  buf ^= 1;
+#pragma unroll
+  for (int o = N / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) a[i] += a[i + o];
+  return a[0];
 }
 __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
   const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
@@ -96,13 +113,13 @@ __global__ void __launch_bounds__(TR > 32 ? TR : kRowThreads) rmsnorm_fwd_kernel
                                                                   __nv_bfloat16* __restrict__ y,
                                                                   __nv_bfloat16* __restrict__ sum_out,
                                                                   float* __restrict__ rstd, int T, int D, float eps) {
-  __shared__ float red[2 * (kRowThreads / 32)];
-  constexpr int RPB = TR > 32 ? 1 : kRowThreads / TR;
+  constexpr int RPB = TR > 32 ? 1 : kRowThreads / TR, PARTS = row_parts<TR, NV>();
+  __shared__ float red[2 * PARTS * (kRowThreads / 32)];
   const int t = threadIdx.x % TR;
   int buf = 0;
   for (int row = blockIdx.x * RPB + threadIdx.x / TR; row < T; row += gridDim.x * RPB) {
     float v[NV][8];
-    float ss = 0.f;
+    float ss[PARTS] = {0.f};
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int col = (i * TR + t) * 8;
@@ -116,11 +133,10 @@ __global__ void __launch_bounds__(TR > 32 ? TR : kRowThreads) rmsnorm_fwd_kernel
           if (sum_out != nullptr) store8(sum_out + (int64_t)row * D + col, v[i]);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
+        for (int j = 0; j < 8; ++j) ss[PARTS > 1 ? i : 0] += v[i][j] * v[i][j];
       }
     }
-    ss = row_sum<TR, true>(ss, red, buf);
-    const float r = rsqrtf(ss / (float)D + eps);
+    const float r = rsqrtf(row_sum<TR, PARTS, true>(ss, red, buf) / (float)D + eps);
     if (t == 0 && rstd != nullptr) rstd[row] = r;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -151,8 +167,8 @@ __global__ void __launch_bounds__(RowBlock<TR>::kThreads, 512 / RowBlock<TR>::kT
                                                                      const __nv_bfloat16* __restrict__ dres,
                                                                      __nv_bfloat16* __restrict__ dx,
                                                                      float* __restrict__ dw_partial, int T, int D) {
-  constexpr int NT = RowBlock<TR>::kThreads, RPB = RowBlock<TR>::kRows;
-  __shared__ float red[2 * (NT / 32)];
+  constexpr int NT = RowBlock<TR>::kThreads, RPB = RowBlock<TR>::kRows, PARTS = row_parts<TR, NV>();
+  __shared__ float red[2 * PARTS * (NT / 32)];
   __shared__ float parts[RPB > 1 ? RPB * NV * TR * 8 : 1];
   const int t = threadIdx.x % TR, grp = threadIdx.x / TR;
   int buf = 0;
@@ -186,22 +202,21 @@ __global__ void __launch_bounds__(RowBlock<TR>::kThreads, 512 / RowBlock<TR>::kT
   int row = blockIdx.x * RPB + grp;
   if (row < T) fetch(row, xr, dr, er, r);
   for (; row < T; row += step) {
-    float c = 0.f;
+    float c[PARTS] = {0.f};
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       float xv[8], d[8], wv[8];
       unpack8(xr[i], xv); unpack8(dr[i], d); unpack8(wr[i], wv);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        c += d[j] * wv[j] * xv[j];
+        c[PARTS > 1 ? i : 0] += d[j] * wv[j] * xv[j];
         dw[i][j] += d[j] * xv[j] * r;
       }
     }
     uint4 nx[NV], nd[NV], ne[NV];
     float nr = 0.f;
     if (row + step < T) fetch(row + step, nx, nd, ne, nr);
-    c = row_sum<TR, (RPB == 1)>(c, red, buf);
-    const float k = r * r * r * c / (float)D;
+    const float k = r * r * r * row_sum<TR, PARTS, (RPB == 1)>(c, red, buf) / (float)D;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int col = (i * TR + t) * 8;
