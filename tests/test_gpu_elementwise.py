@@ -252,7 +252,7 @@ def test_cross_entropy_kernel_at_its_size_limits(rows, V, mask):
 
 
 @pytest.mark.parametrize("rows", [2, 600])
-@pytest.mark.parametrize("V", [4096, 4104, 8192, 8200, 16384, 16392, 76800, 76808])
+@pytest.mark.parametrize("V", [4096, 4104, 8192, 8200, 16384, 16392, 51200, 51208, 76800, 76808])
 def test_cross_entropy_kernel_on_both_sides_of_its_rule(rows, V):
     """Thread counts depend on the width, on whether there are more rows than SMs and on whether gradients are written: loss and gradients
     against 64 bits, and the loss alone leaves the logits as they are."""

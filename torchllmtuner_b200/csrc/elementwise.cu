@@ -1003,13 +1003,14 @@ extern "C" int llmt_ce_fwd_bwd(void* logits, const int64_t* labels, float* row_l
   };
   // With more rows than SMs, rows in flight times their size decides: up to 150 KB a row, four blocks of 512 threads per SM stay
   // inside L2 (592 rows); beyond that two blocks of 1024 with 64 KB of each row in shared memory do. Without gradients nothing is
-  // read twice: 512 threads there too. Measured us, 256 / 512 / 1024 threads at 1000 x 4096: 6.8 / 8.6 / 13, 4000 x 32000: 98 / 96 / 114,
-  // 2000 x 50000: 95 / 80 / 89, 2000 x 151936: 300 / 274 / 247; no gradients 4000 x 76808: 101 / 103 / 121.
+  // read twice: 512 threads there too, and 256 for more than four rows per SM of up to 51200 columns. Measured us, 256 / 512 / 1024 threads at 1000 x 4096: 6.8 / 8.6 / 13, 4000 x 32000: 98 / 96 / 114,
+  // 2000 x 50000: 95 / 80 / 89, 2000 x 151936: 300 / 274 / 247; no gradients 4000 x 20536: 33 / 41 / 59, 1000 x 76800: 31.5 / 30.7 / 33.6,
+  // 4000 x 76808: 101 / 103 / 121.
   // Up to one row per SM it is the chain of one row: 110 x 4096 2.8 / 2.9 / 3.1, 40 x 11728 4.4 / 3.8 / 4.2, 40 x 20536 6.3 / 5.5 / 4.9,
   // 110 x 76800 25 / 17 / 13.
   const bool few = rows <= sm_count();
   using std::integral_constant;
-  if (V <= (few ? 4096 : 8192)) go(integral_constant<int, 256>{}, 1024);
+  if (V <= (few ? 4096 : 8192) || (!write_grad && rows > 4 * sm_count() && V <= 51200)) go(integral_constant<int, 256>{}, 1024);
   else if (V <= (few ? 16384 : 76800) || !(few || write_grad)) go(integral_constant<int, 512>{}, 2560);
   else go(integral_constant<int, 1024>{}, 4096);
   LLMT_CHECK_LAUNCH();
