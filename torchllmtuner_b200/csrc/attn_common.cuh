@@ -52,7 +52,7 @@ __device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
 // where tcgen05.mma takes them. In a single-thread branch every operand is moved there instruction by instruction, and beside
 // two softmax warps on the same scheduler that took twice as long as the 64 clocks of a product. 8192 tokens, 32 / 8 heads of
 // 128: forward 642 us -> 513 us, one-kernel backward with its passes 1726 -> 1482; 4096 tokens, 16 / 4 heads of 256, backward
-// 461 -> 368; nothing else changed.
+// kernel 461 -> 368; nothing else changed.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 // Store 32 consecutive bf16 (packed in 16 words) of row `row`, columns [col0, col0+32) into a swizzled K-major tile.

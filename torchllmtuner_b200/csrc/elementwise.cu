@@ -535,7 +535,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const 
 // Bound by memory. The second pass must not go to DRAM again: the first `cached` vectors of the row stay in shared memory and
 // few enough rows are in flight that the rest of them is still in L2 (the launch picks threads and cache). Two vectors per
 // thread and step keep it at 32 registers and the SM full; four took 64 registers and half the threads. 2048 x 151936:
-// 252 us, 4.9 TB/s (before, with the whole row read again from DRAM: 305 us).
+// 250 us, 5.0 TB/s (before, with the whole row read again from DRAM: 305 us).
 template <int NT>
 __global__ void __launch_bounds__(NT, 2048 / NT) ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int64_t* __restrict__ labels,
                                                         float* __restrict__ row_loss, float* __restrict__ row_lse,

@@ -24,8 +24,11 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf
 
 // ------------------------------------------------------------------------------------------ causal convolution + SiLU
 // z[t, c] = sum_j x[t - j, c] * w[c, K - 1 - j] over j = 0 and the taps j <= pos[t] (the index of row t in its document); y = silu(z).
-// Bound by memory: a thread owns 8 channels and walks the `tok` rows of its block with the last K rows in registers, so every row is
-// read once (plus K - 1 rows per block). 2048 x 8192, K = 4: 25 us forward, 86 us backward (67 and 100 MB; as tensor expressions about 1.1 ms together).
+// A thread owns 8 channels and walks the `tok` rows of its block with the last K rows in registers, so every row is read once (plus
+// K - 1 rows per block). Bound by the latency of one row's loads per thread: at 96 and 144 registers 28 % and 17 % of the warps are
+// resident, DRAM is at 30 % and 22 %, issue slots at 37 % and 43 %; the backward also writes and sums fp32 partials of the weight gradient
+// ([blocks, C, K], 17 MB at 2048 x 8192). 2048 x 8192, K = 4: 26 us forward, 82 us backward (67 and 100 MB; as tensor expressions
+// about 1.1 ms together).
 // 16 rows per block; rows of more than 16 x kConvBlocks tokens get longer blocks, which bounds the grid (gridDim.y ends at 65535) and the
 // partial sums of the weight gradient.
 constexpr int kConvTok = 16, kConvBlocks = 4096;
