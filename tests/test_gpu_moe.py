@@ -98,6 +98,15 @@ def test_plan_segments_kernel_matches_tensor_statement(n, E, skew):
         assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
 
 
+def test_traced_plan_follows_its_input():
+    from torchllmtuner_b200.models.moe.experts import plan_segments
+    torch.manual_seed(0)
+    first, second = (torch.randint(0, 8, (100,), device="cuda") for _ in range(2))
+    traced = torch.jit.trace(lambda f: plan_segments(f, 8), (first,), check_trace=False)
+    for a, b in zip(traced(second), plan_segments(second, 8)):
+        assert a.dtype == b.dtype and torch.equal(a, b)
+
+
 @pytest.fixture
 def poisoned():
     """Every buffer that is allocated without a value is full of NaN (torch's deterministic mode does that)."""

@@ -27,7 +27,8 @@ def padded_capacity(num_copies: int, num_experts: int) -> int:
 def plan_segments(flat_expert: torch.Tensor, num_experts: int):
     """From the expert id of each token copy: (dest_row [n] int64 in the padded layout, seg_offsets [E+1] int32,
     counts [E] int64). Copies of one expert keep their order. On the device three kernels and no host synchronisation."""
-    if flat_expert.is_cuda and flat_expert.dtype == torch.int64 and 1 <= num_experts <= PLAN_MAX_EXPERTS:
+    if (flat_expert.is_cuda and flat_expert.dtype == torch.int64 and 1 <= num_experts <= PLAN_MAX_EXPERTS
+            and not torch.jit.is_tracing()):             # a trace would record the kernels' results as constants
         return tuple(_ext().moe_plan(flat_expert.contiguous(), num_experts, SEG_ALIGN))
     counts = torch.bincount(flat_expert, minlength=num_experts)
     padded = (counts + (SEG_ALIGN - 1)) // SEG_ALIGN * SEG_ALIGN
