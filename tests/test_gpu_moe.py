@@ -110,10 +110,13 @@ def test_traced_plan_follows_its_input():
 @pytest.fixture
 def poisoned():
     """Every buffer that is allocated without a value is full of NaN (torch's deterministic mode does that)."""
+    fill = torch.utils.deterministic.fill_uninitialized_memory
     before, warn = torch.are_deterministic_algorithms_enabled(), torch.is_deterministic_algorithms_warn_only_enabled()
     torch.use_deterministic_algorithms(True, warn_only=True)
-    assert torch.utils.deterministic.fill_uninitialized_memory and torch.empty(64, device="cuda", dtype=torch.bfloat16).isnan().all()
+    torch.utils.deterministic.fill_uninitialized_memory = True
+    assert torch.empty(64, device="cuda", dtype=torch.bfloat16).isnan().all()
     yield
+    torch.utils.deterministic.fill_uninitialized_memory = fill
     torch.use_deterministic_algorithms(before, warn_only=warn)
 
 
