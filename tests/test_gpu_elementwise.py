@@ -347,3 +347,24 @@ def test_traced_ops_follow_their_inputs():
         dys = [torch.randn_like(t) for t in ys[0]]
         for a, b in zip((*ys[0], *torch.autograd.grad(ys[0], ins, dys)), (*ys[1], *torch.autograd.grad(ys[1], ins, dys))):
             assert torch.equal(a, b)
+
+
+def test_row_kernels_refuse_views_off_the_16_byte_boundary():
+    """The host answers with an error where a 16-byte access would be misaligned; no kernel is launched."""
+    from torchllmtuner_b200.models.moe.experts import plan_segments
+    from torchllmtuner_b200.ops.cuda_ext import load
+    ext = load()
+    flat = torch.randn(8 * 64 + 8, device="cuda").bfloat16()
+    off, x, w = flat[1:8 * 64 + 1].view(8, 64), torch.randn(8, 64, device="cuda").bfloat16(), torch.randn(64, device="cuda").bfloat16()
+    rstd, y = torch.ones(8, device="cuda"), torch.zeros(8, dtype=torch.int64, device="cuda")
+    dest, seg, counts = plan_segments(torch.zeros(8, dtype=torch.int64, device="cuda"), 1)
+    rows, ones = torch.zeros(128, 64, device="cuda", dtype=torch.bfloat16), torch.ones(8, device="cuda")
+    calls = [lambda: ext.rmsnorm_fwd(off, None, w, 1e-6), lambda: ext.rmsnorm_fwd(x, off, w, 1e-6), lambda: ext.rmsnorm_fwd(x, None, flat[1:65], 1e-6),
+             lambda: ext.rmsnorm_bwd(off, x, w, rstd, None), lambda: ext.rmsnorm_bwd(x, off, w, rstd, None), lambda: ext.rmsnorm_bwd(x, x, w, rstd, off),
+             lambda: ext.ce_fwd_bwd(off, y, 1.0, None, -100, True), lambda: ext.permute_rows(off, dest, rows, 1, seg, counts),
+             lambda: ext.combine_rows(off, y, None, 8, 1), lambda: ext.combine_bwd(off, rows, dest, ones, 1, seg, counts)]
+    before = ext.launch_count()
+    for call in calls:
+        with pytest.raises(RuntimeError, match="-10"):
+            call()
+    assert ext.launch_count() == before

@@ -3,6 +3,7 @@
 // deterministic squared-norm. bf16 storage, fp32 math, 16-byte vector accesses.
 // (reference call sites: llmtuner/models/qwen/ops.py:80-131,503; llmtuner/components/loss.py:35-70;
 //  llmtuner/components/optimizer/optimizer.py:62-106; llmtuner/accelerator/collectives.py:290-558)
+#include <initializer_list>
 #include <type_traits>
 #include "common.cuh"
 #include "kernels.h"
@@ -836,6 +837,13 @@ using namespace llmt;
 
 #define LLMT_CHECK_LAUNCH() return (cudaGetLastError() == cudaSuccess) ? 0 : -3
 
+// Is one of the addresses off a 16-byte boundary? The launchers refuse those (-10): the kernels load and store 16 bytes at a time.
+static inline bool off16(std::initializer_list<const void*> ps) {
+  uintptr_t a = 0;
+  for (const void* p : ps) a |= reinterpret_cast<uintptr_t>(p);
+  return (a & 15) != 0;
+}
+
 // The forward by width: the smallest thread group that covers a row with one vector per thread, up to 256 threads (two or four
 // vectors beyond). A row's time is the chain load - reduce - store, which a second vector lengthens, and the two-vector groups of 64 and
 // 128 threads take 40 registers, so that only 12 of 16 blocks of the grid are resident. us without / with the residual, two vectors on
@@ -868,7 +876,7 @@ static inline void bwd_by_row_width(int D, F&& f) {
 extern "C" int llmt_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* sum_out, float* rstd, int T,
                                 int D, float eps, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (D % 8 || D > 8 * kRowThreads * 4) return -10;
+  if (D % 8 || D > 8 * kRowThreads * 4 || off16({x, res, w, y, sum_out})) return -10;
   auto X = (const __nv_bfloat16*)x; auto R = (const __nv_bfloat16*)res; auto W = (const __nv_bfloat16*)w;
   auto Y = (__nv_bfloat16*)y; auto S = (__nv_bfloat16*)sum_out;
   fwd_by_row_width(T, D, [&](auto nv, auto tr) {
@@ -889,7 +897,7 @@ extern "C" int llmt_rmsnorm_bwd(const void* dy, const void* x, const void* w, co
                                 float* dw_partial, float* dw_f32, void* dw_bf16, int accumulate, int T, int D,
                                 cudaStream_t st) {
   if (T <= 0) return 0;
-  if (D % 8 || D > 8 * kRowThreads * 4) return -10;
+  if (D % 8 || D > 8 * kRowThreads * 4 || off16({dy, x, w, dres, dx, dw_partial})) return -10;
   auto DY = (const __nv_bfloat16*)dy; auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
   auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
   int grid = 0;
@@ -990,7 +998,7 @@ extern "C" int llmt_ce_fwd_bwd(void* logits, const int64_t* labels, float* row_l
                                int64_t ld, const float* grad_scale_ptr, float grad_scale, int ignore_index, int write_grad,
                                cudaStream_t st) {
   if (rows <= 0) return 0;
-  if (ld % 8) return -10;
+  if (ld % 8 || (V >= 8 && off16({logits}))) return -10;
   auto L = (__nv_bfloat16*)logits;
   const int nvec = V / 8;
   auto go = [&](auto nt, int most) {                       // `most`: vectors of a row that may be cached

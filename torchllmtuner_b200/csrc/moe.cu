@@ -404,11 +404,15 @@ extern "C" int llmt_moe_plan(const int64_t* flat, int64_t n, int E, int align, i
   if (nb > 0) moe_plan_place_kernel<<<nb, kPlanBlock, 0, st>>>(flat, n, E, hist, dest);
   LLMT_CHECK_LAUNCH();
 }
+// Is one of the addresses off a 16-byte boundary? The launchers refuse those (-10): the kernels load and store 16 bytes at a time.
+static inline bool off16(const void* a, const void* b, const void* c = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) != 0;
+}
 // With `seg` [E + 1] and `counts` [E] the padding rows of every segment are zeroed too.
 extern "C" int llmt_permute_rows(const void* x, const int64_t* dest, void* rows, int64_t ncopies, int k, int D, const int* seg,
                                  const int64_t* counts, int E, cudaStream_t st) {
   if (ncopies <= 0) return 0;
-  if (D % 8) return -10;
+  if (D % 8 || off16(x, rows)) return -10;
   const int nb = (int)((ncopies + 7) / 8);
   permute_rows_kernel<<<nb + (seg ? E * kPadBlocks : 0), 256, 0, st>>>((const __nv_bfloat16*)x, dest, (__nv_bfloat16*)rows, ncopies, k, D, nb, seg,
                                                                       counts);
@@ -416,7 +420,7 @@ extern "C" int llmt_permute_rows(const void* x, const int64_t* dest, void* rows,
 }
 extern "C" int llmt_combine_rows(const void* y, const int64_t* dest, const float* w, void* out, int T, int k, int D, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (D % 8 || k < 1) return -10;
+  if (D % 8 || k < 1 || off16(y, out)) return -10;
   const int slices = (D / 8 + 31) / 32;
   combine_rows_kernel<<<(unsigned)(((int64_t)T * slices + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)y, dest, w, (__nv_bfloat16*)out, T, k, D, slices);
   LLMT_CHECK_LAUNCH();
@@ -424,7 +428,7 @@ extern "C" int llmt_combine_rows(const void* y, const int64_t* dest, const float
 extern "C" int llmt_combine_bwd(const void* dout, const void* y, const int64_t* dest, const float* w, void* dy, float* dw,
                                 int64_t ncopies, int k, int D, const int* seg, const int64_t* counts, int E, cudaStream_t st) {
   if (ncopies <= 0) return 0;
-  if (D % 8) return -10;
+  if (D % 8 || off16(dout, y, dy)) return -10;
   const int nb = (int)((ncopies + 7) / 8);
   combine_bwd_kernel<<<nb + (seg ? E * kPadBlocks : 0), 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)y, dest, w,
                                                                      (__nv_bfloat16*)dy, dw, ncopies, k, D, nb, seg, counts);
